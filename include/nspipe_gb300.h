@@ -43,7 +43,8 @@ extern "C" {
                                 loop stopped at maxit with err > tol; the steps were
                                 taken as the reference takes them                   */
 
-#define NSP_FP64 0  /* plain form: every operation in FP64 (matches the reference)         */
+#define NSP_FP64 0  /* plain form: FP64 (matches the reference); its FFTs in 64-bit fixed point, one scale
+                             per transform line, whose error is below an FP64 FFT's                    */
 #define NSP_MIXED 1 /* transforms + nonlinear product in FP32 (theta DFT 3xTF32); solves and corrections
                              in double-float (FP32 pairs) or FP32 on corrector increments; state in FP64 */
 

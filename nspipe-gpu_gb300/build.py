@@ -29,13 +29,13 @@ CU_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-Wall", "-I", os.path.join(CUDA, "include"),
              "-I", os.path.join(HERE, "..", "include")]
 
-CU_UNITS = ["nsp_api.cu", "nsp_linear.cu", "nsp_transform.cu", "nsp_noalloc.cu", "nsp_theta_tc.cu", "nsp_remesh.cu",
+CU_UNITS = ["nsp_api.cu", "nsp_linear.cu", "nsp_transform.cu", "nsp_transform_fx.cu", "nsp_noalloc.cu", "nsp_theta_tc.cu", "nsp_remesh.cu",
             "nsp_setup_dev.cu"]
 # Per-unit extra flags.  nsp_setup_dev.cu builds the operator tables that nsp_setup.cpp
 # builds on the host (-ffp-contract=off): without FMA contraction both give the same bits.
 CU_EXTRA = {"nsp_setup_dev.cu": ["-fmad=false"]}
 CXX_UNITS = ["nsp_setup.cpp", "nsp_run.cpp"]
-HEADERS = ["nsp_internal.h", "nsp_setup_mode.h", "nsp_fft.cuh", "nsp_cvt.cuh", "nsp_state.cuh", "nsp_tc.cuh",
+HEADERS = ["nsp_internal.h", "nsp_setup_mode.h", "nsp_fft.cuh", "nsp_fx.cuh", "nsp_cvt.cuh", "nsp_state.cuh", "nsp_tc.cuh",
            "nsp_bounds.cuh", "nsp_df.cuh", os.path.join("..", "..", "include", "nspipe_gb300.h")]
 
 

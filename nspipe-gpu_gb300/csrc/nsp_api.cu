@@ -810,7 +810,8 @@ int nsp_setup(nsp_ctx* c) {
     }
     std::vector<double2> wt = twiddles(tb.NTP), wz = twiddles(tb.NZR);
     if ((rc = upload(c, &tb.tw_t, wt)) || (rc = upload(c, &tb.tw_z, wz)) || (rc = upload(c, &tb.tw_t32, to_f32(wt))) ||
-        (rc = upload(c, &tb.tw_z32, to_f32(wz))))
+        (rc = upload(c, &tb.tw_z32, to_f32(wz))) || (rc = upload(c, &tb.tw_tx, fx_twiddles(tb.NTP))) ||
+        (rc = upload(c, &tb.tw_zx, fx_twiddles(tb.NZR))))
       return rc;
     make_plan(tb.NTP, tb.pt);
     make_plan(tb.NZR, tb.pz);
@@ -842,6 +843,7 @@ int nsp_setup(nsp_ctx* c) {
     }
   }
   configure_transform_kernels();
+  configure_transform_fx_kernels();
   configure_linear_kernels();
   configure_theta_tc_kernels();
   CK(cudaGetLastError());

@@ -10,6 +10,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "nsp_internal.h"
 
 namespace nsp {
@@ -31,6 +33,17 @@ template <typename T, int SIGN> __device__ __forceinline__ cpx<T> muli(cpx<T> a)
   return SIGN > 0 ? mk<T>(-a.y, a.x) : mk<T>(a.y, -a.x);
 }
 
+// 64-bit fixed point (nsp_fx.cuh): the value type of the FP64 form's transforms.
+using fx = long long;
+template <> struct vec2<fx> { using type = int4; };  // a twiddle as two split 62-bit fractions
+
+// v times the table's twiddle w = exp(-2 pi i e / n), conjugated for the inverse (SIGN > 0).
+template <typename T, int SIGN>
+__device__ __forceinline__ cpx<T> twmul(const cpx<T>& v, const typename vec2<T>::type& w) {
+  return cmulv(v, mk<T>(w.x, SIGN > 0 ? -w.y : w.y));
+}
+template <int SIGN> __device__ __forceinline__ void dft3_fx(cpx<fx>* v);  // nsp_fx.cuh
+
 template <typename T, int SIGN, int P> __device__ __forceinline__ void dft(cpx<T>* v) {
   if (P == 2) {
     cpx<T> a = v[0], b = v[1];
@@ -43,7 +56,9 @@ template <typename T, int SIGN, int P> __device__ __forceinline__ void dft(cpx<T
     v[2] = csub(t0, t2);
     v[1] = cadd(t1, t3);
     v[3] = csub(t1, t3);
-  } else {  // P == 3
+  } else if constexpr (std::is_same<T, fx>::value) {  // P == 3
+    dft3_fx<SIGN>(v);
+  } else {
     const T s3 = (T)0.8660254037844386;  // sin(pi/3)
     cpx<T> s = cadd(v[1], v[2]), d = csub(v[1], v[2]);
     cpx<T> a = v[0];
@@ -87,9 +102,7 @@ __device__ __forceinline__ void fft_stage(cpx<T>* buf, int n, int nb, int es, in
       if (k) {
 #pragma unroll
         for (int q = 1; q < P; q++) {
-          typename vec2<T>::type w = __ldg(tw + (q * k * tstride) % n);
-          cpx<T> wc = mk<T>(w.x, SIGN > 0 ? -w.y : w.y);
-          v[rr][q] = cmulv(v[rr][q], wc);
+          v[rr][q] = twmul<T, SIGN>(v[rr][q], __ldg(tw + (q * k * tstride) % n));
         }
       }
       dft<T, SIGN, P>(v[rr]);
@@ -164,8 +177,7 @@ __device__ __forceinline__ void fft_stage_ct(cpx<T>* buf, const typename vec2<T>
       if (NS > 1) {
 #pragma unroll
         for (int q = 1; q < P; q++) {
-          typename vec2<T>::type w = __ldg(tw + q * k * TSTR);
-          v[rr][q] = cmulv(v[rr][q], mk<T>(w.x, SIGN > 0 ? -w.y : w.y));
+          v[rr][q] = twmul<T, SIGN>(v[rr][q], __ldg(tw + q * k * TSTR));
         }
       }
       dft<T, SIGN, P>(v[rr]);

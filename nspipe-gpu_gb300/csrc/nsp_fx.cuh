@@ -1,0 +1,315 @@
+// nsp_fx.cuh -- 64-bit fixed point for the FP64 form's transforms.
+//
+// GB300 issues one FP64 warp instruction per 64 cycles and SM sub-partition, a 32-bit
+// integer one per 2: an FP64 transform is bound by that pipe alone.  A transform is a
+// sum of its inputs with coefficients of modulus 1, so with the inputs of one line
+// (all of them, one scale) held as 64-bit integers no partial sum overflows and every
+// addition is exact: two integer instructions instead of 64 cycles.  Only the
+// twiddle products round, at one unit of the last place.
+//
+//   scale     a line's values are multiplied by 2^(61 - E), E the exponent of an upper
+//             bound of sum |Re| + |Im| over the line (two-sided for a real field's half
+//             spectrum), so the unit is 2^-61 of that sum and everything stays below 2^62
+//             with two real fields packed into one complex transform;
+//   error     a white line of n values has a sum of sqrt(n) times its norm, so the unit is
+//             2^-57 of the result's norm at n = 257 and less elsewhere; the products' rounding
+//             leaves 2^-55 .. 2^-58 of the norm where an FP64 transform leaves 2^-53;
+//   products  x w with w = 2^62 times a twiddle, both split into 32-bit halves with a signed
+//             low part: 3 of the 4 half products (the low-low one is below one unit), the
+//             middle ones rounded to nearest: 6 wide multiply-adds per real output.
+//             Measured against 64-bit long-double arithmetic (N at one level, norm-wise):
+//             1.2e-16 .. 3.3e-16 for decaying and 1.5e-16 .. 4.0e-16 for white spectra of
+//             32 x 65 to 128 x 257 modes, 2.7e-16 .. 6.4e-16 and 1.3e-15 .. 3.6e-15 with the
+//             FP64 transforms it replaced;
+//   Inf, NaN  a line that holds one gives NaN (its E is FX_BAD), as its FP64 transform would.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "nsp_fft.cuh"
+
+namespace nsp {
+
+constexpr int FX_BITS = 61;      // a line's sum of magnitudes stays below 2^FX_BITS
+constexpr int FX_BAD = 1 << 20;  // exponent of a line that holds Inf or NaN
+
+// Upper 31 bits of |x|: orders like the value (as an unsigned integer).
+__device__ __forceinline__ unsigned fx_key(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
+
+// |x| of key k in units of 2^(emax - 20), rounded up, for keys with exponents up to emax.
+__device__ __forceinline__ unsigned fx_mag(unsigned k, unsigned emax) {
+  return (((k & 0xFFFFFu) | 0x100000u) >> min(emax - (k >> 20), 31u)) + 1u;
+}
+
+// The line's exponent E from its largest key and its sum of magnitudes (fx_mag units):
+// the sum is below 2^E.  Clamped so that zero and subnormal lines convert to 0.
+__device__ __forceinline__ int fx_exponent(unsigned kmax, unsigned sum) {
+  const int emax = (int)(kmax >> 20);
+  if (emax >= 0x7FF) return FX_BAD;
+  return max(emax - 1043 + (32 - __clz((int)sum)), -900);
+}
+
+// x 2^(FX_BITS - E) rounded to the nearest integer; |x| < 2^E.  (Truncation would stop every
+// coefficient below one unit; rounded, the units of the others carry it on average as the
+// roundings of a floating-point sum do.)
+__device__ __forceinline__ fx fx_from(double x, int E) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned mh = (hi & 0xFFFFFu) | 0x100000u;
+  // 1.m left-aligned below the sign bit, then shifted right by r >= 2
+  const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, 10) << 32) | (lo << 10);
+  const int r = E + 1085 - FX_BITS - (int)((hi >> 20) & 0x7FFu);
+  const fx v = (fx)(((m >> (min(max(r, 1), 64) - 1)) + 1) >> 1);
+  const fx s = (fx)((int)hi >> 31);
+  return (v ^ s) - s;
+}
+// The same for x q, q < 2^9 a whole number: the product is formed exactly.
+__device__ __forceinline__ fx fx_from_times(double x, unsigned q, int E) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned mh = (hi & 0xFFFFFu) | 0x100000u;
+  const int z = __clz((int)q) - 22;  // q 2^z in [2^9, 2^10): the product in [2^61, 2^63)
+  const unsigned qz = q << z;
+  const unsigned long long m = (unsigned long long)lo * qz + ((unsigned long long)(mh * qz) << 32);
+  const int r = E + 1075 - FX_BITS - (int)((hi >> 20) & 0x7FFu) + z;
+  const fx v = q ? (fx)(((m >> (min(max(r, 1), 64) - 1)) + 1) >> 1) : 0;
+  const fx s = (fx)((int)hi >> 31);
+  return (v ^ s) - s;
+}
+
+// v 2^e rounded to nearest; 0 below 2^-1022, Inf above FP64's range.
+__device__ __forceinline__ double fx_to(fx v, int e) {
+  const int s = (int)(v >> 63);
+  const unsigned long long a = (unsigned long long)((v ^ (fx)s) - (fx)s);
+  const int lz = __clzll((long long)a);
+  const unsigned long long m = a << (lz & 63);
+  const int be = 1086 - lz + e;  // biased exponent of the leading bit
+  const unsigned long long q = (m >> 11) + ((m >> 10) & 1u);
+  unsigned hi = (unsigned)(q >> 32) + ((unsigned)(be - 1) << 20), lo = (unsigned)q;
+  if (be < 1 || a == 0) hi = lo = 0;
+  if (be > 2046) hi = 0x7FF00000u, lo = 0;
+  return __hiloint2double((int)(hi | ((unsigned)s & 0x80000000u)), (int)lo);
+}
+
+__device__ __forceinline__ double fx_nan() { return __hiloint2double(0x7FF80000, 0); }
+
+// Signed halves: x = h 2^32 + l.
+__device__ __forceinline__ void fx_split(fx x, int& h, int& l) {
+  l = (int)x;
+  h = (int)(x >> 32) - (l >> 31);
+}
+__device__ __forceinline__ long long fx_mad(int a, int b, long long c) { return (long long)a * b + c; }
+// Products are summed as hi 2^64 + mid 2^32, mid first (from the rounding constant); its upper
+// word then starts hi, so that the two words shifted out of (hi, low word of mid) are the
+// result / 2^62.
+constexpr long long FX_HALF = 1ll << 29;
+__device__ __forceinline__ fx fx_out(long long hi, long long mid) {
+  const unsigned h0 = (unsigned)hi, h1 = (unsigned)(hi >> 32);
+  return (fx)(((unsigned long long)__funnelshift_l(h0, h1, 2) << 32) | __funnelshift_l((unsigned)mid, h0, 2));
+}
+
+// x c / 2^62 for c = (ch, cl) in signed halves.
+__device__ __forceinline__ fx fx_mulc(fx x, int ch, int cl) {
+  int h, l;
+  fx_split(x, h, l);
+  const long long mid = fx_mad(l, ch, fx_mad(h, cl, FX_HALF));
+  return fx_out(fx_mad(h, ch, mid >> 32), mid);
+}
+
+// v (re + i im), the factor's parts in signed halves.
+__device__ __forceinline__ cpx<fx> fx_cmul(const cpx<fx>& v, int rh, int rl, int ih, int il) {
+  int xh, xl, yh, yl;
+  fx_split(v.x, xh, xl);
+  fx_split(v.y, yh, yl);
+  const int nh = -ih, nl = -il;
+  const long long mx = fx_mad(yl, nh, fx_mad(yh, nl, fx_mad(xl, rh, fx_mad(xh, rl, FX_HALF))));
+  const long long my = fx_mad(xl, ih, fx_mad(xh, il, fx_mad(yl, rh, fx_mad(yh, rl, FX_HALF))));
+  return mk<fx>(fx_out(fx_mad(yh, nh, fx_mad(xh, rh, mx >> 32)), mx),
+                fx_out(fx_mad(xh, ih, fx_mad(yh, rh, my >> 32)), my));
+}
+// w = exp(-2 pi i e / n) of the table; the inverse takes its conjugate.
+template <> __device__ __forceinline__ cpx<fx> twmul<fx, +1>(const cpx<fx>& v, const int4& w) {
+  return fx_cmul(v, w.x, w.y, -w.z, -w.w);
+}
+template <> __device__ __forceinline__ cpx<fx> twmul<fx, -1>(const cpx<fx>& v, const int4& w) {
+  return fx_cmul(v, w.x, w.y, w.z, w.w);
+}
+
+// Constants exp(2 pi i e / n) of the register transforms as 2^62 fractions in signed halves
+// (Re h, Re l, Im h, Im l): n = 16 for e = 1, 2 and n = 9 for e = 1, 2, 4.
+struct FxConst { int rh, rl, ih, il; };
+constexpr FxConst FX_W16_1{992008094, 1696238673, 410903207, -1364630830};
+constexpr FxConst FX_W16_2{759250125, -25716447, 759250125, -25716447};
+constexpr FxConst FX_W9_1{822533958, -1633652124, 690187940, 2016164183};
+constexpr FxConst FX_W9_2{186453311, 96060625, 1057429273, 37236404};
+constexpr FxConst FX_W9_4{-1008987269, 1537591498, 367241333, -1978927779};
+template <int SIGN> __device__ __forceinline__ cpx<fx> fx_rot(const cpx<fx>& v, FxConst c) {
+  return fx_cmul(v, c.rh, c.rl, SIGN * c.ih, SIGN * c.il);
+}
+
+// s / 2, an odd s rounded to the even neighbour (no bias).
+__device__ __forceinline__ fx fx_half(fx s) {
+  const fx t = s >> 1;
+  return t + (s & t & 1);
+}
+
+// 2^62 sin(pi/3) = 0x376CF5D0B09954E7 rounded, in signed halves.
+constexpr int FX_S3_H = 0x376CF5D1, FX_S3_L = (int)0xB09954E7;
+template <int SIGN> __device__ __forceinline__ void dft3_fx(cpx<fx>* v) {
+  const cpx<fx> s = cadd(v[1], v[2]), id = muli<fx, SIGN>(csub(v[1], v[2])), a = v[0];
+  v[0] = cadd(a, s);
+  const cpx<fx> m = mk<fx>(a.x - fx_half(s.x), a.y - fx_half(s.y));
+  const cpx<fx> e = mk<fx>(fx_mulc(id.x, FX_S3_H, FX_S3_L), fx_mulc(id.y, FX_S3_H, FX_S3_L));
+  v[1] = cadd(m, e);
+  v[2] = csub(m, e);
+}
+
+
+// v exp(SIGN 2 pi i E / N) for the constants of the register transforms, N = 8, 9 or 16.
+template <int SIGN, int N, int E> __device__ __forceinline__ cpx<fx> rotk(const cpx<fx>& v) {
+  if constexpr (N == 9) {
+    return fx_rot<SIGN>(v, E == 1 ? FX_W9_1 : E == 2 ? FX_W9_2 : FX_W9_4);
+  } else {
+    constexpr int e = N == 8 ? 2 * E : E;
+    if constexpr (e == 4) return muli<fx, SIGN>(v);
+    else if constexpr (e == 2 || e == 6) {  // (+-1 + SIGN i) sqrt(1/2)
+      const cpx<fx> i = muli<fx, SIGN>(v), a = e == 2 ? cadd(v, i) : csub(i, v);
+      return mk<fx>(fx_mulc(a.x, FX_W16_2.rh, FX_W16_2.rl), fx_mulc(a.y, FX_W16_2.rh, FX_W16_2.rl));
+    } else if constexpr (e == 1) return fx_rot<SIGN>(v, FX_W16_1);
+    else if constexpr (e == 3) return fx_cmul(v, FX_W16_1.ih, FX_W16_1.il, SIGN * FX_W16_1.rh, SIGN * FX_W16_1.rl);
+    else return fx_cmul(v, -FX_W16_1.rh, -FX_W16_1.rl, -SIGN * FX_W16_1.ih, -SIGN * FX_W16_1.il);  // e == 9
+  }
+}
+
+// P-point transform in registers, natural order: 2, 3, 4 (dft), 8 = 2 x 4, 9 = 3 x 3 and
+// 16 = 4 x 4 with constant twiddles, 6 = 2 x 3 and 12 = 3 x 4 by Good and Thomas without any.
+template <int SIGN, int P> __device__ __forceinline__ void fx_dft(cpx<fx>* v) {
+  if constexpr (P <= 4) {
+    dft<fx, SIGN, P>(v);
+  } else if constexpr (P == 6 || P == 12) {
+    constexpr int A = P / 3;  // 3 x A, coprime; input (A a + 3 b) mod P, output (KA a + KB b) mod P
+    constexpr int KA = 4, KB = A == 4 ? 9 : 3;
+    cpx<fx> t[P];
+#pragma unroll
+    for (int b = 0; b < A; b++) {
+      cpx<fx> x[3] = {v[(3 * b) % P], v[(A + 3 * b) % P], v[(2 * A + 3 * b) % P]};
+      dft<fx, SIGN, 3>(x);
+#pragma unroll
+      for (int a = 0; a < 3; a++) t[a * A + b] = x[a];
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      dft<fx, SIGN, A>(t + a * A);
+#pragma unroll
+      for (int b = 0; b < A; b++) v[(KA * a + KB * b) % P] = t[a * A + b];
+    }
+  } else {
+    constexpr int B = P == 8 ? 2 : P == 9 ? 3 : 4, A = P / B;  // input B a + b, output a + A b
+    cpx<fx> t[B][A];
+#pragma unroll
+    for (int b = 0; b < B; b++) {
+#pragma unroll
+      for (int a = 0; a < A; a++) t[b][a] = v[B * a + b];
+      dft<fx, SIGN, A>(t[b]);
+    }
+    if constexpr (P == 8) {
+      t[1][1] = rotk<SIGN, 8, 1>(t[1][1]);
+      t[1][2] = rotk<SIGN, 8, 2>(t[1][2]);
+      t[1][3] = rotk<SIGN, 8, 3>(t[1][3]);
+    } else if constexpr (P == 9) {
+      t[1][1] = rotk<SIGN, 9, 1>(t[1][1]);
+      t[1][2] = rotk<SIGN, 9, 2>(t[1][2]);
+      t[2][1] = rotk<SIGN, 9, 2>(t[2][1]);
+      t[2][2] = rotk<SIGN, 9, 4>(t[2][2]);
+    } else {
+      t[1][1] = rotk<SIGN, 16, 1>(t[1][1]);
+      t[1][2] = rotk<SIGN, 16, 2>(t[1][2]);
+      t[1][3] = rotk<SIGN, 16, 3>(t[1][3]);
+      t[2][1] = rotk<SIGN, 16, 2>(t[2][1]);
+      t[2][2] = rotk<SIGN, 16, 4>(t[2][2]);
+      t[2][3] = rotk<SIGN, 16, 6>(t[2][3]);
+      t[3][1] = rotk<SIGN, 16, 3>(t[3][1]);
+      t[3][2] = rotk<SIGN, 16, 6>(t[3][2]);
+      t[3][3] = rotk<SIGN, 16, 9>(t[3][3]);
+    }
+#pragma unroll
+    for (int a = 0; a < A; a++) {
+      cpx<fx> x[B];
+#pragma unroll
+      for (int b = 0; b < B; b++) x[b] = t[b][a];
+      dft<fx, SIGN, B>(x);
+#pragma unroll
+      for (int b = 0; b < B; b++) v[a + A * b] = x[b];
+    }
+  }
+}
+
+// Radices of the compiled lengths, chosen so that a transform makes few passes over
+// shared memory (two up to 192 points) with at most 16 complex values in registers;
+// 0: the length has no compiled transform.
+__host__ __device__ constexpr int fx_radix(int n, int s) {
+  constexpr int R[][4] = {{12, 12, 0, 0}, {18, 2, 9, 0}, {24, 4, 6, 0}, {36, 6, 6, 0}, {48, 6, 8, 0},
+                          {54, 6, 9, 0}, {72, 9, 8, 0}, {96, 8, 12, 0}, {108, 9, 12, 0}, {144, 12, 12, 0},
+                          {162, 9, 2, 9}, {192, 16, 12, 0}, {216, 6, 6, 6}, {288, 6, 6, 8}, {384, 8, 6, 8},
+                          {432, 6, 8, 9}, {576, 8, 8, 9}, {768, 8, 8, 12}};
+  for (const auto& r : R)
+    if (r[0] == n) return s < 3 ? r[1 + s] : 0;
+  return 0;
+}
+
+// Place of element e in a line of contiguous elements: one gap per 16 so that the strided
+// stores of a first pass spread over the banks.
+__host__ __device__ constexpr int fx_pad(int e) { return e + (e >> 4); }
+
+// One Stockham pass of radix P over NB transforms of length N (see fft_stage_ct), in place:
+// element e of transform t at t BS + e ES (COLS: neighbouring threads on neighbouring
+// transforms) or at t BS + fx_pad(e).  Elements [Z0, Z1] are known to be zero on the way in
+// (first pass), elements [D0, D1] not needed on the way out (last pass); empty if Z1 < Z0.
+template <int SIGN, int N, int NB, int ES, int BS, bool COLS, int NTH, int P, int NS, int Z0, int Z1, int D0, int D1>
+__device__ __forceinline__ void fx_pass(cpx<fx>* buf, const int4* __restrict__ tw) {
+  constexpr int NBF = N / P, TOTAL = NB * NBF, R = (TOTAL + NTH - 1) / NTH, TSTR = N / (NS * P);
+  cpx<fx> v[R][P];
+#pragma unroll
+  for (int rr = 0; rr < R; rr++) {
+    const int b = threadIdx.x + rr * NTH;
+    if (TOTAL % NTH == 0 || b < TOTAL) {
+      const int t = COLS ? b % NB : b / NBF, j = COLS ? b / NB : b - t * NBF;
+#pragma unroll
+      for (int q = 0; q < P; q++) {
+        const int e = j + q * NBF;
+        if (NS == 1 && q * NBF >= Z0 && (q + 1) * NBF - 1 <= Z1) v[rr][q] = mk<fx>(0, 0);
+        else v[rr][q] = buf[t * BS + (COLS ? e * ES : fx_pad(e))];
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int rr = 0; rr < R; rr++) {
+    const int b = threadIdx.x + rr * NTH;
+    if (TOTAL % NTH == 0 || b < TOTAL) {
+      const int t = COLS ? b % NB : b / NBF, j = COLS ? b / NB : b - t * NBF;
+      const int k = (NS == 1) ? 0 : j % NS;
+      if (NS > 1) {
+#pragma unroll
+        for (int q = 1; q < P; q++) v[rr][q] = twmul<fx, SIGN>(v[rr][q], __ldg(tw + q * k * TSTR));
+      }
+      fx_dft<SIGN, P>(v[rr]);
+      const int base = (NS == 1) ? j * P : (j / NS) * NS * P + k;
+#pragma unroll
+      for (int q = 0; q < P; q++) {
+        if (NS * P == N && q * NS >= D0 && (q + 1) * NS - 1 <= D1) continue;
+        const int e = base + q * NS;
+        buf[t * BS + (COLS ? e * ES : fx_pad(e))] = v[rr][q];
+      }
+    }
+  }
+  __syncthreads();
+}
+
+template <int SIGN, int N, int NB, int ES, int BS, bool COLS, int NTH, int Z0, int Z1, int D0, int D1, int S = 0, int NS = 1>
+__device__ __forceinline__ void fx_fft(cpx<fx>* buf, const int4* __restrict__ tw) {
+  constexpr int P = fx_radix(N, S);
+  if constexpr (P > 0) {
+    fx_pass<SIGN, N, NB, ES, BS, COLS, NTH, P, NS, Z0, Z1, D0, D1>(buf, tw);
+    fx_fft<SIGN, N, NB, ES, BS, COLS, NTH, Z0, Z1, D0, D1, S + 1, NS * P>(buf, tw);
+  }
+}
+
+}  // namespace nsp

@@ -63,6 +63,8 @@ struct Tables {
   const double2* tw_z; // [NZR]
   const float2* tw_t32;
   const float2* tw_z32;
+  const int4* tw_tx;   // the same twiddles as 62-bit fractions (nsp_fx.cuh)
+  const int4* tw_zx;
   FftPlan pt, pz;
   int lin_variant;     // block shape of the linear pass (autotuned at setup)
   int lin_variant_inc; // mixed form: block shape of the increment (corrector) pass
@@ -172,6 +174,11 @@ void launch_split_fac(const double* fac, float2* dfo, float* f32o, long long n, 
 // The FP32 mirror and its radial derivative (DR32) of a group's state U (mixed form).
 void launch_mirror(const Tables& tb, const double2* U, float2* U32, float2* DR32, cudaStream_t st);
 int kernels_per_nonlinear();
+// The FP64 form's transforms (nsp_transform_fx.cu), 64-bit fixed point inside; mask as above.
+void launch_nonlinear_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, const double2* src, double2* dst,
+                         cudaStream_t st, int mask);
+void configure_transform_fx_kernels();
+std::vector<int4> fx_twiddles(int n);
 // z-stage kernels of a length (nsp_transform.cu): the number of two-pass splits compiled
 // for NZR (rows per block dividing NTP) in the precision, and a description of variant v.
 int z_variants(int NZR, int NTP, bool fp32);

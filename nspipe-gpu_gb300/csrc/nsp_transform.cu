@@ -20,9 +20,9 @@
 //                 (theta Nyquist and l = NZ-1 zeroed) and apply the wall-shear
 //                 forcing to N_z(0,0).
 //
-// T = double gives the plain FP64 form; T = float the mixed form (the state is
-// rounded to FP32 on load, the stencils and products run in FP32, N is written
-// back in FP64).  Transform lengths used by the supported configurations are
+// These are the mixed form's kernels (T = float: the transforms read the FP32 mirror of
+// the state, the stencils and products run in FP32); the FP64 form's, over the same
+// arrays, are in nsp_transform_fx.cu.  Transform lengths used by the supported configurations are
 // compile-time template arguments (all index arithmetic by constants); other
 // 2^a 3^b lengths use the run-time FFT.
 #include <cmath>
@@ -44,10 +44,8 @@ constexpr int ZTH = 256;  // threads of the z kernel
 constexpr int Z2TH = 192; // threads of the two-pass z kernel (its passes run 192, 144, 384, 48, 36, 384 tasks)
 
 template <typename T> __device__ __forceinline__ const typename vec2<T>::type* tw_t(const Tables& tb);
-template <> __device__ __forceinline__ const double2* tw_t<double>(const Tables& tb) { return tb.tw_t; }
 template <> __device__ __forceinline__ const float2* tw_t<float>(const Tables& tb) { return tb.tw_t32; }
 template <typename T> __device__ __forceinline__ const typename vec2<T>::type* tw_z(const Tables& tb);
-template <> __device__ __forceinline__ const double2* tw_z<double>(const Tables& tb) { return tb.tw_z; }
 template <> __device__ __forceinline__ const float2* tw_z<float>(const Tables& tb) { return tb.tw_z32; }
 
 template <typename T, int NTPC>
@@ -111,14 +109,14 @@ __global__ void __launch_bounds__(TTH) nl_theta_inv(Tables tb, Bufs bf, const Ct
         v = mk<T>(sx, sy);
       } else {  // derivt_k, mod_deriv.cu:10-21
         int m = it < NT / 2 ? it : it - NT;
-        T kt = (sizeof(T) == 8) ? (T)(tb.kts * (double)m) : (T)m * ktsT;
+        T kt = (T)m * ktsT;
         cpx<T> a = U.ld((size_t)i * NTNZ + col);
         v = mk<T>(-kt * a.y * rinv, kt * a.x * rinv);
       }
       // mixed form: the mean flow is recorded for the linear pass (member steps) and kept
       // out of the transforms; its terms are added by the linear pass, or for an explicit
       // field by nl_theta_fwd
-      if (sizeof(T) == 4 && it == 0 && coll[lc] == 0) {
+      if (it == 0 && coll[lc] == 0) {
         const int slot = f == 0 ? MEAN_V : f == 1 ? MEAN_W : f == 2 ? MEAN_U : f == 4 ? MEAN_WP : f == 5 ? MEAN_UP : -1;
         if (!src_override && slot >= 0) bf.MEAN[((size_t)mloc * NR + i) * MEAN_N + slot] = (float)v.x;
         if (mean_field(f)) v = mk<T>(0, 0);
@@ -243,10 +241,8 @@ __global__ void __launch_bounds__(ZTH) nl_z(Tables tb, Bufs bf, const Ctl* ctl, 
 
 // exp(-2 pi i e / 96): every register sub-transform length used (4 .. 32) divides 96.
 __constant__ float2 c_w96f[96];
-__constant__ double2 c_w96d[96];
 template <typename T> __device__ __forceinline__ cpx<T> w96(int e);
 template <> __device__ __forceinline__ cpx<float> w96<float>(int e) { float2 w = c_w96f[e]; return mk<float>(w.x, w.y); }
-template <> __device__ __forceinline__ cpx<double> w96<double>(int e) { double2 w = c_w96d[e]; return mk<double>(w.x, w.y); }
 
 // In-register Stockham FFT of length N | 96 (every index a compile-time constant
 // once unrolled, so the array stays in registers); natural order in and out.
@@ -492,11 +488,9 @@ __global__ void __launch_bounds__(TTH) nl_theta_fwd(Tables tb, Bufs bf, const Ct
   // mixed form, explicit field: the mean-flow terms (nsp_state.cuh), from its FP32 copy
   const float2* U32 = nullptr;
   Mean32 mf{};
-  if constexpr (sizeof(T) == 4) {
-    if (src_override) {  // a member state's terms are added by the linear pass
-      U32 = src32_override;
-      mf = mean_flow32(tb, U32, nullptr, i);
-    }
+  if (src_override) {  // a member state's terms are added by the linear pass
+    U32 = src32_override;
+    mf = mean_flow32(tb, U32, nullptr, i);
   }
   for (int idx = threadIdx.x; idx < NT * LC; idx += TTH) {
     int it = idx / LC, lc = idx % LC;
@@ -505,9 +499,7 @@ __global__ void __launch_bounds__(TTH) nl_theta_fwd(Tables tb, Bufs bf, const Ct
     int p = it < NT / 2 ? it : NTP + it - NT;
     cpx<T> b = buf[p * LC + lc];
     double2 v;
-    if constexpr (sizeof(T) == 8) {
-      v = make_double2((double)b.x * tb.inv_norm, (double)b.y * tb.inv_norm);
-    } else if (!dst_override) {
+    if (!dst_override) {
       // a member's N in the mixed form: FP32 (its values are FP32 numbers), the wall forcing
       // of Re N_z(0,0) kept apart in FP64 -- the same at every level, written by level 0
       const bool drop = it == NT / 2 || l == NZ - 1;
@@ -572,18 +564,15 @@ static void launch_z2(const Tables& tb, const Bufs& bf, Ctl* dctl, bool standalo
 
 #define NSP_NTP_LIST(X) X(12) X(24) X(48) X(72) X(96) X(144) X(192)
 #define NSP_NZR_LIST(X) X(24, 2) X(48, 2) X(96, 2) X(192, 2) X(384, 2) X(576, 1) X(768, 1)
-// Two-pass z stage: (NZR, N1, N2, rows per block), the splits compiled for FP32 and for
-// FP64 (whose shared memory, twice FP32's, limits it to NZR <= 384); the setup-time
-// autotuner picks among them and the radix-stage kernel per shape.
-#define NSP_Z2_LIST_F(X) X(24, 4, 6, 2) X(48, 8, 6, 2) X(96, 8, 12, 2) X(96, 12, 8, 2) X(192, 16, 12, 2) \
+// Two-pass z stage: (NZR, N1, N2, rows per block); the setup-time autotuner picks among
+// the splits and the radix-stage kernel per shape.
+#define NSP_Z2_LIST(X) X(24, 4, 6, 2) X(48, 8, 6, 2) X(96, 8, 12, 2) X(96, 12, 8, 2) X(192, 16, 12, 2) \
   X(192, 12, 16, 2) X(384, 16, 24, 2) X(384, 24, 16, 2) X(576, 24, 24, 2) X(768, 32, 24, 2) X(768, 24, 32, 2)
-#define NSP_Z2_LIST_D(X) X(24, 4, 6, 2) X(48, 8, 6, 2) X(96, 8, 12, 2) X(192, 16, 12, 2) X(192, 12, 16, 2) \
-  X(384, 16, 24, 2)
 
 int z_variants(int NZR, int NTP, bool fp32) {
   int n = 0;
 #define NSP_Z2_COUNT(len, a, b, r) n += (NZR == len && NTP % r == 0);
-  if (fp32) { NSP_Z2_LIST_F(NSP_Z2_COUNT) } else { NSP_Z2_LIST_D(NSP_Z2_COUNT) }
+  if (fp32) { NSP_Z2_LIST(NSP_Z2_COUNT) }
 #undef NSP_Z2_COUNT
   return n;
 }
@@ -597,12 +586,13 @@ int z_default_variant(int NZR, int NTP, bool fp32) {
 }
 
 std::string z_variant_name(int NZR, int NTP, bool fp32, int v) {
+  if (!fp32) return "radix, 64-bit fixed point";
   if (v <= 0) return "radix";
   int k = 0;
   std::string s = "radix";
 #define NSP_Z2_NAME(len, a, b, r) \
   if (NZR == len && NTP % r == 0 && ++k == v) s = "two-pass " #a "x" #b;
-  if (fp32) { NSP_Z2_LIST_F(NSP_Z2_NAME) } else { NSP_Z2_LIST_D(NSP_Z2_NAME) }
+  NSP_Z2_LIST(NSP_Z2_NAME)
 #undef NSP_Z2_NAME
   return s;
 }
@@ -611,7 +601,7 @@ template <typename T>
 static void launch_nl_t(const Tables& tb, const Bufs& bf, Ctl* dctl, const double2* src, const float2* src32,
                         double2* dst, cudaStream_t st, int mask) {
   int nm = src ? 1 : tb.nmem;
-  const bool tc = sizeof(T) == 4 && tb.tc_theta;  // mixed form: theta transforms on the tensor cores
+  const bool tc = tb.tc_theta;  // mixed form: theta transforms on the tensor cores
   if ((mask & 1) && tc) {
     launch_theta_tc(tb, bf, dctl, 0, src, src32, dst, st);
   } else if (mask & 1) {
@@ -633,7 +623,7 @@ static void launch_nl_t(const Tables& tb, const Bufs& bf, Ctl* dctl, const doubl
     launch_z2<T, n, a, b, r>(tb, bf, dctl, src != nullptr, st, nm);                  \
     done = true;                                                                     \
   }
-      if constexpr (sizeof(T) == 4) { NSP_Z2_LIST_F(NSP_CASE_Z2) } else { NSP_Z2_LIST_D(NSP_CASE_Z2) }
+      NSP_Z2_LIST(NSP_CASE_Z2)
 #undef NSP_CASE_Z2
     }
     if (!done) {
@@ -677,28 +667,19 @@ static void configure_t() {
 }
 
 void configure_transform_kernels() {
-  configure_t<double>();
   configure_t<float>();
 #define NSP_CFG_Z2F(n, a, b, r)                                                          \
   cudaFuncSetAttribute(nl_z2<float, n, a, b, r>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                        (int)z2_smem<float, n, a, b, r>());
-  NSP_Z2_LIST_F(NSP_CFG_Z2F)
+  NSP_Z2_LIST(NSP_CFG_Z2F)
 #undef NSP_CFG_Z2F
-#define NSP_CFG_Z2D(n, a, b, r)                                                           \
-  cudaFuncSetAttribute(nl_z2<double, n, a, b, r>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                       (int)z2_smem<double, n, a, b, r>());
-  NSP_Z2_LIST_D(NSP_CFG_Z2D)
-#undef NSP_CFG_Z2D
   // Twiddles of the register sub-transforms, exp(-2 pi i e / 96), from long double.
   float2 wf[96];
-  double2 wd[96];
   for (int e = 0; e < 96; e++) {
     const long double a = -6.283185307179586476925286766559L * (long double)e / 96.0L;
-    wd[e] = make_double2((double)cosl(a), (double)sinl(a));
     wf[e] = make_float2((float)cosl(a), (float)sinl(a));
   }
   cudaMemcpyToSymbol(c_w96f, wf, sizeof(wf));
-  cudaMemcpyToSymbol(c_w96d, wd, sizeof(wd));
 }
 
 bool transform_supported(int NTP, int NZR) {
@@ -718,7 +699,7 @@ bool transform_supported(int NTP, int NZR) {
 void launch_nonlinear(const Tables& tb, const Bufs& bf, Ctl* dctl, bool mixed, const double2* src, double2* dst,
                       cudaStream_t st, int mask, const float2* src32) {
   if (mixed) launch_nl_t<float>(tb, bf, dctl, src, src32, dst, st, mask);
-  else launch_nl_t<double>(tb, bf, dctl, src, nullptr, dst, st, mask);
+  else launch_nonlinear_fx(tb, bf, dctl, src, dst, st, mask);
 }
 
 __global__ void to_f32_k(const double2* __restrict__ src, float2* __restrict__ dst, long long n) {
