@@ -29,7 +29,7 @@ CU_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-Wall", "-I", os.path.join(CUDA, "include"),
              "-I", os.path.join(HERE, "..", "include")]
 
-CU_UNITS = ["nsp_api.cu", "nsp_linear.cu", "nsp_transform.cu", "nsp_transform_fx.cu", "nsp_noalloc.cu", "nsp_theta_tc.cu", "nsp_remesh.cu",
+CU_UNITS = ["nsp_api.cu", "nsp_linear.cu", "nsp_transform.cu", "nsp_transform_fx.cu", "nsp_cross.cu", "nsp_noalloc.cu", "nsp_theta_tc.cu", "nsp_remesh.cu",
             "nsp_setup_dev.cu"]
 # Per-unit extra flags.  nsp_setup_dev.cu builds the operator tables that nsp_setup.cpp
 # builds on the host (-ffp-contract=off): without FMA contraction both give the same bits.

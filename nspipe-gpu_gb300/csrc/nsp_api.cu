@@ -844,6 +844,7 @@ int nsp_setup(nsp_ctx* c) {
   }
   configure_transform_kernels();
   configure_transform_fx_kernels();
+  configure_cross_kernels();
   configure_linear_kernels();
   configure_theta_tc_kernels();
   CK(cudaGetLastError());
@@ -1499,35 +1500,30 @@ int nsp_cross_sections_all(nsp_ctx* c, double* q, double* u) {
   if (!c) return NSP_ERR_ARG;
   if (!q || !u) return fail(c, NSP_ERR_ARG, "null output");
   if (!c->setup_done) return fail(c, NSP_ERR_STATE, "nsp_cross_sections_all before nsp_setup");
-  std::vector<size_t> poff(c->groups.size());
-  size_t n = 0;
+  std::vector<size_t> ooff(c->groups.size()), poff(c->groups.size());
+  size_t no = 0, np = 0;
   for (size_t k = 0; k < c->groups.size(); k++) {
-    poff[k] = n;
-    n += (size_t)c->groups[k].tb.nmem * 2 * c->groups[k].tb.NR * c->groups[k].tb.NZR;
+    const Tables& tb = c->groups[k].tb;
+    ooff[k] = no;
+    poff[k] = np;
+    no += (size_t)tb.nmem * 2 * tb.NZR;
+    np += (size_t)tb.nmem * 3 * tb.NR * tb.NZR;
   }
-  if (int rc = ensure_crossbuf(c, n)) return rc;
+  if (int rc = ensure_crossbuf(c, no + np)) return rc;
   for (size_t k = 0; k < c->groups.size(); k++) {
     const Group& g = c->groups[k];
-    launch_diag_cross(g.tb, g.bf.U[c->parity], c->crossbuf + poff[k], c->st, g.tb.nmem);
+    launch_diag_cross(g.tb, g.bf.U[c->parity], c->crossbuf + no + poff[k], c->crossbuf + ooff[k], c->st, g.tb.nmem);
   }
   CK(cudaGetLastError());
-  std::vector<double> part(n);
-  CK(cudaMemcpyAsync(part.data(), c->crossbuf, n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  std::vector<double> out(no);
+  CK(cudaMemcpyAsync(out.data(), c->crossbuf, no * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
   size_t o = 0;
   for (int m = 0; m < c->nmem; m++) {
-    const Group& g = c->groups[c->grp[m]];
-    const int NR = g.tb.NR, NZR = g.tb.NZR;
-    const double* pm = part.data() + poff[c->grp[m]] + (size_t)c->slot[m] * 2 * NR * NZR;
-    for (int z = 0; z < NZR; z++) {
-      double sq = 0.0, su = 0.0;
-      for (int i = 0; i < NR; i++) {  // the radial quadrature, in level order
-        sq += pm[(size_t)i * NZR + z];
-        su += pm[(size_t)(NR + i) * NZR + z];
-      }
-      q[o + z] = sq;
-      u[o + z] = su;
-    }
+    const int NZR = c->groups[c->grp[m]].tb.NZR;
+    const double* pm = out.data() + ooff[c->grp[m]] + (size_t)c->slot[m] * 2 * NZR;
+    memcpy(q + o, pm, sizeof(double) * NZR);
+    memcpy(u + o, pm + NZR, sizeof(double) * NZR);
     o += NZR;
   }
   return NSP_OK;
@@ -1538,23 +1534,15 @@ int nsp_cross_sections(nsp_ctx* c, int m, double* q, double* u) {
   if (!q || !u) return fail(c, NSP_ERR_ARG, "null output");
   if (!c->setup_done) return fail(c, NSP_ERR_STATE, "nsp_cross_sections before nsp_setup");
   const Group& g = c->groups[c->grp[m]];
-  const int NR = g.tb.NR, NZR = g.tb.NZR;
-  const size_t n = (size_t)2 * NR * NZR;
-  if (int rc = ensure_crossbuf(c, n)) return rc;
-  launch_diag_cross(g.tb, state_ptr(c, m, 0), c->crossbuf, c->st);
+  const size_t NZR = g.tb.NZR;
+  if (int rc = ensure_crossbuf(c, 2 * NZR + 3 * (size_t)g.tb.NR * NZR)) return rc;
+  launch_diag_cross(g.tb, state_ptr(c, m, 0), c->crossbuf + 2 * NZR, c->crossbuf, c->st);
   CK(cudaGetLastError());
-  std::vector<double> part(n);
-  CK(cudaMemcpyAsync(part.data(), c->crossbuf, n * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  std::vector<double> out(2 * NZR);
+  CK(cudaMemcpyAsync(out.data(), c->crossbuf, out.size() * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
-  for (int z = 0; z < NZR; z++) {
-    double sq = 0.0, su = 0.0;
-    for (int i = 0; i < NR; i++) {  // the radial quadrature, in level order
-      sq += part[(size_t)i * NZR + z];
-      su += part[(size_t)(NR + i) * NZR + z];
-    }
-    q[z] = sq;
-    u[z] = su;
-  }
+  memcpy(q, out.data(), sizeof(double) * NZR);
+  memcpy(u, out.data() + NZR, sizeof(double) * NZR);
   return NSP_OK;
 }
 

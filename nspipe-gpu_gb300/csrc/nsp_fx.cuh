@@ -312,4 +312,20 @@ __device__ __forceinline__ void fx_fft(cpx<fx>* buf, const int4* __restrict__ tw
   }
 }
 
+__device__ __forceinline__ double2 fx_value(const cpx<fx>& v, int E) {
+  if (E == FX_BAD) return make_double2(fx_nan(), fx_nan());
+  return make_double2(fx_to(v.x, E - FX_BITS), fx_to(v.y, E - FX_BITS));
+}
+
+// ---- kernels along z (the z stage, the cross sections)
+constexpr int MAXRZ = 6;  // register rounds of the run-time FFT
+// Threads of the z kernel: about the butterflies of a pass over its 6 RPB transforms.
+constexpr int z_threads(int nzr) { return nzr >= 576 ? 288 : nzr == 0 || nzr >= 96 ? 192 : nzr >= 54 ? 128 : 96; }
+constexpr int z_blocks(int nzr) { return nzr >= 576 ? 2 : nzr == 0 ? 1 : nzr >= 96 ? 3 : 4; }
+
+// Compiled z lengths and theta rows per block: two (three packed forward transforms for both)
+// while the six lines of each leave three blocks on an SM.
+#define NSP_NZR_LIST(X) X(24, 2) X(36, 2) X(48, 2) X(54, 2) X(72, 2) X(96, 2) X(108, 2) X(144, 2) X(162, 2) \
+  X(192, 2) X(216, 2) X(288, 2) X(384, 1) X(432, 1) X(576, 1) X(768, 1)
+
 }  // namespace nsp

@@ -160,8 +160,9 @@ void launch_fp64_peak(double* out, int blocks, int threads, int iters, cudaStrea
 // max |div u| over the interior rows -> out[0], over the wall row -> out[1] (ordered bits);
 // nmem consecutive members from U: out[2 * member + 0/1].
 void launch_diag_div(const Tables& tb, const double2* U, unsigned long long* out, cudaStream_t st, int nmem = 1);
-// Per-level partials of the q / u cross-section diagnostics: part[member][2][NR][NZR].
-void launch_diag_cross(const Tables& tb, const double2* U, double* part, cudaStream_t st, int nmem = 1);
+// The q / u cross-section diagnostics of nmem consecutive members: out[member][2][NZR]; part
+// holds the theta mean squares on the way, [member][3][NR][NZR].
+void launch_diag_cross(const Tables& tb, const double2* U, double* part, double* out, cudaStream_t st, int nmem = 1);
 // Re u_z(0,0)(r_i) of nmem consecutive members: out[member][NR].
 void launch_gather_mean(const Tables& tb, const double2* U, double* out, int nmem, cudaStream_t st);
 // Fixed device scratch of the allocation-free entry point (nsp_noalloc.cu).
@@ -178,6 +179,7 @@ int kernels_per_nonlinear();
 void launch_nonlinear_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, const double2* src, double2* dst,
                          cudaStream_t st, int mask);
 void configure_transform_fx_kernels();
+void configure_cross_kernels();
 std::vector<int4> fx_twiddles(int n);
 // z-stage kernels of a length (nsp_transform.cu): the number of two-pass splits compiled
 // for NZR (rows per block dividing NTP) in the precision, and a description of variant v.

@@ -35,16 +35,11 @@ namespace nsp {
 namespace {
 
 constexpr int MAXR = 4;   // register rounds of the run-time FFT along theta
-constexpr int MAXRZ = 6;  // ... and along z
 constexpr int TTH = 256;  // threads of the theta kernels
 
 // Columns per block of the theta kernels: 32 (512-byte rows of G) while that leaves several
 // blocks' columns in shared memory, so that a pass has about as many butterflies as threads.
 constexpr int theta_lc(int ntp) { return ntp == 0 || ntp >= 96 ? 16 : 32; }
-// Threads of the z kernel: about the butterflies of a pass over its 6 RPB transforms.
-constexpr int z_threads(int nzr) { return nzr >= 576 ? 288 : nzr == 0 || nzr >= 96 ? 192 : nzr >= 54 ? 128 : 96; }
-constexpr int z_blocks(int nzr) { return nzr >= 576 ? 2 : nzr == 0 ? 1 : nzr >= 96 ? 3 : 4; }
-
 template <int NTPC, int SIGN>
 __device__ __forceinline__ void theta_fft(cpx<fx>* buf, const Tables& tb) {
   constexpr int LC = theta_lc(NTPC);
@@ -86,11 +81,6 @@ __device__ __forceinline__ int columns_to_fx(double2* buf, int total, unsigned k
   }
   __syncthreads();
   return E;
-}
-
-__device__ __forceinline__ double2 fx_value(const cpx<fx>& v, int E) {
-  if (E == FX_BAD) return make_double2(fx_nan(), fx_nan());
-  return make_double2(fx_to(v.x, E - FX_BITS), fx_to(v.y, E - FX_BITS));
 }
 
 }  // namespace
@@ -424,8 +414,7 @@ __global__ void __launch_bounds__(TTH) fx_theta_fwd(Tables tb, Bufs bf, const Ct
 
 // ---------------------------------------------------------------- launcher
 #define NSP_NTP_LIST(X) X(12) X(18) X(24) X(36) X(48) X(54) X(72) X(96) X(144) X(192)
-#define NSP_NZR_LIST(X) X(24, 2) X(36, 2) X(48, 2) X(54, 2) X(72, 2) X(96, 2) X(108, 2) X(144, 2) X(162, 2) \
-  X(192, 2) X(216, 2) X(288, 2) X(384, 1) X(432, 1) X(576, 1) X(768, 1)
+
 
 template <int NTPC>
 static void launch_theta_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, const double2* src, double2* dst,

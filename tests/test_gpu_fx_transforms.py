@@ -51,6 +51,34 @@ def test_nonlinear_lengths(nsp, oracle_lib, NT, NZ):
     o.close()
 
 
+@pytest.mark.parametrize("NT,NZ", SHAPES)
+def test_cross_sections_lengths(nsp, NT, NZ):
+    """q and u as the theta means of the squared physical fields (numpy transforms).  Both sum
+    squares of transforms good to 1e-15 of their norm: 1e-13 relative."""
+    st = nsp.Stepper(nsp.make_params(NR, NT, NZ, Re, 0.01, LZ), precision=nsp.NSP_FP64)
+    u = rough_field(NT, NZ, 11)
+    rng = np.random.default_rng(12)
+    for a in u:  # the slots without a partner count too
+        a[:, NT // 2] = rng.standard_normal((NR, NZ)) + 1j * rng.standard_normal((NR, NZ))
+        a[:, :, NZ - 1] = rng.standard_normal((NR, NT))
+    st.set_state(0, u)
+    q, w = st.cross_sections(0)
+    rdr = st.grid(0)[1]
+    nzr = 3 * (NZ - 1)
+    e = np.exp(2j * np.pi * np.outer(np.arange(NZ), np.arange(nzr)) / nzr)
+    ms = []
+    for a in u:
+        p = 2.0 * (a[:, :, 1:] @ e[1:]) + a[:, :, :1]
+        s = p[:, 0].real ** 2 + 0.5 * np.abs(p[:, NT // 2]) ** 2
+        for mu in range(1, NT // 2):
+            s = s + 2.0 * np.abs(0.5 * (p[:, mu] + p[:, NT - mu].conj())) ** 2
+        ms.append(rdr @ s)
+    assert rel(q, ms[0] + ms[1]) < 1e-13 and rel(w, ms[2]) < 1e-13
+    qa, wa = st.cross_sections_all()
+    assert np.array_equal(qa[0], q) and np.array_equal(wa[0], w)
+    st.close()
+
+
 @pytest.mark.parametrize("NT,NZ", [(32, 65), (12, 13)])
 def test_scale(nsp, NT, NZ):
     """N is quadratic in u, so a power of two comes out exactly, but for the wall forcing of
