@@ -239,18 +239,19 @@ __global__ void __launch_bounds__(ZTH) nl_z(Tables tb, Bufs bf, const Ctl* ctl, 
 // bank conflicts; pass A of the inverse gathers the Hermitian spectra straight from
 // G.  Two shared-memory round trips per transform instead of one per radix stage.
 
-// exp(-2 pi i e / 96): every register sub-transform length used (4 .. 32) divides 96.
-__constant__ float2 c_w96f[96];
-template <typename T> __device__ __forceinline__ cpx<T> w96(int e);
-template <> __device__ __forceinline__ cpx<float> w96<float>(int e) { float2 w = c_w96f[e]; return mk<float>(w.x, w.y); }
+// exp(-2 pi i e / 288): every register sub-transform length used (4 .. 32) divides 288.
+constexpr int WN = 288;
+__constant__ float2 c_wf[WN];
+template <typename T> __device__ __forceinline__ cpx<T> wreg(int e);
+template <> __device__ __forceinline__ cpx<float> wreg<float>(int e) { float2 w = c_wf[e]; return mk<float>(w.x, w.y); }
 
-// In-register Stockham FFT of length N | 96 (every index a compile-time constant
+// In-register Stockham FFT of length N | WN (every index a compile-time constant
 // once unrolled, so the array stays in registers); natural order in and out.
 template <typename T, int SIGN, int N, int S = 0, int NS = 1>
 __device__ __forceinline__ void reg_fft(cpx<T>* v) {
   if constexpr (S < ct_nstages(N)) {
     constexpr int P = ct_radix(N, S), NB = N / P;
-    static_assert(96 % (NS * P) == 0, "sub-transform length must divide 96");
+    static_assert(WN % (NS * P) == 0, "sub-transform length must divide WN");
     cpx<T> o[N];
 #pragma unroll
     for (int j = 0; j < NB; j++) {
@@ -261,7 +262,7 @@ __device__ __forceinline__ void reg_fft(cpx<T>* v) {
       if (NS > 1 && k > 0) {
 #pragma unroll
         for (int q = 1; q < P; q++) {
-          const cpx<T> w = w96<T>((q * k * (96 / (NS * P))) % 96);
+          const cpx<T> w = wreg<T>((q * k * (WN / (NS * P))) % WN);
           x[q] = cmulv(x[q], mk<T>(w.x, SIGN > 0 ? -w.y : w.y));
         }
       }
@@ -562,11 +563,16 @@ static void launch_z2(const Tables& tb, const Bufs& bf, Ctl* dctl, bool standalo
   nl_z2<T, NZRC, N1, N2, R><<<g, Z2TH, z2_smem<T, NZRC, N1, N2, R>(), st>>>(tb, bf, dctl, standalone ? 1 : 0);
 }
 
-#define NSP_NTP_LIST(X) X(12) X(24) X(48) X(72) X(96) X(144) X(192)
+#define NSP_NTP_LIST(X) X(12) X(18) X(24) X(36) X(48) X(54) X(72) X(96) X(144) X(192)
 #define NSP_NZR_LIST(X) X(24, 2) X(48, 2) X(96, 2) X(192, 2) X(384, 2) X(576, 1) X(768, 1)
 // Two-pass z stage: (NZR, N1, N2, rows per block); the setup-time autotuner picks among
-// the splits and the radix-stage kernel per shape.
-#define NSP_Z2_LIST(X) X(24, 4, 6, 2) X(48, 8, 6, 2) X(96, 8, 12, 2) X(96, 12, 8, 2) X(192, 16, 12, 2) \
+// the splits and the radix-stage kernel per shape.  Every 2^a 3^b length up to 432 that a
+// register pass of at most 24 points splits is here: the run-time kernel, bound by its index
+// arithmetic, takes 1066 us where the 18 x 9 split takes 89 (7 members of NR=61, 36 x 54
+// modes); its theta transforms (NTP = 54) 274 and 85 us where the compiled ones take 80 and 27.
+#define NSP_Z2_LIST(X) X(24, 4, 6, 2) X(36, 6, 6, 2) X(48, 8, 6, 2) X(54, 9, 6, 2) X(72, 12, 6, 2) \
+  X(108, 9, 12, 2) X(108, 12, 9, 2) X(144, 12, 12, 2) X(162, 9, 18, 2) X(162, 18, 9, 2) X(216, 18, 12, 2) \
+  X(288, 16, 18, 2) X(288, 12, 24, 2) X(432, 18, 24, 2) X(432, 24, 18, 2) X(96, 8, 12, 2) X(96, 12, 8, 2) X(192, 16, 12, 2) \
   X(192, 12, 16, 2) X(384, 16, 24, 2) X(384, 24, 16, 2) X(576, 24, 24, 2) X(768, 32, 24, 2) X(768, 24, 32, 2)
 
 int z_variants(int NZR, int NTP, bool fp32) {
@@ -673,13 +679,13 @@ void configure_transform_kernels() {
                        (int)z2_smem<float, n, a, b, r>());
   NSP_Z2_LIST(NSP_CFG_Z2F)
 #undef NSP_CFG_Z2F
-  // Twiddles of the register sub-transforms, exp(-2 pi i e / 96), from long double.
-  float2 wf[96];
-  for (int e = 0; e < 96; e++) {
-    const long double a = -6.283185307179586476925286766559L * (long double)e / 96.0L;
+  // Twiddles of the register sub-transforms, exp(-2 pi i e / WN), from long double.
+  float2 wf[WN];
+  for (int e = 0; e < WN; e++) {
+    const long double a = -6.283185307179586476925286766559L * (long double)e / (long double)WN;
     wf[e] = make_float2((float)cosl(a), (float)sinl(a));
   }
-  cudaMemcpyToSymbol(c_w96f, wf, sizeof(wf));
+  cudaMemcpyToSymbol(c_wf, wf, sizeof(wf));
 }
 
 bool transform_supported(int NTP, int NZR) {
