@@ -30,8 +30,8 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
   cpx<fx>* Z = reinterpret_cast<cpx<fx>*>(smraw);  // [NB] lines of ZP
   __shared__ int sE[NB];
   const int NT = tb.NT, NZR = NZRC > 0 ? NZRC : tb.NZR, NZ = NZRC > 0 ? NZRC / 3 + 1 : tb.NZ;
-  const int ZP = NZRC > 0 ? fx_pad(NZRC - 1) + 1 : NZR;
-  auto at = [](int e) { return NZRC > 0 ? fx_pad(e) : e; };
+  const int ZP = NZRC > 0 ? line_pad(NZRC - 1) + 1 : NZR;
+  auto at = [](int e) { return NZRC > 0 ? line_pad(e) : e; };
   const double2* row = U + ((size_t)blockIdx.z * 3 + c) * tb.S + (size_t)i * tb.NTNZ;
   double ms[KZ];
 #pragma unroll
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
     }
     __syncthreads();
     if constexpr (NZRC > 0)
-      fx_fft<+1, NZRC, NB, 1, fx_pad(NZRC - 1) + 1, false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx);
+      pass_fft<fx, +1, NZRC, NB, 1, line_pad(NZRC - 1) + 1, false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx);
     else
       fft_batch<fx, +1, MAXRZ, false>(Z, tb.pz, NB, 1, NZR, tb.tw_zx);
     const int nb = min(NB, NT / 2 + 1 - mu0);
@@ -119,7 +119,7 @@ __global__ void cross_sum_k(Tables tb, const double* __restrict__ part, double* 
 
 template <int NZRC, int RPB>
 static void launch_cross_t(const Tables& tb, const double2* U, double* part, cudaStream_t st, int nmem) {
-  const size_t sm = sizeof(cpx<fx>) * 6 * RPB * (NZRC > 0 ? fx_pad(NZRC - 1) + 1 : tb.NZR);
+  const size_t sm = sizeof(cpx<fx>) * 6 * RPB * (NZRC > 0 ? line_pad(NZRC - 1) + 1 : tb.NZR);
   fx_cross<NZRC, RPB><<<dim3(tb.NR, 3, nmem), z_threads(NZRC), sm, st>>>(tb, U, part);
 }
 

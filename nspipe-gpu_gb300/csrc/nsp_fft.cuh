@@ -199,6 +199,162 @@ __device__ __forceinline__ void fft_ct(cpx<T>* buf, const typename vec2<T>::type
   }
 }
 
+// ---------------------------------------------------------------------------
+// Transforms of few passes: radices up to 16 with the butterflies in registers.
+
+// v exp(SIGN 2 pi i E / N) for the constants of the register transforms, N = 8, 9 or 16
+// (nsp_fx.cuh: fixed point).
+template <typename T> struct Rot {
+  template <int SIGN, int N, int E> static __device__ __forceinline__ cpx<T> by(const cpx<T>& v) {
+    constexpr T h = (T)0.70710678118654752440, c = (T)0.92387953251128675613, s = (T)0.38268343236508977173;
+    constexpr T c9[5] = {1, (T)0.76604444311897803520, (T)0.17364817766693034885, 0, (T)-0.93969262078590838405};
+    constexpr T s9[5] = {0, (T)0.64278760968653932632, (T)0.98480775301220805937, 0, (T)0.34202014332566873304};
+    constexpr int e = N == 8 ? 2 * E : E;
+    if constexpr (N == 9) return cmulv(v, mk<T>(c9[E], SIGN * s9[E]));
+    else if constexpr (e == 4) return muli<T, SIGN>(v);
+    else if constexpr (e == 2 || e == 6) {  // (+-1 + SIGN i) sqrt(1/2)
+      const cpx<T> i = muli<T, SIGN>(v), a = e == 2 ? cadd(v, i) : csub(i, v);
+      return mk<T>(h * a.x, h * a.y);
+    } else if constexpr (e == 1) return cmulv(v, mk<T>(c, SIGN * s));
+    else if constexpr (e == 3) return cmulv(v, mk<T>(s, SIGN * c));
+    else return cmulv(v, mk<T>(-c, -SIGN * s));  // e == 9
+  }
+};
+
+// P-point transform in registers, natural order: 2, 3, 4 (dft), 8 = 2 x 4, 9 = 3 x 3 and
+// 16 = 4 x 4 with constant twiddles, 6 = 2 x 3 and 12 = 3 x 4 by Good and Thomas without any.
+template <typename T, int SIGN, int P> __device__ __forceinline__ void reg_dft(cpx<T>* v) {
+  if constexpr (P <= 4) {
+    dft<T, SIGN, P>(v);
+  } else if constexpr (P == 6 || P == 12) {
+    constexpr int A = P / 3;  // 3 x A, coprime; input (A a + 3 b) mod P, output (KA a + KB b) mod P
+    constexpr int KA = 4, KB = A == 4 ? 9 : 3;
+    cpx<T> t[P];
+#pragma unroll
+    for (int b = 0; b < A; b++) {
+      cpx<T> x[3] = {v[(3 * b) % P], v[(A + 3 * b) % P], v[(2 * A + 3 * b) % P]};
+      dft<T, SIGN, 3>(x);
+#pragma unroll
+      for (int a = 0; a < 3; a++) t[a * A + b] = x[a];
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      dft<T, SIGN, A>(t + a * A);
+#pragma unroll
+      for (int b = 0; b < A; b++) v[(KA * a + KB * b) % P] = t[a * A + b];
+    }
+  } else {
+    constexpr int B = P == 8 ? 2 : P == 9 ? 3 : 4, A = P / B;  // input B a + b, output a + A b
+    cpx<T> t[B][A];
+#pragma unroll
+    for (int b = 0; b < B; b++) {
+#pragma unroll
+      for (int a = 0; a < A; a++) t[b][a] = v[B * a + b];
+      dft<T, SIGN, A>(t[b]);
+    }
+    if constexpr (P == 8) {
+      t[1][1] = Rot<T>::template by<SIGN, 8, 1>(t[1][1]);
+      t[1][2] = Rot<T>::template by<SIGN, 8, 2>(t[1][2]);
+      t[1][3] = Rot<T>::template by<SIGN, 8, 3>(t[1][3]);
+    } else if constexpr (P == 9) {
+      t[1][1] = Rot<T>::template by<SIGN, 9, 1>(t[1][1]);
+      t[1][2] = Rot<T>::template by<SIGN, 9, 2>(t[1][2]);
+      t[2][1] = Rot<T>::template by<SIGN, 9, 2>(t[2][1]);
+      t[2][2] = Rot<T>::template by<SIGN, 9, 4>(t[2][2]);
+    } else {
+      t[1][1] = Rot<T>::template by<SIGN, 16, 1>(t[1][1]);
+      t[1][2] = Rot<T>::template by<SIGN, 16, 2>(t[1][2]);
+      t[1][3] = Rot<T>::template by<SIGN, 16, 3>(t[1][3]);
+      t[2][1] = Rot<T>::template by<SIGN, 16, 2>(t[2][1]);
+      t[2][2] = Rot<T>::template by<SIGN, 16, 4>(t[2][2]);
+      t[2][3] = Rot<T>::template by<SIGN, 16, 6>(t[2][3]);
+      t[3][1] = Rot<T>::template by<SIGN, 16, 3>(t[3][1]);
+      t[3][2] = Rot<T>::template by<SIGN, 16, 6>(t[3][2]);
+      t[3][3] = Rot<T>::template by<SIGN, 16, 9>(t[3][3]);
+    }
+#pragma unroll
+    for (int a = 0; a < A; a++) {
+      cpx<T> x[B];
+#pragma unroll
+      for (int b = 0; b < B; b++) x[b] = t[b][a];
+      dft<T, SIGN, B>(x);
+#pragma unroll
+      for (int b = 0; b < B; b++) v[a + A * b] = x[b];
+    }
+  }
+}
+
+// Radices of the compiled lengths, chosen so that a transform makes few passes over
+// shared memory (two up to 192 points) with at most 16 complex values in registers;
+// 0: the length has no compiled transform.
+__host__ __device__ constexpr int pass_radix(int n, int s) {
+  constexpr int R[][4] = {{12, 12, 0, 0}, {18, 2, 9, 0}, {24, 4, 6, 0}, {36, 6, 6, 0}, {48, 6, 8, 0},
+                          {54, 6, 9, 0}, {72, 9, 8, 0}, {96, 8, 12, 0}, {108, 9, 12, 0}, {144, 12, 12, 0},
+                          {162, 9, 2, 9}, {192, 16, 12, 0}, {216, 6, 6, 6}, {288, 6, 6, 8}, {384, 8, 6, 8},
+                          {432, 6, 8, 9}, {576, 8, 8, 9}, {768, 8, 8, 12}};
+  for (const auto& r : R)
+    if (r[0] == n) return s < 3 ? r[1 + s] : 0;
+  return 0;
+}
+
+// Place of element e in a line of contiguous elements: one gap per 16 so that the strided
+// stores of a first pass spread over the banks.
+__host__ __device__ constexpr int line_pad(int e) { return e + (e >> 4); }
+
+// One Stockham pass of radix P over NB transforms of length N (see fft_stage_ct), in place:
+// element e of transform t at t BS + e ES (COLS: neighbouring threads on neighbouring
+// transforms) or at t BS + line_pad(e).  Elements [Z0, Z1] are known to be zero on the way in
+// (first pass), elements [D0, D1] not needed on the way out (last pass); empty if Z1 < Z0.
+template <typename T, int SIGN, int N, int NB, int ES, int BS, bool COLS, int NTH, int P, int NS, int Z0, int Z1, int D0, int D1>
+__device__ __forceinline__ void fft_pass(cpx<T>* buf, const typename vec2<T>::type* __restrict__ tw) {
+  constexpr int NBF = N / P, TOTAL = NB * NBF, R = (TOTAL + NTH - 1) / NTH, TSTR = N / (NS * P);
+  cpx<T> v[R][P];
+#pragma unroll
+  for (int rr = 0; rr < R; rr++) {
+    const int b = threadIdx.x + rr * NTH;
+    if (TOTAL % NTH == 0 || b < TOTAL) {
+      const int t = COLS ? b % NB : b / NBF, j = COLS ? b / NB : b - t * NBF;
+#pragma unroll
+      for (int q = 0; q < P; q++) {
+        const int e = j + q * NBF;
+        if (NS == 1 && q * NBF >= Z0 && (q + 1) * NBF - 1 <= Z1) v[rr][q] = mk<T>(0, 0);
+        else v[rr][q] = buf[t * BS + (COLS ? e * ES : line_pad(e))];
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int rr = 0; rr < R; rr++) {
+    const int b = threadIdx.x + rr * NTH;
+    if (TOTAL % NTH == 0 || b < TOTAL) {
+      const int t = COLS ? b % NB : b / NBF, j = COLS ? b / NB : b - t * NBF;
+      const int k = (NS == 1) ? 0 : j % NS;
+      if (NS > 1) {
+#pragma unroll
+        for (int q = 1; q < P; q++) v[rr][q] = twmul<T, SIGN>(v[rr][q], __ldg(tw + q * k * TSTR));
+      }
+      reg_dft<T, SIGN, P>(v[rr]);
+      const int base = (NS == 1) ? j * P : (j / NS) * NS * P + k;
+#pragma unroll
+      for (int q = 0; q < P; q++) {
+        if (NS * P == N && q * NS >= D0 && (q + 1) * NS - 1 <= D1) continue;
+        const int e = base + q * NS;
+        buf[t * BS + (COLS ? e * ES : line_pad(e))] = v[rr][q];
+      }
+    }
+  }
+  __syncthreads();
+}
+
+template <typename T, int SIGN, int N, int NB, int ES, int BS, bool COLS, int NTH, int Z0, int Z1, int D0, int D1, int S = 0, int NS = 1>
+__device__ __forceinline__ void pass_fft(cpx<T>* buf, const typename vec2<T>::type* __restrict__ tw) {
+  constexpr int P = pass_radix(N, S);
+  if constexpr (P > 0) {
+    fft_pass<T, SIGN, N, NB, ES, BS, COLS, NTH, P, NS, Z0, Z1, D0, D1>(buf, tw);
+    pass_fft<T, SIGN, N, NB, ES, BS, COLS, NTH, Z0, Z1, D0, D1, S + 1, NS * P>(buf, tw);
+  }
+}
+
 // Largest butterfly count of any stage (for the MAXR bound check on the host).
 inline int max_butterflies(const FftPlan& pl, int nb) {
   int mx = 0;

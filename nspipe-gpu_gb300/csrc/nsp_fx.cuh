@@ -162,155 +162,22 @@ template <int SIGN> __device__ __forceinline__ void dft3_fx(cpx<fx>* v) {
 }
 
 
-// v exp(SIGN 2 pi i E / N) for the constants of the register transforms, N = 8, 9 or 16.
-template <int SIGN, int N, int E> __device__ __forceinline__ cpx<fx> rotk(const cpx<fx>& v) {
-  if constexpr (N == 9) {
-    return fx_rot<SIGN>(v, E == 1 ? FX_W9_1 : E == 2 ? FX_W9_2 : FX_W9_4);
-  } else {
-    constexpr int e = N == 8 ? 2 * E : E;
-    if constexpr (e == 4) return muli<fx, SIGN>(v);
-    else if constexpr (e == 2 || e == 6) {  // (+-1 + SIGN i) sqrt(1/2)
-      const cpx<fx> i = muli<fx, SIGN>(v), a = e == 2 ? cadd(v, i) : csub(i, v);
-      return mk<fx>(fx_mulc(a.x, FX_W16_2.rh, FX_W16_2.rl), fx_mulc(a.y, FX_W16_2.rh, FX_W16_2.rl));
-    } else if constexpr (e == 1) return fx_rot<SIGN>(v, FX_W16_1);
-    else if constexpr (e == 3) return fx_cmul(v, FX_W16_1.ih, FX_W16_1.il, SIGN * FX_W16_1.rh, SIGN * FX_W16_1.rl);
-    else return fx_cmul(v, -FX_W16_1.rh, -FX_W16_1.rl, -SIGN * FX_W16_1.ih, -SIGN * FX_W16_1.il);  // e == 9
-  }
-}
-
-// P-point transform in registers, natural order: 2, 3, 4 (dft), 8 = 2 x 4, 9 = 3 x 3 and
-// 16 = 4 x 4 with constant twiddles, 6 = 2 x 3 and 12 = 3 x 4 by Good and Thomas without any.
-template <int SIGN, int P> __device__ __forceinline__ void fx_dft(cpx<fx>* v) {
-  if constexpr (P <= 4) {
-    dft<fx, SIGN, P>(v);
-  } else if constexpr (P == 6 || P == 12) {
-    constexpr int A = P / 3;  // 3 x A, coprime; input (A a + 3 b) mod P, output (KA a + KB b) mod P
-    constexpr int KA = 4, KB = A == 4 ? 9 : 3;
-    cpx<fx> t[P];
-#pragma unroll
-    for (int b = 0; b < A; b++) {
-      cpx<fx> x[3] = {v[(3 * b) % P], v[(A + 3 * b) % P], v[(2 * A + 3 * b) % P]};
-      dft<fx, SIGN, 3>(x);
-#pragma unroll
-      for (int a = 0; a < 3; a++) t[a * A + b] = x[a];
-    }
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      dft<fx, SIGN, A>(t + a * A);
-#pragma unroll
-      for (int b = 0; b < A; b++) v[(KA * a + KB * b) % P] = t[a * A + b];
-    }
-  } else {
-    constexpr int B = P == 8 ? 2 : P == 9 ? 3 : 4, A = P / B;  // input B a + b, output a + A b
-    cpx<fx> t[B][A];
-#pragma unroll
-    for (int b = 0; b < B; b++) {
-#pragma unroll
-      for (int a = 0; a < A; a++) t[b][a] = v[B * a + b];
-      dft<fx, SIGN, A>(t[b]);
-    }
-    if constexpr (P == 8) {
-      t[1][1] = rotk<SIGN, 8, 1>(t[1][1]);
-      t[1][2] = rotk<SIGN, 8, 2>(t[1][2]);
-      t[1][3] = rotk<SIGN, 8, 3>(t[1][3]);
-    } else if constexpr (P == 9) {
-      t[1][1] = rotk<SIGN, 9, 1>(t[1][1]);
-      t[1][2] = rotk<SIGN, 9, 2>(t[1][2]);
-      t[2][1] = rotk<SIGN, 9, 2>(t[2][1]);
-      t[2][2] = rotk<SIGN, 9, 4>(t[2][2]);
+template <> struct Rot<fx> {
+  template <int SIGN, int N, int E> static __device__ __forceinline__ cpx<fx> by(const cpx<fx>& v) {
+    if constexpr (N == 9) {
+      return fx_rot<SIGN>(v, E == 1 ? FX_W9_1 : E == 2 ? FX_W9_2 : FX_W9_4);
     } else {
-      t[1][1] = rotk<SIGN, 16, 1>(t[1][1]);
-      t[1][2] = rotk<SIGN, 16, 2>(t[1][2]);
-      t[1][3] = rotk<SIGN, 16, 3>(t[1][3]);
-      t[2][1] = rotk<SIGN, 16, 2>(t[2][1]);
-      t[2][2] = rotk<SIGN, 16, 4>(t[2][2]);
-      t[2][3] = rotk<SIGN, 16, 6>(t[2][3]);
-      t[3][1] = rotk<SIGN, 16, 3>(t[3][1]);
-      t[3][2] = rotk<SIGN, 16, 6>(t[3][2]);
-      t[3][3] = rotk<SIGN, 16, 9>(t[3][3]);
-    }
-#pragma unroll
-    for (int a = 0; a < A; a++) {
-      cpx<fx> x[B];
-#pragma unroll
-      for (int b = 0; b < B; b++) x[b] = t[b][a];
-      dft<fx, SIGN, B>(x);
-#pragma unroll
-      for (int b = 0; b < B; b++) v[a + A * b] = x[b];
+      constexpr int e = N == 8 ? 2 * E : E;
+      if constexpr (e == 4) return muli<fx, SIGN>(v);
+      else if constexpr (e == 2 || e == 6) {  // (+-1 + SIGN i) sqrt(1/2)
+        const cpx<fx> i = muli<fx, SIGN>(v), a = e == 2 ? cadd(v, i) : csub(i, v);
+        return mk<fx>(fx_mulc(a.x, FX_W16_2.rh, FX_W16_2.rl), fx_mulc(a.y, FX_W16_2.rh, FX_W16_2.rl));
+      } else if constexpr (e == 1) return fx_rot<SIGN>(v, FX_W16_1);
+      else if constexpr (e == 3) return fx_cmul(v, FX_W16_1.ih, FX_W16_1.il, SIGN * FX_W16_1.rh, SIGN * FX_W16_1.rl);
+      else return fx_cmul(v, -FX_W16_1.rh, -FX_W16_1.rl, -SIGN * FX_W16_1.ih, -SIGN * FX_W16_1.il);  // e == 9
     }
   }
-}
-
-// Radices of the compiled lengths, chosen so that a transform makes few passes over
-// shared memory (two up to 192 points) with at most 16 complex values in registers;
-// 0: the length has no compiled transform.
-__host__ __device__ constexpr int fx_radix(int n, int s) {
-  constexpr int R[][4] = {{12, 12, 0, 0}, {18, 2, 9, 0}, {24, 4, 6, 0}, {36, 6, 6, 0}, {48, 6, 8, 0},
-                          {54, 6, 9, 0}, {72, 9, 8, 0}, {96, 8, 12, 0}, {108, 9, 12, 0}, {144, 12, 12, 0},
-                          {162, 9, 2, 9}, {192, 16, 12, 0}, {216, 6, 6, 6}, {288, 6, 6, 8}, {384, 8, 6, 8},
-                          {432, 6, 8, 9}, {576, 8, 8, 9}, {768, 8, 8, 12}};
-  for (const auto& r : R)
-    if (r[0] == n) return s < 3 ? r[1 + s] : 0;
-  return 0;
-}
-
-// Place of element e in a line of contiguous elements: one gap per 16 so that the strided
-// stores of a first pass spread over the banks.
-__host__ __device__ constexpr int fx_pad(int e) { return e + (e >> 4); }
-
-// One Stockham pass of radix P over NB transforms of length N (see fft_stage_ct), in place:
-// element e of transform t at t BS + e ES (COLS: neighbouring threads on neighbouring
-// transforms) or at t BS + fx_pad(e).  Elements [Z0, Z1] are known to be zero on the way in
-// (first pass), elements [D0, D1] not needed on the way out (last pass); empty if Z1 < Z0.
-template <int SIGN, int N, int NB, int ES, int BS, bool COLS, int NTH, int P, int NS, int Z0, int Z1, int D0, int D1>
-__device__ __forceinline__ void fx_pass(cpx<fx>* buf, const int4* __restrict__ tw) {
-  constexpr int NBF = N / P, TOTAL = NB * NBF, R = (TOTAL + NTH - 1) / NTH, TSTR = N / (NS * P);
-  cpx<fx> v[R][P];
-#pragma unroll
-  for (int rr = 0; rr < R; rr++) {
-    const int b = threadIdx.x + rr * NTH;
-    if (TOTAL % NTH == 0 || b < TOTAL) {
-      const int t = COLS ? b % NB : b / NBF, j = COLS ? b / NB : b - t * NBF;
-#pragma unroll
-      for (int q = 0; q < P; q++) {
-        const int e = j + q * NBF;
-        if (NS == 1 && q * NBF >= Z0 && (q + 1) * NBF - 1 <= Z1) v[rr][q] = mk<fx>(0, 0);
-        else v[rr][q] = buf[t * BS + (COLS ? e * ES : fx_pad(e))];
-      }
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int rr = 0; rr < R; rr++) {
-    const int b = threadIdx.x + rr * NTH;
-    if (TOTAL % NTH == 0 || b < TOTAL) {
-      const int t = COLS ? b % NB : b / NBF, j = COLS ? b / NB : b - t * NBF;
-      const int k = (NS == 1) ? 0 : j % NS;
-      if (NS > 1) {
-#pragma unroll
-        for (int q = 1; q < P; q++) v[rr][q] = twmul<fx, SIGN>(v[rr][q], __ldg(tw + q * k * TSTR));
-      }
-      fx_dft<SIGN, P>(v[rr]);
-      const int base = (NS == 1) ? j * P : (j / NS) * NS * P + k;
-#pragma unroll
-      for (int q = 0; q < P; q++) {
-        if (NS * P == N && q * NS >= D0 && (q + 1) * NS - 1 <= D1) continue;
-        const int e = base + q * NS;
-        buf[t * BS + (COLS ? e * ES : fx_pad(e))] = v[rr][q];
-      }
-    }
-  }
-  __syncthreads();
-}
-
-template <int SIGN, int N, int NB, int ES, int BS, bool COLS, int NTH, int Z0, int Z1, int D0, int D1, int S = 0, int NS = 1>
-__device__ __forceinline__ void fx_fft(cpx<fx>* buf, const int4* __restrict__ tw) {
-  constexpr int P = fx_radix(N, S);
-  if constexpr (P > 0) {
-    fx_pass<SIGN, N, NB, ES, BS, COLS, NTH, P, NS, Z0, Z1, D0, D1>(buf, tw);
-    fx_fft<SIGN, N, NB, ES, BS, COLS, NTH, Z0, Z1, D0, D1, S + 1, NS * P>(buf, tw);
-  }
-}
+};
 
 __device__ __forceinline__ double2 fx_value(const cpx<fx>& v, int E) {
   if (E == FX_BAD) return make_double2(fx_nan(), fx_nan());

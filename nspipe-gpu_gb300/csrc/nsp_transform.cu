@@ -38,7 +38,8 @@
 namespace nsp {
 
 constexpr int MAXR = 4;   // register rounds of the run-time FFT
-constexpr int LC = 16;    // theta columns per block
+// Theta columns per block: 32 while that gives a pass about as many butterflies as threads.
+constexpr int theta_cols(int ntp) { return ntp == 0 || ntp > 108 ? 16 : 32; }
 constexpr int TTH = 256;  // threads of the theta kernels
 constexpr int ZTH = 256;  // threads of the z kernel
 constexpr int Z2TH = 192; // threads of the two-pass z kernel (its passes run 192, 144, 384, 48, 36, 384 tasks)
@@ -48,14 +49,16 @@ template <> __device__ __forceinline__ const float2* tw_t<float>(const Tables& t
 template <typename T> __device__ __forceinline__ const typename vec2<T>::type* tw_z(const Tables& tb);
 template <> __device__ __forceinline__ const float2* tw_z<float>(const Tables& tb) { return tb.tw_z32; }
 
-template <typename T, int NTPC>
-__device__ __forceinline__ void theta_fft(cpx<T>* buf, const Tables& tb, int sign) {
+template <typename T, int NTPC, int SIGN>
+__device__ __forceinline__ void theta_fft(cpx<T>* buf, const Tables& tb) {
+  constexpr int LC = theta_cols(NTPC);
   if constexpr (NTPC > 0) {
-    if (sign > 0) fft_ct<T, +1, NTPC, LC, LC, 1, true, TTH>(buf, tw_t<T>(tb));
-    else fft_ct<T, -1, NTPC, LC, LC, 1, true, TTH>(buf, tw_t<T>(tb));
+    // zero (inverse) or dropped (forward) middle third
+    constexpr int A = NTPC / 3, B = 2 * NTPC / 3 - 1;
+    if constexpr (SIGN > 0) pass_fft<T, SIGN, NTPC, LC, LC, 1, true, TTH, A, B, 0, -1>(buf, tw_t<T>(tb));
+    else pass_fft<T, SIGN, NTPC, LC, LC, 1, true, TTH, 0, -1, A, B>(buf, tw_t<T>(tb));
   } else {
-    if (sign > 0) fft_batch<T, +1, MAXR, true>(buf, tb.pt, LC, LC, 1, tw_t<T>(tb));
-    else fft_batch<T, -1, MAXR, true>(buf, tb.pt, LC, LC, 1, tw_t<T>(tb));
+    fft_batch<T, SIGN, MAXR, true>(buf, tb.pt, LC, LC, 1, tw_t<T>(tb));
   }
 }
 
@@ -63,11 +66,13 @@ __device__ __forceinline__ void theta_fft(cpx<T>* buf, const Tables& tb, int sig
 template <typename T, int NTPC>
 __global__ void __launch_bounds__(TTH) nl_theta_inv(Tables tb, Bufs bf, const Ctl* ctl, const double2* src_override,
                                                     const float2* src32_override) {
+  constexpr int LC = theta_cols(NTPC);
   const int mloc = blockIdx.z, i = blockIdx.y, c0 = blockIdx.x * LC;
   bool skip;
   member_source(tb, bf, ctl, mloc, src_override, skip);
   if (skip) return;
   const StateIn<T> U = member_input<T>(tb, bf, ctl, mloc, src_override, src32_override);
+  const float2* DR = member_dr32(tb, bf, ctl, mloc, src_override);
   extern __shared__ __align__(16) unsigned char smraw[];
   cpx<T>* buf = reinterpret_cast<cpx<T>*>(smraw);
   __shared__ int colf[LC], coll[LC];
@@ -95,6 +100,9 @@ __global__ void __launch_bounds__(TTH) nl_theta_inv(Tables tb, Bufs bf, const Ct
       size_t col = (size_t)comp * S + (size_t)it * NZ + coll[lc];
       if (f < 3) {
         v = U.ld((size_t)i * NTNZ + col);
+      } else if (f < 6 && DR) {  // the mirror the linear pass wrote (the same stencil's bits)
+        const float2 a = __ldg(DR + (size_t)i * NTNZ + col);
+        v = mk<T>(a.x, a.y);
       } else if (f < 6) {  // derivr_k, mod_radialFD.cu:10-30 (flag 1 for u_r, u_theta; 0 for u_z)
         int m = it < NT / 2 ? it : it - NT;
         int tab = abs((abs(m) % 2) - (comp < 2 ? 1 : 0));
@@ -125,7 +133,7 @@ __global__ void __launch_bounds__(TTH) nl_theta_inv(Tables tb, Bufs bf, const Ct
     buf[idx] = v;
   }
   __syncthreads();
-  theta_fft<T, NTPC>(buf, tb, +1);
+  theta_fft<T, NTPC, +1>(buf, tb);
   cpx<T>* G = reinterpret_cast<cpx<T>*>(bf.G) + (size_t)mloc * 9 * NR * NTP * NZ;
   for (int idx = threadIdx.x; idx < NTP * LC; idx += TTH) {
     int p = idx / LC, lc = idx % LC;
@@ -452,6 +460,7 @@ __global__ void __launch_bounds__(Z2TH) nl_z2(Tables tb, Bufs bf, const Ctl* ctl
 template <typename T, int NTPC>
 __global__ void __launch_bounds__(TTH) nl_theta_fwd(Tables tb, Bufs bf, const Ctl* ctl, const double2* src_override,
                                                     const float2* src32_override, double2* dst_override) {
+  constexpr int LC = theta_cols(NTPC);
   const int mloc = blockIdx.z, i = blockIdx.y, c0 = blockIdx.x * LC;
   bool skip;
   const double2* U = member_source(tb, bf, ctl, mloc, src_override, skip);
@@ -478,7 +487,7 @@ __global__ void __launch_bounds__(TTH) nl_theta_fwd(Tables tb, Bufs bf, const Ct
                                                                                                 : mk<T>(0, 0);
   }
   __syncthreads();
-  theta_fft<T, NTPC>(buf, tb, -1);
+  theta_fft<T, NTPC, -1>(buf, tb);
   // Wall derivative of u_z(0,0) for the mean forcing (pressGrad_k).
   double dwall = 0.0;
   if (c0 <= 2 * NZ && c0 + LC > 2 * NZ) {
@@ -534,6 +543,7 @@ __global__ void __launch_bounds__(TTH) nl_theta_fwd(Tables tb, Bufs bf, const Ct
 template <typename T, int NTPC>
 static void launch_theta(const Tables& tb, const Bufs& bf, Ctl* dctl, const double2* src, const float2* src32,
                          double2* dst, cudaStream_t st, int mask, int nm) {
+  constexpr int LC = theta_cols(NTPC);
   size_t sm = sizeof(cpx<T>) * tb.NTP * LC;
   if (mask & 1) {
     dim3 g((9 * tb.NZ + LC - 1) / LC, tb.NR, nm);
@@ -699,7 +709,7 @@ bool transform_supported(int NTP, int NZR) {
   FftPlan pt, pz;
   make_plan(NTP, pt);
   make_plan(NZR, pz);
-  return (ct_t || max_butterflies(pt, LC) <= MAXR * TTH) && (ct_z || max_butterflies(pz, 6) <= MAXR * ZTH);
+  return (ct_t || max_butterflies(pt, 16) <= MAXR * TTH) && (ct_z || max_butterflies(pz, 6) <= MAXR * ZTH);
 }
 
 void launch_nonlinear(const Tables& tb, const Bufs& bf, Ctl* dctl, bool mixed, const double2* src, double2* dst,

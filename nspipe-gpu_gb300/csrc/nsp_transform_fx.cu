@@ -46,8 +46,8 @@ __device__ __forceinline__ void theta_fft(cpx<fx>* buf, const Tables& tb) {
   if constexpr (NTPC > 0) {
     // zero (inverse) or dropped (forward) middle third
     constexpr int A = NTPC / 3, B = 2 * NTPC / 3 - 1;
-    if constexpr (SIGN > 0) fx_fft<SIGN, NTPC, LC, LC, 1, true, TTH, A, B, 0, -1>(buf, tb.tw_tx);
-    else fx_fft<SIGN, NTPC, LC, LC, 1, true, TTH, 0, -1, A, B>(buf, tb.tw_tx);
+    if constexpr (SIGN > 0) pass_fft<fx, SIGN, NTPC, LC, LC, 1, true, TTH, A, B, 0, -1>(buf, tb.tw_tx);
+    else pass_fft<fx, SIGN, NTPC, LC, LC, 1, true, TTH, 0, -1, A, B>(buf, tb.tw_tx);
   } else {
     fft_batch<fx, SIGN, MAXR, true>(buf, tb.pt, LC, LC, 1, tb.tw_tx);
   }
@@ -162,8 +162,8 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
   __shared__ unsigned skey[RPB * 3], ssum[RPB * 3];
   const int NR = tb.NR, NTP = tb.NTP;
   const int NZR = NZRC > 0 ? NZRC : tb.NZR, NZ = NZRC > 0 ? NZRC / 3 + 1 : tb.NZ;
-  const int ZP = NZRC > 0 ? fx_pad(NZRC - 1) + 1 : NZR;
-  auto at = [](int e) { return NZRC > 0 ? fx_pad(e) : e; };
+  const int ZP = NZRC > 0 ? line_pad(NZRC - 1) + 1 : NZR;
+  auto at = [](int e) { return NZRC > 0 ? line_pad(e) : e; };
   const double2* G = reinterpret_cast<const double2*>(bf.G) + (size_t)mloc * 9 * NR * NTP * NZ;
   double2* H = reinterpret_cast<double2*>(bf.H) + (size_t)mloc * 3 * NR * NTP * NZ;
   const int lane = threadIdx.x & 31;
@@ -255,9 +255,9 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
     for (int q = NZ + lane; q <= NZR - NZ; q += 32) Zt[at(q)] = mk<fx>(0, 0);
   }
   __syncthreads();
-  constexpr int BS = NZRC > 0 ? fx_pad(NZRC - 1) + 1 : 0;
+  constexpr int BS = NZRC > 0 ? line_pad(NZRC - 1) + 1 : 0;
   if constexpr (NZRC > 0)
-    fx_fft<+1, NZRC, RPB * 6, 1, BS, false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx);
+    pass_fft<fx, +1, NZRC, RPB * 6, 1, BS, false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx);
   else
     fft_batch<fx, +1, MAXRZ, false>(Z, tb.pz, RPB * 6, 1, NZR, tb.tw_zx);
   // -(u.grad)u (calcNonlinear_k) in FP64, packed for the forward transforms:
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
   }
   __syncthreads();
   if constexpr (NZRC > 0)
-    fx_fft<-1, NZRC, NFWD, 1, BS, false, NTH, 0, -1, NZRC / 3, 2 * NZRC / 3>(Z, tb.tw_zx);
+    pass_fft<fx, -1, NZRC, NFWD, 1, BS, false, NTH, 0, -1, NZRC / 3, 2 * NZRC / 3>(Z, tb.tw_zx);
   else
     fft_batch<fx, -1, MAXRZ, false>(Z, tb.pz, NFWD, 1, NZR, tb.tw_zx);
   // Unpack: x = a + i b  ->  A_q = (X_q + conj X_{-q})/2,  B_q = (X_q - conj X_{-q})/(2i).
@@ -429,7 +429,7 @@ static void launch_theta_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, const d
 
 template <int NZRC, int RPB>
 static void launch_z_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, bool standalone, cudaStream_t st, int nm) {
-  const size_t sm = sizeof(cpx<fx>) * 6 * RPB * (NZRC > 0 ? fx_pad(NZRC - 1) + 1 : tb.NZR);
+  const size_t sm = sizeof(cpx<fx>) * 6 * RPB * (NZRC > 0 ? line_pad(NZRC - 1) + 1 : tb.NZR);
   fx_z<NZRC, RPB><<<dim3((tb.NTP + RPB - 1) / RPB, tb.NR, nm), z_threads(NZRC), sm, st>>>(tb, bf, dctl, standalone ? 1 : 0);
 }
 
