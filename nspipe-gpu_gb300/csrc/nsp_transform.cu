@@ -63,10 +63,13 @@ __device__ __forceinline__ void theta_fft(cpx<T>* buf, const Tables& tb) {
 }
 
 // ---------------------------------------------------------------- theta inverse
+// A thread keeps one column (TTH is a multiple of LC): its field, its place in the state and
+// its twiddle-free index arithmetic are computed once.
 template <typename T, int NTPC>
 __global__ void __launch_bounds__(TTH) nl_theta_inv(Tables tb, Bufs bf, const Ctl* ctl, const double2* src_override,
                                                     const float2* src32_override) {
-  constexpr int LC = theta_cols(NTPC);
+  constexpr int LC = theta_cols(NTPC), PS = TTH / LC;
+  static_assert(TTH % LC == 0, "a thread stays on one column");
   const int mloc = blockIdx.z, i = blockIdx.y, c0 = blockIdx.x * LC;
   bool skip;
   member_source(tb, bf, ctl, mloc, src_override, skip);
@@ -75,73 +78,61 @@ __global__ void __launch_bounds__(TTH) nl_theta_inv(Tables tb, Bufs bf, const Ct
   const float2* DR = member_dr32(tb, bf, ctl, mloc, src_override);
   extern __shared__ __align__(16) unsigned char smraw[];
   cpx<T>* buf = reinterpret_cast<cpx<T>*>(smraw);
-  __shared__ int colf[LC], coll[LC];
-  const int NR = tb.NR, NT = tb.NT, NZ = tb.NZ, NTNZ = tb.NTNZ;
+  const int NR = tb.NR, NT = NTPC > 0 ? 2 * NTPC / 3 : tb.NT, NZ = tb.NZ, NTNZ = tb.NTNZ;
   const int NTP = NTPC > 0 ? NTPC : tb.NTP;
   const long long S = tb.S;
-  if (threadIdx.x < LC) {
-    int c = c0 + threadIdx.x;
-    colf[threadIdx.x] = c < 9 * NZ ? c / NZ : -1;
-    coll[threadIdx.x] = c % NZ;
-  }
-  __syncthreads();
+  const int lc = threadIdx.x % LC, c = c0 + lc, f = c < 9 * NZ ? c / NZ : -1, l = c - max(f, 0) * NZ, comp = max(f, 0) % 3;
   const int left = max(0, i - IW), right = min(i + IW, NR - 1);
   const int len = right + 1 - left, i0 = i + IW - right;
   const T rinv = tb_rinv<T>(tb, i);
   const T ktsT = tb_kts<T>(tb);
-  for (int idx = threadIdx.x; idx < NTP * LC; idx += TTH) {
-    int p = idx / LC, lc = idx % LC;
-    int f = colf[lc];
-    int it = (p < NT / 2) ? p : (p >= NT ? p - NT / 2 : -1);
+  // the padded middle third is zero
+  for (int p = NT / 2 + threadIdx.x / LC; p < NT; p += PS) buf[p * LC + lc] = mk<T>(0, 0);
+  const size_t col0 = (size_t)comp * S + l, row0 = (size_t)i * NTNZ + col0;
+  const bool live = f >= 0 && NSP_IN_BOUNDS(tb, (size_t)right * NTNZ + col0 + (size_t)(NT - 1) * NZ, 3 * S, BC_THETA_IN);
+  const bool mirror = f >= 3 && f < 6 && DR;  // d_r: the mirror the linear pass wrote (the same stencil's bits)
+  for (int it = threadIdx.x / LC; it < NT; it += PS) {
+    const int m = it < NT / 2 ? it : it - NT;
+    const unsigned off = (unsigned)it * (unsigned)NZ;
     cpx<T> v = mk<T>(0, 0);
-    if (f >= 0 && it >= 0 &&
-        NSP_IN_BOUNDS(tb, (size_t)right * NTNZ + (size_t)(f % 3) * S + (size_t)it * NZ + coll[lc], 3 * S, BC_THETA_IN)) {
-      int comp = f % 3;
-      size_t col = (size_t)comp * S + (size_t)it * NZ + coll[lc];
-      if (f < 3) {
-        v = U.ld((size_t)i * NTNZ + col);
-      } else if (f < 6 && DR) {  // the mirror the linear pass wrote (the same stencil's bits)
-        const float2 a = __ldg(DR + (size_t)i * NTNZ + col);
-        v = mk<T>(a.x, a.y);
-      } else if (f < 6) {  // derivr_k, mod_radialFD.cu:10-30 (flag 1 for u_r, u_theta; 0 for u_z)
-        int m = it < NT / 2 ? it : it - NT;
-        int tab = abs((abs(m) % 2) - (comp < 2 ? 1 : 0));
+    if (live) {
+      if (f >= 3 && f < 6 && !mirror) {  // derivr_k, mod_radialFD.cu:10-30 (flag 1 for u_r, u_theta; 0 for u_z)
+        const int tab = abs((abs(m) % 2) - (comp < 2 ? 1 : 0));
         const T* Dr = dtab<T>(tb) + tab * STEN * NR + STEN * i + i0;
         T sx = 0, sy = 0;
         for (int j = 0; j < len; j++) {
           T de = __ldg(Dr + j);
-          cpx<T> a = U.ld((size_t)(left + j) * NTNZ + col);
+          cpx<T> a = U.ld((size_t)(left + j) * NTNZ + col0 + off);
           sx += de * a.x;
           sy += de * a.y;
         }
         v = mk<T>(sx, sy);
-      } else {  // derivt_k, mod_deriv.cu:10-21
-        int m = it < NT / 2 ? it : it - NT;
-        T kt = (T)m * ktsT;
-        cpx<T> a = U.ld((size_t)i * NTNZ + col);
-        v = mk<T>(-kt * a.y * rinv, kt * a.x * rinv);
+      } else {
+        const float2 a = __ldg((mirror ? DR : U.p) + row0 + off);
+        v = mk<T>(a.x, a.y);
+        if (f >= 6) {  // derivt_k, mod_deriv.cu:10-21
+          const T kt = (T)m * ktsT;
+          v = mk<T>(-kt * a.y * rinv, kt * a.x * rinv);
+        }
       }
       // mixed form: the mean flow is recorded for the linear pass (member steps) and kept
       // out of the transforms; its terms are added by the linear pass, or for an explicit
       // field by nl_theta_fwd
-      if (it == 0 && coll[lc] == 0) {
+      if (it == 0 && l == 0) {
         const int slot = f == 0 ? MEAN_V : f == 1 ? MEAN_W : f == 2 ? MEAN_U : f == 4 ? MEAN_WP : f == 5 ? MEAN_UP : -1;
         if (!src_override && slot >= 0) bf.MEAN[((size_t)mloc * NR + i) * MEAN_N + slot] = (float)v.x;
         if (mean_field(f)) v = mk<T>(0, 0);
       }
     }
-    buf[idx] = v;
+    buf[(it < NT / 2 ? it : it + NT / 2) * LC + lc] = v;
   }
   __syncthreads();
   theta_fft<T, NTPC, +1>(buf, tb);
-  cpx<T>* G = reinterpret_cast<cpx<T>*>(bf.G) + (size_t)mloc * 9 * NR * NTP * NZ;
-  for (int idx = threadIdx.x; idx < NTP * LC; idx += TTH) {
-    int p = idx / LC, lc = idx % LC;
-    int f = colf[lc];
-    if (f >= 0 && NSP_IN_BOUNDS(tb, (((size_t)f * NR + i) * NTP + p) * NZ + coll[lc], (size_t)9 * NR * NTP * NZ,
-                                BC_THETA_OUT))
-      G[(((size_t)f * NR + i) * NTP + p) * NZ + coll[lc]] = buf[idx];
-  }
+  if (f < 0) return;
+  const size_t g0 = (((size_t)f * NR + i) * NTP) * NZ + l;
+  if (!NSP_IN_BOUNDS(tb, g0 + (size_t)(NTP - 1) * NZ, (size_t)9 * NR * NTP * NZ, BC_THETA_OUT)) return;
+  cpx<T>* G = reinterpret_cast<cpx<T>*>(bf.G) + (size_t)mloc * 9 * NR * NTP * NZ + g0;
+  for (int p = threadIdx.x / LC; p < NTP; p += PS) G[(size_t)p * NZ] = buf[p * LC + lc];
 }
 
 // ---------------------------------------------------------------- z stage
@@ -460,82 +451,68 @@ __global__ void __launch_bounds__(Z2TH) nl_z2(Tables tb, Bufs bf, const Ctl* ctl
 template <typename T, int NTPC>
 __global__ void __launch_bounds__(TTH) nl_theta_fwd(Tables tb, Bufs bf, const Ctl* ctl, const double2* src_override,
                                                     const float2* src32_override, double2* dst_override) {
-  constexpr int LC = theta_cols(NTPC);
+  constexpr int LC = theta_cols(NTPC), PS = TTH / LC;
   const int mloc = blockIdx.z, i = blockIdx.y, c0 = blockIdx.x * LC;
   bool skip;
   const double2* U = member_source(tb, bf, ctl, mloc, src_override, skip);
   if (skip) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   cpx<T>* buf = reinterpret_cast<cpx<T>*>(smraw);
-  __shared__ int colc[LC], coll[LC];
-  const int NR = tb.NR, NT = tb.NT, NZ = tb.NZ, NTNZ = tb.NTNZ;
+  const int NR = tb.NR, NT = NTPC > 0 ? 2 * NTPC / 3 : tb.NT, NZ = tb.NZ, NTNZ = tb.NTNZ;
   const int NTP = NTPC > 0 ? NTPC : tb.NTP;
   const long long S = tb.S;
-  if (threadIdx.x < LC) {
-    int c = c0 + threadIdx.x;
-    colc[threadIdx.x] = c < 3 * NZ ? c / NZ : -1;
-    coll[threadIdx.x] = c % NZ;
-  }
-  __syncthreads();
-  const cpx<T>* H = reinterpret_cast<const cpx<T>*>(bf.H) + (size_t)mloc * 3 * NR * NTP * NZ;
-  double2* Nout = dst_override ? dst_override : (bf.N ? bf.N + (size_t)mloc * 3 * S : nullptr);  // (null: mixed, N32)
-  for (int idx = threadIdx.x; idx < NTP * LC; idx += TTH) {
-    int p = idx / LC, lc = idx % LC;
-    int c = colc[lc], l = coll[lc];
-    const size_t hi = (((size_t)c * NR + i) * NTP + p) * NZ + l;
-    buf[idx] = (c >= 0 && l < NZ - 1 && NSP_IN_BOUNDS(tb, hi, (size_t)3 * NR * NTP * NZ, BC_THETA_IN)) ? H[hi]
-                                                                                                : mk<T>(0, 0);
-  }
+  const int lc = threadIdx.x % LC, q = c0 + lc, c = q < 3 * NZ ? q / NZ : -1, l = q - max(c, 0) * NZ;
+  const size_t h0 = (((size_t)max(c, 0) * NR + i) * NTP) * NZ + l;
+  const cpx<T>* H = reinterpret_cast<const cpx<T>*>(bf.H) + (size_t)mloc * 3 * NR * NTP * NZ + h0;
+  const bool live = c >= 0 && l < NZ - 1 &&
+                    NSP_IN_BOUNDS(tb, h0 + (size_t)(NTP - 1) * NZ, (size_t)3 * NR * NTP * NZ, BC_THETA_IN);
+  for (int p = threadIdx.x / LC; p < NTP; p += PS) buf[p * LC + lc] = live ? H[(size_t)p * NZ] : mk<T>(0, 0);
   __syncthreads();
   theta_fft<T, NTPC, -1>(buf, tb);
+  if (c < 0) return;
   // Wall derivative of u_z(0,0) for the mean forcing (pressGrad_k).
   double dwall = 0.0;
-  if (c0 <= 2 * NZ && c0 + LC > 2 * NZ) {
+  if (c == 2 && l == 0) {
     const double* Dw = tb.D + STEN * (NR - 1) + IW;
     for (int j = 0; j <= IW; j++) dwall += Dw[j] * U[2 * S + (size_t)(NR - 1 - IW + j) * NTNZ].x;
   }
   const T scale = tb_inv_norm<T>(tb);
-  // mixed form, explicit field: the mean-flow terms (nsp_state.cuh), from its FP32 copy
-  const float2* U32 = nullptr;
-  Mean32 mf{};
-  if (src_override) {  // a member state's terms are added by the linear pass
-    U32 = src32_override;
-    mf = mean_flow32(tb, U32, nullptr, i);
-  }
-  for (int idx = threadIdx.x; idx < NT * LC; idx += TTH) {
-    int it = idx / LC, lc = idx % LC;
-    int c = colc[lc], l = coll[lc];
-    if (c < 0) continue;
-    int p = it < NT / 2 ? it : NTP + it - NT;
-    cpx<T> b = buf[p * LC + lc];
-    double2 v;
-    if (!dst_override) {
-      // a member's N in the mixed form: FP32 (its values are FP32 numbers), the wall forcing
-      // of Re N_z(0,0) kept apart in FP64 -- the same at every level, written by level 0
-      const bool drop = it == NT / 2 || l == NZ - 1;
-      const size_t e = c * S + (size_t)i * NTNZ + (size_t)it * NZ + l;
-      if (c == 2 && it == 0 && l == 0 && i == 0) bf.NF[mloc] = -(tb.sscal[4 * member_set(tb, mloc) + 1] * dwall);
-      if (NSP_IN_BOUNDS(tb, e, 3 * S, BC_THETA_OUT))
-        bf.N32[(size_t)mloc * 3 * S + e] = drop ? make_float2(0.f, 0.f) : make_float2(b.x * scale, b.y * scale);
-      continue;
-    } else {
-      float2 w = make_float2(b.x * scale, b.y * scale);
-      if (U32 && it != NT / 2 && l != NZ - 1) {
-        const bool zm = it == 0 && l == 0;
-        const size_t hq = (size_t)i * NTNZ + (size_t)it * NZ + l;
-        const float2 ur = U32[hq], uq = zm ? make_float2(0.f, 0.f) : U32[(c == 2 ? 2 : 1) * S + hq];
-        const float kt = (float)(it < NT / 2 ? it : it - NT) * tb.kts32;
-        const float2 ml = mean_terms32(mf, c, zm, kt, tb.kzs32 * (float)l, ur, c < 2 ? uq : make_float2(0.f, 0.f),
-                                       c == 2 ? uq : make_float2(0.f, 0.f));
-        w.x += ml.x;
-        w.y += ml.y;
-      }
-      v = make_double2(f32_to_f64(w.x), f32_to_f64(w.y));  // exact, integer pipe
+  const size_t e0 = (size_t)c * S + (size_t)i * NTNZ + l;
+  if (!NSP_IN_BOUNDS(tb, e0 + (size_t)(NT - 1) * NZ, 3 * S, BC_THETA_OUT)) return;
+  if (!dst_override) {
+    // a member's N in the mixed form: FP32 (its values are FP32 numbers), the wall forcing
+    // of Re N_z(0,0) kept apart in FP64 -- the same at every level, written by level 0
+    if (c == 2 && l == 0 && i == 0 && threadIdx.x < LC) bf.NF[mloc] = -(tb.sscal[4 * member_set(tb, mloc) + 1] * dwall);
+    float2* N32 = bf.N32 + (size_t)mloc * 3 * S + e0;
+    for (int it = threadIdx.x / LC; it < NT; it += PS) {
+      const cpx<T> b = buf[(it < NT / 2 ? it : NTP + it - NT) * LC + lc];
+      N32[(size_t)it * NZ] = it == NT / 2 || l == NZ - 1 ? make_float2(0.f, 0.f) : make_float2(b.x * scale, b.y * scale);
     }
+    return;
+  }
+  // explicit field: the mean-flow terms (nsp_state.cuh), from its FP32 copy (a member state's
+  // terms are added by the linear pass)
+  const float2* U32 = src_override ? src32_override : nullptr;
+  Mean32 mf{};
+  if (U32) mf = mean_flow32(tb, U32, nullptr, i);
+  double2* Nout = dst_override + e0;
+  for (int it = threadIdx.x / LC; it < NT; it += PS) {
+    const cpx<T> b = buf[(it < NT / 2 ? it : NTP + it - NT) * LC + lc];
+    float2 w = make_float2(b.x * scale, b.y * scale);
+    if (U32 && it != NT / 2 && l != NZ - 1) {
+      const bool zm = it == 0 && l == 0;
+      const size_t hq = (size_t)i * NTNZ + (size_t)it * NZ + l;
+      const float2 ur = U32[hq], uq = zm ? make_float2(0.f, 0.f) : U32[(c == 2 ? 2 : 1) * S + hq];
+      const float kt = (float)(it < NT / 2 ? it : it - NT) * tb.kts32;
+      const float2 ml = mean_terms32(mf, c, zm, kt, tb.kzs32 * (float)l, ur, c < 2 ? uq : make_float2(0.f, 0.f),
+                                     c == 2 ? uq : make_float2(0.f, 0.f));
+      w.x += ml.x;
+      w.y += ml.y;
+    }
+    double2 v = make_double2(f32_to_f64(w.x), f32_to_f64(w.y));  // exact, integer pipe
     if (it == NT / 2 || l == NZ - 1) v = make_double2(0.0, 0.0);
     if (c == 2 && it == 0 && l == 0) v.x -= tb.sscal[4 * member_set(tb, mloc) + 1] * dwall;  // 2/Re
-    if (NSP_IN_BOUNDS(tb, c * S + (size_t)i * NTNZ + (size_t)it * NZ + l, 3 * S, BC_THETA_OUT))
-      Nout[c * S + (size_t)i * NTNZ + (size_t)it * NZ + l] = v;
+    Nout[(size_t)it * NZ] = v;
   }
 }
 
@@ -573,7 +550,7 @@ static void launch_z2(const Tables& tb, const Bufs& bf, Ctl* dctl, bool standalo
   nl_z2<T, NZRC, N1, N2, R><<<g, Z2TH, z2_smem<T, NZRC, N1, N2, R>(), st>>>(tb, bf, dctl, standalone ? 1 : 0);
 }
 
-#define NSP_NTP_LIST(X) X(12) X(18) X(24) X(36) X(48) X(54) X(72) X(96) X(144) X(192)
+#define NSP_NTP_LIST(X) X(12) X(18) X(24) X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(192)
 #define NSP_NZR_LIST(X) X(24, 2) X(48, 2) X(96, 2) X(192, 2) X(384, 2) X(576, 1) X(768, 1)
 // Two-pass z stage: (NZR, N1, N2, rows per block); the setup-time autotuner picks among
 // the splits and the radix-stage kernel per shape.  Every 2^a 3^b length up to 432 that a

@@ -53,9 +53,29 @@ __device__ __forceinline__ void theta_fft(cpx<fx>* buf, const Tables& tb) {
   }
 }
 
-// The block's columns, in FP64 at buf (element p of column lc at p LC + lc, thread t holding
-// the elements t + k TTH of column t % LC), to fixed point in place; kmax: the thread's
-// largest key.  skey / ssum: zeroed shared arrays of LC.  Returns the column's exponent.
+// Scale of a column whose V values per thread (threads t and t + LC, t + 2 LC ... hold one
+// column) are in registers: its exponent, from its largest key and its sum of magnitudes.
+// skey / ssum: zeroed shared arrays of LC.
+template <int LC, int V>
+__device__ __forceinline__ int column_exponent(const double2 (&g)[V], unsigned* skey, unsigned* ssum) {
+  const int lc = threadIdx.x % LC;
+  unsigned kmax = 0u, sum = 0u;
+#pragma unroll
+  for (int k = 0; k < V; k++) kmax = max(kmax, max(fx_key(g[k].x), fx_key(g[k].y)));
+  if (LC < 32) kmax = max(kmax, __shfl_xor_sync(0xFFFFFFFFu, kmax, LC));
+  if ((threadIdx.x & 31) < LC) atomicMax(skey + lc, kmax);
+  __syncthreads();
+  kmax = skey[lc];
+#pragma unroll
+  for (int k = 0; k < V; k++) sum += fx_mag(fx_key(g[k].x), kmax >> 20) + fx_mag(fx_key(g[k].y), kmax >> 20);
+  if (LC < 32) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, LC);
+  if ((threadIdx.x & 31) < LC) atomicAdd(ssum + lc, sum);
+  __syncthreads();
+  return fx_exponent(kmax, ssum[lc]);
+}
+
+// The same for a run-time length: the block's columns, in FP64 at buf (element p of column
+// lc at p LC + lc), to fixed point in place; kmax: the thread's largest key.
 template <int LC>
 __device__ __forceinline__ int columns_to_fx(double2* buf, int total, unsigned kmax, unsigned* skey, unsigned* ssum) {
   const int lc = threadIdx.x % LC;
@@ -67,8 +87,7 @@ __device__ __forceinline__ int columns_to_fx(double2* buf, int total, unsigned k
   unsigned sum = 0;
   for (int idx = threadIdx.x; idx < total; idx += TTH) {
     const double2 v = buf[idx];
-    const unsigned kx = fx_key(v.x), ky = fx_key(v.y);
-    if (kx | ky) sum += fx_mag(kx, emax) + fx_mag(ky, emax);
+    sum += fx_mag(fx_key(v.x), emax) + fx_mag(fx_key(v.y), emax);
   }
   if (LC < 32) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, LC);
   if ((threadIdx.x & 31) < LC) atomicAdd(ssum + lc, sum);
@@ -96,7 +115,7 @@ __global__ void __launch_bounds__(TTH) fx_theta_inv(Tables tb, Bufs bf, const Ct
   double2* buf = reinterpret_cast<double2*>(smraw);
   constexpr int LC = theta_lc(NTPC);
   __shared__ unsigned skey[LC], ssum[LC];
-  const int NR = tb.NR, NT = tb.NT, NZ = tb.NZ, NTNZ = tb.NTNZ;
+  const int NR = tb.NR, NT = NTPC > 0 ? 2 * NTPC / 3 : tb.NT, NZ = tb.NZ, NTNZ = tb.NTNZ;
   const int NTP = NTPC > 0 ? NTPC : tb.NTP;
   const long long S = tb.S;
   const int lc = threadIdx.x % LC, c = c0 + lc;
@@ -106,44 +125,67 @@ __global__ void __launch_bounds__(TTH) fx_theta_inv(Tables tb, Bufs bf, const Ct
   const int left = max(0, i - IW), right = min(i + IW, NR - 1);
   const int len = right + 1 - left, i0 = i + IW - right;
   const double rinv = tb.rinv[i];
-  unsigned kmax = 0u;
-  for (int idx = threadIdx.x; idx < NTP * LC; idx += TTH) {
-    const int p = idx / LC;
-    const int it = (p < NT / 2) ? p : (p >= NT ? p - NT / 2 : -1);
+  const size_t col0 = (size_t)max(f, 0) % 3 * S + l;
+  const bool live = f >= 0 && NSP_IN_BOUNDS(tb, (size_t)right * NTNZ + col0 + (size_t)(NT - 1) * NZ, 3 * S, BC_THETA_IN);
+  auto value = [&](int it) {
     double2 v = make_double2(0.0, 0.0);
-    if (f >= 0 && it >= 0 &&
-        NSP_IN_BOUNDS(tb, (size_t)right * NTNZ + (size_t)(f % 3) * S + (size_t)it * NZ + l, 3 * S, BC_THETA_IN)) {
-      const int comp = f % 3, m = it < NT / 2 ? it : it - NT;
-      const double2* col = U + (size_t)comp * S + (size_t)it * NZ + l;
-      if (f < 3) {
-        v = col[(size_t)i * NTNZ];
-      } else if (f < 6) {  // derivr_k, mod_radialFD.cu:10-30 (flag 1 for u_r, u_theta; 0 for u_z)
-        const int tab = abs((abs(m) % 2) - (comp < 2 ? 1 : 0));
-        const double* Dr = tb.D + tab * STEN * NR + STEN * i + i0;
-        for (int j = 0; j < len; j++) {
-          const double de = __ldg(Dr + j);
-          const double2 a = col[(size_t)(left + j) * NTNZ];
-          v.x += de * a.x;
-          v.y += de * a.y;
-        }
-      } else {  // derivt_k, mod_deriv.cu:10-21
+    if (!live) return v;
+    const int m = it < NT / 2 ? it : it - NT;
+    const double2* col = U + col0 + (unsigned)it * (unsigned)NZ;
+    if (f >= 3 && f < 6) {  // derivr_k, mod_radialFD.cu:10-30 (flag 1 for u_r, u_theta; 0 for u_z)
+      const int tab = abs((abs(m) % 2) - (f < 5 ? 1 : 0));
+      const double* Dr = tb.D + tab * STEN * NR + STEN * i + i0;
+      for (int j = 0; j < len; j++) {
+        const double de = __ldg(Dr + j);
+        const double2 a = col[(size_t)(left + j) * NTNZ];
+        v.x += de * a.x;
+        v.y += de * a.y;
+      }
+    } else {
+      v = col[(size_t)i * NTNZ];
+      if (f >= 6) {  // derivt_k, mod_deriv.cu:10-21
         const double kt = tb.kts * (double)m;
-        const double2 a = col[(size_t)i * NTNZ];
-        v = make_double2(-kt * a.y * rinv, kt * a.x * rinv);
+        v = make_double2(-kt * v.y * rinv, kt * v.x * rinv);
       }
     }
-    kmax = max(kmax, max(fx_key(v.x), fx_key(v.y)));
-    buf[idx] = v;
-  }
-  const int E = columns_to_fx<LC>(buf, NTP * LC, kmax, skey, ssum);
+    return v;
+  };
+  // the padded middle third is zero
   cpx<fx>* X = reinterpret_cast<cpx<fx>*>(buf);
-  theta_fft<NTPC, +1>(X, tb);
-  double2* G = reinterpret_cast<double2*>(bf.G) + (size_t)mloc * 9 * NR * NTP * NZ;
-  if (f < 0) return;
-  for (int idx = threadIdx.x; idx < NTP * LC; idx += TTH) {
-    const size_t g = (((size_t)f * NR + i) * NTP + idx / LC) * NZ + l;
-    if (NSP_IN_BOUNDS(tb, g, (size_t)9 * NR * NTP * NZ, BC_THETA_OUT)) G[g] = fx_value(X[idx], E);
+  constexpr int PS = TTH / LC;
+  const int t0 = threadIdx.x / LC;
+  for (int p = NT / 2 + t0; p < NT; p += PS) X[p * LC + lc] = mk<fx>(0, 0);
+  int E;
+  if constexpr (NTPC > 0) {
+    constexpr int V = (2 * NTPC / 3 + PS - 1) / PS;
+    double2 g[V];
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      const int it = t0 + k * PS;
+      g[k] = it < NT ? value(it) : make_double2(0.0, 0.0);
+    }
+    E = column_exponent<LC, V>(g, skey, ssum);
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      const int it = t0 + k * PS;
+      if (it < NT) X[(it < NT / 2 ? it : it + NT / 2) * LC + lc] = mk<fx>(fx_from(g[k].x, E), fx_from(g[k].y, E));
+    }
+    __syncthreads();
+  } else {
+    unsigned kmax = 0u;
+    for (int it = t0; it < NT; it += PS) {
+      const double2 v = value(it);
+      kmax = max(kmax, max(fx_key(v.x), fx_key(v.y)));
+      buf[(it < NT / 2 ? it : it + NT / 2) * LC + lc] = v;
+    }
+    E = columns_to_fx<LC>(buf, NTP * LC, kmax, skey, ssum);
   }
+  theta_fft<NTPC, +1>(X, tb);
+  if (f < 0) return;
+  const size_t g0 = (((size_t)f * NR + i) * NTP) * NZ + l;
+  if (!NSP_IN_BOUNDS(tb, g0 + (size_t)(NTP - 1) * NZ, (size_t)9 * NR * NTP * NZ, BC_THETA_OUT)) return;
+  double2* G = reinterpret_cast<double2*>(bf.G) + (size_t)mloc * 9 * NR * NTP * NZ + g0;
+  for (int p = t0; p < NTP; p += PS) G[(unsigned)p * (unsigned)NZ] = fx_value(X[p * LC + lc], E);
 }
 
 // ---------------------------------------------------------------- z stage
@@ -373,25 +415,44 @@ __global__ void __launch_bounds__(TTH) fx_theta_fwd(Tables tb, Bufs bf, const Ct
   double2* buf = reinterpret_cast<double2*>(smraw);
   constexpr int LC = theta_lc(NTPC);
   __shared__ unsigned skey[LC], ssum[LC];
-  const int NR = tb.NR, NT = tb.NT, NZ = tb.NZ, NTNZ = tb.NTNZ;
+  const int NR = tb.NR, NT = NTPC > 0 ? 2 * NTPC / 3 : tb.NT, NZ = tb.NZ, NTNZ = tb.NTNZ;
   const int NTP = NTPC > 0 ? NTPC : tb.NTP;
   const long long S = tb.S;
   const int lc = threadIdx.x % LC, q = c0 + lc;
   const int c = q < 3 * NZ ? q / NZ : -1, l = q % NZ;
   if (threadIdx.x < LC) skey[threadIdx.x] = ssum[threadIdx.x] = 0u;
   __syncthreads();
-  const double2* H = reinterpret_cast<const double2*>(bf.H) + (size_t)mloc * 3 * NR * NTP * NZ;
+  const size_t h0 = (((size_t)max(c, 0) * NR + i) * NTP) * NZ + l;
+  const double2* H = reinterpret_cast<const double2*>(bf.H) + (size_t)mloc * 3 * NR * NTP * NZ + h0;
+  const bool live = c >= 0 && l < NZ - 1 &&
+                    NSP_IN_BOUNDS(tb, h0 + (size_t)(NTP - 1) * NZ, (size_t)3 * NR * NTP * NZ, BC_THETA_IN);
   double2* Nout = dst_override ? dst_override : bf.N + (size_t)mloc * 3 * S;
-  unsigned kmax = 0u;
-  for (int idx = threadIdx.x; idx < NTP * LC; idx += TTH) {
-    const size_t hi = (((size_t)c * NR + i) * NTP + idx / LC) * NZ + l;
-    const double2 v = (c >= 0 && l < NZ - 1 && NSP_IN_BOUNDS(tb, hi, (size_t)3 * NR * NTP * NZ, BC_THETA_IN))
-                          ? H[hi] : make_double2(0.0, 0.0);
-    kmax = max(kmax, max(fx_key(v.x), fx_key(v.y)));
-    buf[idx] = v;
-  }
-  const int E = columns_to_fx<LC>(buf, NTP * LC, kmax, skey, ssum);
   cpx<fx>* X = reinterpret_cast<cpx<fx>*>(buf);
+  constexpr int PS = TTH / LC;
+  const int t0 = threadIdx.x / LC;
+  int E;
+  if constexpr (NTPC > 0) {
+    constexpr int V = (NTPC + PS - 1) / PS;
+    double2 g[V];
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      const int p = t0 + k * PS;
+      g[k] = live && p < NTP ? H[(unsigned)p * (unsigned)NZ] : make_double2(0.0, 0.0);
+    }
+    E = column_exponent<LC, V>(g, skey, ssum);
+#pragma unroll
+    for (int k = 0; k < V; k++)
+      if (t0 + k * PS < NTP) X[(t0 + k * PS) * LC + lc] = mk<fx>(fx_from(g[k].x, E), fx_from(g[k].y, E));
+    __syncthreads();
+  } else {
+    unsigned kmax = 0u;
+    for (int p = t0; p < NTP; p += PS) {
+      const double2 v = live ? H[(unsigned)p * (unsigned)NZ] : make_double2(0.0, 0.0);
+      kmax = max(kmax, max(fx_key(v.x), fx_key(v.y)));
+      buf[p * LC + lc] = v;
+    }
+    E = columns_to_fx<LC>(buf, NTP * LC, kmax, skey, ssum);
+  }
   theta_fft<NTPC, -1>(X, tb);
   if (c < 0) return;
   // Wall derivative of u_z(0,0) for the mean forcing (pressGrad_k).
@@ -413,7 +474,7 @@ __global__ void __launch_bounds__(TTH) fx_theta_fwd(Tables tb, Bufs bf, const Ct
 }
 
 // ---------------------------------------------------------------- launcher
-#define NSP_NTP_LIST(X) X(12) X(18) X(24) X(36) X(48) X(54) X(72) X(96) X(144) X(192)
+#define NSP_NTP_LIST(X) X(12) X(18) X(24) X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(192)
 
 
 template <int NTPC>
