@@ -30,8 +30,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
   cpx<fx>* Z = reinterpret_cast<cpx<fx>*>(smraw);  // [NB] lines of ZP
   __shared__ int sE[NB];
   const int NT = tb.NT, NZR = NZRC > 0 ? NZRC : tb.NZR, NZ = NZRC > 0 ? NZRC / 3 + 1 : tb.NZ;
-  const int ZP = NZRC > 0 ? line_pad(NZRC - 1) + 1 : NZR;
-  auto at = [](int e) { return NZRC > 0 ? line_pad(e) : e; };
+  const int ZP = NZRC > 0 ? line_pitch(NZRC) : NZR;
   const double2* row = U + ((size_t)blockIdx.z * 3 + c) * tb.S + (size_t)i * tb.NTNZ;
   double ms[KZ];
 #pragma unroll
@@ -41,43 +40,36 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
       const int mu = mu0 + b;
       cpx<fx>* Zt = Z + (size_t)b * ZP;
       if (mu > NT / 2) {
-        for (int q = lane; q < NZR; q += 32) Zt[at(q)] = mk<fx>(0, 0);
+        for (int q = lane; q < NZR; q += 32) Zt[q] = mk<fx>(0, 0);
         continue;
       }
       const double2* P = row + (size_t)mu * NZ;
       const double2* M = row + (size_t)(mu ? NT - mu : 0) * NZ;  // (mu = NT/2: the same line, unused)
       const bool pair = mu < NT / 2;
-      unsigned kmax = 0u, sum = 0u;
+      FxSum sum;
       for (int q = lane; q < NZ; q += 32) {
         const double2 a = P[q], m = M[q];
-        kmax = max(max(kmax, max(fx_key(a.x), fx_key(a.y))), max(fx_key(m.x), fx_key(m.y)));
+        sum.add(fx_key(a.x), fx_key(a.y));
+        if (pair) sum.add(fx_key(m.x), fx_key(m.y));
       }
-      kmax = __reduce_max_sync(0xFFFFFFFFu, kmax);
-      for (int q = lane; q < NZ; q += 32) {
-        const double2 a = P[q], m = M[q];
-        const unsigned e = kmax >> 20;
-        sum += fx_mag(fx_key(a.x), e) + fx_mag(fx_key(a.y), e);
-        if (pair) sum += fx_mag(fx_key(m.x), e) + fx_mag(fx_key(m.y), e);
-      }
-      sum = __reduce_add_sync(0xFFFFFFFFu, sum);
-      const int E = fx_exponent(kmax, sum);
+      const int E = sum.warp_exponent();
       if (lane == 0) sE[b] = E;
       for (int q = lane; q < NZ; q += 32) {
         const double2 a = P[q], m = M[q];
         const cpx<fx> x = mk<fx>(fx_from(a.x, E), fx_from(a.y, E));
         const cpx<fx> y = pair ? mk<fx>(fx_from(m.x, E), -fx_from(m.y, E)) : mk<fx>(0, 0);
         if (q) {
-          Zt[at(q)] = x;
-          Zt[at(NZR - q)] = y;
+          Zt[q] = x;
+          Zt[NZR - q] = y;
         } else {
           Zt[0] = mk<fx>(fx_half(x.x + y.x), fx_half(x.y + y.y));
         }
       }
-      for (int q = NZ + lane; q <= NZR - NZ; q += 32) Zt[at(q)] = mk<fx>(0, 0);
+      for (int q = NZ + lane; q <= NZR - NZ; q += 32) Zt[q] = mk<fx>(0, 0);
     }
     __syncthreads();
     if constexpr (NZRC > 0)
-      pass_fft<fx, +1, NZRC, NB, 1, line_pad(NZRC - 1) + 1, false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx);
+      pass_fft<fx, +1, NZRC, NB, 1, line_pitch(NZRC), false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx);
     else
       fft_batch<fx, +1, MAXRZ, false>(Z, tb.pz, NB, 1, NZR, tb.tw_zx);
     const int nb = min(NB, NT / 2 + 1 - mu0);
@@ -86,7 +78,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
       const int n = threadIdx.x + k * NTH;
       if (n < NZR)
         for (int b = 0; b < nb; b++) {
-          const double2 v = fx_value(Z[(size_t)b * ZP + at(n)], sE[b]);
+          const double2 v = fx_value(Z[(size_t)b * ZP + n], sE[b]);
           if (mu0 + b == 0) ms[k] = v.x * v.x;
           else ms[k] += 2.0 * (v.x * v.x + v.y * v.y);
         }
@@ -119,7 +111,7 @@ __global__ void cross_sum_k(Tables tb, const double* __restrict__ part, double* 
 
 template <int NZRC, int RPB>
 static void launch_cross_t(const Tables& tb, const double2* U, double* part, cudaStream_t st, int nmem) {
-  const size_t sm = sizeof(cpx<fx>) * 6 * RPB * (NZRC > 0 ? line_pad(NZRC - 1) + 1 : tb.NZR);
+  const size_t sm = sizeof(cpx<fx>) * 6 * RPB * (NZRC > 0 ? line_pitch(NZRC) : tb.NZR);
   fx_cross<NZRC, RPB><<<dim3(tb.NR, 3, nmem), z_threads(NZRC), sm, st>>>(tb, U, part);
 }
 

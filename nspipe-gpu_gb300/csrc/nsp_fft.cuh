@@ -70,6 +70,11 @@ template <typename T, int SIGN, int P> __device__ __forceinline__ void dft(cpx<T
   }
 }
 
+// Groups of asynchronous global -> shared copies (cp.async) and their waits.
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
 // One Stockham stage over nb transforms of length n.  Element e of transform t
 // lives at buf[t*bs + e*es].  TFAST: consecutive threads take consecutive
 // transforms (for element-strided layouts), else consecutive butterflies.
@@ -284,26 +289,48 @@ template <typename T, int SIGN, int P> __device__ __forceinline__ void reg_dft(c
   }
 }
 
-// Radices of the compiled lengths, chosen so that a transform makes few passes over
-// shared memory (two up to 192 points) with at most 16 complex values in registers;
-// 0: the length has no compiled transform.
-__host__ __device__ constexpr int pass_radix(int n, int s) {
-  constexpr int R[][4] = {{12, 12, 0, 0}, {18, 2, 9, 0}, {24, 4, 6, 0}, {36, 6, 6, 0}, {48, 6, 8, 0},
-                          {54, 6, 9, 0}, {72, 9, 8, 0}, {96, 8, 12, 0}, {108, 9, 12, 0}, {144, 12, 12, 0},
-                          {162, 9, 2, 9}, {192, 16, 12, 0}, {216, 6, 6, 6}, {288, 6, 6, 8}, {384, 8, 6, 8},
-                          {432, 6, 8, 9}, {576, 8, 8, 9}, {768, 8, 8, 12}};
+// Radices of the compiled lengths: few passes over shared memory, with few enough complex
+// values in registers for the kernels' blocks per SM (nsp_fx.cuh: at 192 points 8 x 4 x 6 takes
+// 665, 16 x 12 733 ns per member and mode); 0: the length has no compiled transform.  (768:
+// 8 x 8 x 12 takes 3% less, but its rounding moves the step at which the unstable NR=96 run of
+// tests/test_gpu_c1_diag.py leaves single corrector passes.)
+// Columns (the theta transforms) have no padding and more lines: two passes where three would do.
+__host__ __device__ constexpr int pass_radix(int n, int s, bool cols) {
+  if (cols && n == 192) return s == 0 ? 16 : s == 1 ? 12 : 0;
+  if (cols && n == 144) return s < 2 ? 12 : 0;
+  if (cols && n == 72) return s == 0 ? 9 : s == 1 ? 8 : 0;
+  constexpr int R[][4] = {{12, 12, 0, 0}, {18, 2, 9, 0}, {24, 4, 6, 0}, {36, 6, 6, 0}, {48, 8, 6, 0},
+                          {54, 6, 9, 0}, {72, 8, 9, 0}, {96, 8, 4, 3}, {108, 9, 12, 0}, {144, 16, 9, 0},
+                          {162, 9, 6, 3}, {192, 8, 4, 6}, {216, 6, 6, 6}, {288, 8, 6, 6}, {384, 8, 6, 8},
+                          {432, 16, 9, 3}, {576, 8, 9, 8}, {768, 16, 8, 6}};
   for (const auto& r : R)
     if (r[0] == n) return s < 3 ? r[1 + s] : 0;
   return 0;
 }
 
-// Place of element e in a line of contiguous elements: one gap per 16 so that the strided
-// stores of a first pass spread over the banks.
+// Place of element e in a line of contiguous elements between passes: one gap per 16 so that
+// the strided stores of a first pass spread over the banks.  A transform's input and output
+// are without gaps.
 __host__ __device__ constexpr int line_pad(int e) { return e + (e >> 4); }
+// Place of element b + q D (b of stride-1 origin with b % 16 < R known, q a constant): the gap
+// count splits into b's and a constant's wherever no carry can join them.
+template <int D, int R> __device__ __forceinline__ int line_at(int b, int q) {
+  const int o = q * D;
+  if (D % 16 == 0) return line_pad(b) + o + (o >> 4);
+  if (R + (o & 15) <= 16) return line_pad(b) + o + (o >> 4);
+  return line_pad(b + o);
+}
+// The number of residues mod 16 that the origin of a pass's reads (j < NBF) or stores
+// (multiples of NS P plus k < NS) takes.
+__host__ __device__ constexpr int line_res_read(int nbf) { return nbf <= 16 ? nbf : 16; }
+__host__ __device__ constexpr int line_res_store(int ns, int p) {
+  return ns * p % 16 == 0 ? (ns < 16 ? ns : 16) : ns * p == 8 ? 8 + ns : 16;
+}
 
 // One Stockham pass of radix P over NB transforms of length N (see fft_stage_ct), in place:
 // element e of transform t at t BS + e ES (COLS: neighbouring threads on neighbouring
-// transforms) or at t BS + line_pad(e).  Elements [Z0, Z1] are known to be zero on the way in
+// transforms) or at t BS + e
+// (line_pad(e) between passes).  Elements [Z0, Z1] are known to be zero on the way in
 // (first pass), elements [D0, D1] not needed on the way out (last pass); empty if Z1 < Z0.
 template <typename T, int SIGN, int N, int NB, int ES, int BS, bool COLS, int NTH, int P, int NS, int Z0, int Z1, int D0, int D1>
 __device__ __forceinline__ void fft_pass(cpx<T>* buf, const typename vec2<T>::type* __restrict__ tw) {
@@ -318,7 +345,9 @@ __device__ __forceinline__ void fft_pass(cpx<T>* buf, const typename vec2<T>::ty
       for (int q = 0; q < P; q++) {
         const int e = j + q * NBF;
         if (NS == 1 && q * NBF >= Z0 && (q + 1) * NBF - 1 <= Z1) v[rr][q] = mk<T>(0, 0);
-        else v[rr][q] = buf[t * BS + (COLS ? e * ES : line_pad(e))];
+        else if (COLS) v[rr][q] = buf[t * BS + e * ES];
+        else if (NS == 1) v[rr][q] = buf[t * BS + e];
+        else v[rr][q] = buf[t * BS + line_at<NBF, line_res_read(NBF)>(j, q)];
       }
     }
   }
@@ -338,8 +367,9 @@ __device__ __forceinline__ void fft_pass(cpx<T>* buf, const typename vec2<T>::ty
 #pragma unroll
       for (int q = 0; q < P; q++) {
         if (NS * P == N && q * NS >= D0 && (q + 1) * NS - 1 <= D1) continue;
-        const int e = base + q * NS;
-        buf[t * BS + (COLS ? e * ES : line_pad(e))] = v[rr][q];
+        if (COLS) buf[t * BS + (base + q * NS) * ES] = v[rr][q];
+        else if (NS * P == N) buf[t * BS + base + q * NS] = v[rr][q];
+        else buf[t * BS + line_at<NS, line_res_store(NS, P)>(base, q)] = v[rr][q];
       }
     }
   }
@@ -348,7 +378,7 @@ __device__ __forceinline__ void fft_pass(cpx<T>* buf, const typename vec2<T>::ty
 
 template <typename T, int SIGN, int N, int NB, int ES, int BS, bool COLS, int NTH, int Z0, int Z1, int D0, int D1, int S = 0, int NS = 1>
 __device__ __forceinline__ void pass_fft(cpx<T>* buf, const typename vec2<T>::type* __restrict__ tw) {
-  constexpr int P = pass_radix(N, S);
+  constexpr int P = pass_radix(N, S, COLS);
   if constexpr (P > 0) {
     fft_pass<T, SIGN, N, NB, ES, BS, COLS, NTH, P, NS, Z0, Z1, D0, D1>(buf, tw);
     pass_fft<T, SIGN, N, NB, ES, BS, COLS, NTH, Z0, Z1, D0, D1, S + 1, NS * P>(buf, tw);

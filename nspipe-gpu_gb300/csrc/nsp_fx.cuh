@@ -40,13 +40,31 @@ __device__ __forceinline__ unsigned fx_mag(unsigned k, unsigned emax) {
   return (((k & 0xFFFFFu) | 0x100000u) >> min(emax - (k >> 20), 31u)) + 1u;
 }
 
-// The line's exponent E from its largest key and its sum of magnitudes (fx_mag units):
-// the sum is below 2^E.  Clamped so that zero and subnormal lines convert to 0.
-__device__ __forceinline__ int fx_exponent(unsigned kmax, unsigned sum) {
-  const int emax = (int)(kmax >> 20);
-  if (emax >= 0x7FF) return FX_BAD;
-  return max(emax - 1043 + (32 - __clz((int)sum)), -900);
+// The line's exponent E from its largest exponent field and its sum of magnitudes (fx_mag
+// units): the sum is below 2^E.  Clamped so that zero and subnormal lines convert to 0 and
+// fx_to needs no range checks; a line that sums to 2^1000 or more counts as infinite.
+__device__ __forceinline__ int fx_exponent(int emax, unsigned sum) {
+  const int E = max(emax - 1043 + (32 - __clz((int)sum)), -900);
+  return emax >= 0x7FF || E > 1000 ? FX_BAD : E;
 }
+
+// Largest exponent field and sum of magnitudes of a line in one pass: the sum is kept in units
+// of the largest value so far (rounded up each time the unit grows).
+struct FxSum {
+  int e = 0;
+  unsigned s = 0u;
+  // two values by their keys
+  __device__ __forceinline__ void add(unsigned kx, unsigned ky) {
+    const int n = max(e, (int)(max(kx, ky) >> 20));
+    s = (s >> min(n - e, 31)) + fx_mag(kx, (unsigned)n) + fx_mag(ky, (unsigned)n) + 1u;
+    e = n;
+  }
+  // ... and over the warp; returns the exponent
+  __device__ __forceinline__ int warp_exponent() const {
+    const int n = __reduce_max_sync(0xFFFFFFFFu, e);
+    return fx_exponent(n, __reduce_add_sync(0xFFFFFFFFu, (s >> min(n - e, 31)) + 1u));
+  }
+};
 
 // x 2^(FX_BITS - E) rounded to the nearest integer; |x| < 2^E.  (Truncation would stop every
 // coefficient below one unit; rounded, the units of the others carry it on average as the
@@ -57,7 +75,7 @@ __device__ __forceinline__ fx fx_from(double x, int E) {
   // 1.m left-aligned below the sign bit, then shifted right by r >= 2
   const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, 10) << 32) | (lo << 10);
   const int r = E + 1085 - FX_BITS - (int)((hi >> 20) & 0x7FFu);
-  const fx v = (fx)(((m >> (min(max(r, 1), 64) - 1)) + 1) >> 1);
+  const fx v = (fx)(((m >> min(r - 1, 63)) + 1) >> 1);
   const fx s = (fx)((int)hi >> 31);
   return (v ^ s) - s;
 }
@@ -69,23 +87,19 @@ __device__ __forceinline__ fx fx_from_times(double x, unsigned q, int E) {
   const unsigned qz = q << z;
   const unsigned long long m = (unsigned long long)lo * qz + ((unsigned long long)(mh * qz) << 32);
   const int r = E + 1075 - FX_BITS - (int)((hi >> 20) & 0x7FFu) + z;
-  const fx v = q ? (fx)(((m >> (min(max(r, 1), 64) - 1)) + 1) >> 1) : 0;
+  const fx v = q ? (fx)(((m >> min(r - 1, 63)) + 1) >> 1) : 0;
   const fx s = (fx)((int)hi >> 31);
   return (v ^ s) - s;
 }
 
-// v 2^e rounded to nearest; 0 below 2^-1022, Inf above FP64's range.
+// v 2^e rounded to nearest, |v| < 2^62, e = E - FX_BITS of a line (so the result is normal).
 __device__ __forceinline__ double fx_to(fx v, int e) {
   const int s = (int)(v >> 63);
   const unsigned long long a = (unsigned long long)((v ^ (fx)s) - (fx)s);
-  const int lz = __clzll((long long)a);
-  const unsigned long long m = a << (lz & 63);
-  const int be = 1086 - lz + e;  // biased exponent of the leading bit
-  const unsigned long long q = (m >> 11) + ((m >> 10) & 1u);
-  unsigned hi = (unsigned)(q >> 32) + ((unsigned)(be - 1) << 20), lo = (unsigned)q;
-  if (be < 1 || a == 0) hi = lo = 0;
-  if (be > 2046) hi = 0x7FF00000u, lo = 0;
-  return __hiloint2double((int)(hi | ((unsigned)s & 0x80000000u)), (int)lo);
+  const int z = __clzll((long long)a) - 1;  // leading bit to 62: rounding carries into 63 at most
+  const unsigned long long q = ((a << (z & 63)) + 0x200u) >> 10;
+  const unsigned hi = (unsigned)(q >> 32) + ((unsigned)(1084 + e - z) << 20);
+  return __hiloint2double((int)(a ? hi | ((unsigned)s & 0x80000000u) : 0u), (int)q);
 }
 
 __device__ __forceinline__ double fx_nan() { return __hiloint2double(0x7FF80000, 0); }
@@ -186,10 +200,25 @@ __device__ __forceinline__ double2 fx_value(const cpx<fx>& v, int E) {
 
 // ---- kernels along z (the z stage, the cross sections)
 constexpr int MAXRZ = 6;  // register rounds of the run-time FFT
-// Threads of the z kernel: about the butterflies of a pass over its 6 RPB transforms.
-constexpr int z_threads(int nzr) { return nzr >= 576 ? 288 : nzr == 0 || nzr >= 96 ? 192 : nzr >= 54 ? 128 : 96; }
-constexpr int z_blocks(int nzr) { return nzr >= 576 ? 2 : nzr == 0 ? 1 : nzr >= 96 ? 3 : 4; }
+// Threads of the z kernels, about the butterflies of a pass over their 6 RPB lines, and the
+// blocks per SM that the registers are limited for.  Measured per length, one z-stage launch of
+// NR=48 x 32 x n/3 modes, ns per member and mode against three blocks of 192 threads (two of
+// 288 from 576 points): 72: 800 (905), 96: 811 (1020), 144: 809 (936), 162: 1053 (1232),
+// 192: 665 (733), 216: 922 (931), 288: 775, 384: 734 (788), 432: 863 (912), 576: 943 (989),
+// 768: 855 (930): many small blocks cover the barriers between the passes, where the radix
+// leaves them the registers.
+constexpr int z_threads(int n) { return n == 432 ? 288 : n == 0 || n >= 96 ? 192 : n >= 54 ? 128 : 96; }
+constexpr int z_blocks(int n) {
+  return n == 0 ? 1 : n >= 576 ? 2 : n == 288 || n == 432 ? 3 : n >= 216 ? 4 : n >= 162 ? 5 : n >= 96 ? 6 : 8;
+}
 
+// Values per line in shared memory: the gaps between passes, at least two behind the line.
+constexpr int line_pitch(int n) { return line_pad(n - 1) + 1 > n + 2 ? line_pad(n - 1) + 1 : n + 2; }
+// 16-byte asynchronous copies global -> shared, their groups and waits.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
 // Compiled z lengths and theta rows per block: two (three packed forward transforms for both)
 // while the six lines of each leave three blocks on an SM.
 #define NSP_NZR_LIST(X) X(24, 2) X(36, 2) X(48, 2) X(54, 2) X(72, 2) X(96, 2) X(108, 2) X(144, 2) X(162, 2) \

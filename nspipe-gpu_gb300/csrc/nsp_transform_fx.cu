@@ -16,11 +16,11 @@
 // exponent and then the sum of magnitudes are reduced over the line as integers (so the
 // scale, and with it every bit, is independent of the order), and the line is converted
 // in place.
-// Bound: integer issue and instruction fetch (16 members of NR=48 x 32 x 64 modes: ALU pipe
-// 53%, FP64 pipe 20%, 2.0 instructions per cycle and SM).  FP64 transforms were bound by the
-// FP64 pipe alone.  Per launch there, before and after: theta-inverse 903 -> 384 us, z stage
-// 3457 -> 860 us, theta-forward 283 -> 124 us; one member of 48 x 64 x 256 modes: 530 -> 190,
-// 2154 -> 509, 168 -> 76 us.  Radix-4 passes in the same arithmetic: 1230 us for the z stage.
+// Bound: integer issue, the barriers between the passes and instruction fetch (z stage, 16
+// members of NR=48 x 32 x 64 modes: ALU pipe 55%, IMAD 49%, FP64 pipe 24%).  FP64 transforms
+// were bound by the FP64 pipe alone.  Per launch there, before and after: theta-inverse 903 ->
+// 282 us, z stage 3457 -> 692 us, theta-forward 283 -> 82 us; one member of 48 x 64 x 256
+// modes: 530 -> 160, 2154 -> 451, 168 -> 46 us.
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -71,7 +71,7 @@ __device__ __forceinline__ int column_exponent(const double2 (&g)[V], unsigned* 
   if (LC < 32) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, LC);
   if ((threadIdx.x & 31) < LC) atomicAdd(ssum + lc, sum);
   __syncthreads();
-  return fx_exponent(kmax, ssum[lc]);
+  return fx_exponent((int)(kmax >> 20), ssum[lc]);
 }
 
 // The same for a run-time length: the block's columns, in FP64 at buf (element p of column
@@ -92,7 +92,7 @@ __device__ __forceinline__ int columns_to_fx(double2* buf, int total, unsigned k
   if (LC < 32) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, LC);
   if ((threadIdx.x & 31) < LC) atomicAdd(ssum + lc, sum);
   __syncthreads();
-  const int E = fx_exponent(kmax, ssum[lc]);
+  const int E = fx_exponent((int)emax, ssum[lc]);
   cpx<fx>* o = reinterpret_cast<cpx<fx>*>(buf);
   for (int idx = threadIdx.x; idx < total; idx += TTH) {
     const double2 v = buf[idx];
@@ -204,100 +204,100 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
   __shared__ unsigned skey[RPB * 3], ssum[RPB * 3];
   const int NR = tb.NR, NTP = tb.NTP;
   const int NZR = NZRC > 0 ? NZRC : tb.NZR, NZ = NZRC > 0 ? NZRC / 3 + 1 : tb.NZ;
-  const int ZP = NZRC > 0 ? line_pad(NZRC - 1) + 1 : NZR;
-  auto at = [](int e) { return NZRC > 0 ? line_pad(e) : e; };
+  const int ZP = NZRC > 0 ? line_pitch(NZRC) : NZR;
   const double2* G = reinterpret_cast<const double2*>(bf.G) + (size_t)mloc * 9 * NR * NTP * NZ;
   double2* H = reinterpret_cast<double2*>(bf.H) + (size_t)mloc * 3 * NR * NTP * NZ;
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < RPB * 3) skey[threadIdx.x] = ssum[threadIdx.x] = 0u;
+  // A pair's two columns are copied asynchronously into its own line -- field 2t at slot q,
+  // field 2t+1 at NZ + q, its last two values behind the line -- where the Hermitian extension
+  // then replaces them: slot q is written by the lane that has read it, the mirrored half
+  // starts behind the second field's slots (2 NZ - 2 = NZR - NZ + 1).  (Run-time lengths read
+  // G in place.)
+  auto live_row = [&](int rr) {
+    return j0 + rr < NTP && NSP_IN_BOUNDS(tb, ((size_t)i * NTP + j0 + rr) * NZ + NZ - 1, (size_t)NR * NTP * NZ, BC_Z_IN);
+  };
+  auto column = [&](int fld, int rr) {  // dz u_c comes from the u_c columns
+    return G + (((size_t)(fld >= 9 ? fld - 9 : fld) * NR + i) * NTP + j0 + rr) * NZ;
+  };
+  auto raw2 = [&](int q) { return q < NZ - 2 ? NZ + q : NZR - NZ + 2 + q; };
+  if constexpr (NZRC > 0) {
+    for (int task = threadIdx.x >> 5; task < RPB * 6; task += NTH / 32) {
+      const int t = task % 6, rr = task / 6;
+      if (!live_row(rr)) continue;
+      cpx<fx>* Zt = Z + (size_t)task * ZP;
+      const double2 *a = column(2 * t, rr), *b = column(2 * t + 1, rr);
+      for (int q = lane; q < NZ; q += 32) {
+        cp_async16(Zt + q, a + q);
+        cp_async16(Zt + raw2(q), b + q);
+      }
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncwarp();
+  }
   for (int task = threadIdx.x >> 5; task < RPB * 6; task += NTH / 32) {
-    const int t = task % 6, rr = task / 6, j = j0 + rr;
-    const bool live = j < NTP && NSP_IN_BOUNDS(tb, ((size_t)i * NTP + j) * NZ + NZ - 1, (size_t)NR * NTP * NZ, BC_Z_IN);
+    const int t = task % 6, rr = task / 6;
     cpx<fx>* Zt = Z + (size_t)task * ZP;
-    if (!live) {
-      for (int q = lane; q < NZR; q += 32) Zt[at(q)] = mk<fx>(0, 0);
+    if (!live_row(rr)) {
+      for (int q = lane; q < NZR; q += 32) Zt[q] = mk<fx>(0, 0);
       if (lane < 2) sE[rr * 12 + 2 * t + lane] = 0;
       continue;
     }
-    const double2* Gr[2];
-    bool dz[2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int fld = 2 * t + h;
-      dz[h] = fld >= 9;  // dz u_c comes from the u_c columns
-      Gr[h] = G + (((size_t)(dz[h] ? fld - 9 : fld) * NR + i) * NTP + j) * NZ;
-    }
-    // a line's values stay in registers where their number is known
-    constexpr int IT = NZRC > 0 ? (NZRC / 3 + 32) / 32 : 1;
-    double2 g[2][IT];
-    auto value = [&](int h, int k, int q) {
-      if (NZRC > 0) return g[h][k];
-      double2 v = Gr[h][q];
-      if (q == 0) v.y = 0.0;  // C2R ignores Im of the k_z = 0 coefficient
-      return v;
+    const double2* Gr[2] = {column(2 * t, rr), column(2 * t + 1, rr)};
+    const double2* raw = reinterpret_cast<const double2*>(Zt);
+    const bool dz[2] = {2 * t >= 9, 2 * t + 1 >= 9};
+    auto load = [&](int h, int q) { return NZRC > 0 ? raw[h ? raw2(q) : q] : Gr[h][q]; };
+    // A dz field's coefficient is the u column's times the whole number l, formed exactly in
+    // its conversion; its share of the key is rounded up.  Loops kept short: this kernel
+    // is bound by instruction fetch as much as by issue.
+    auto value = [&](int h, int q) {
+      const double2 v = load(h, q);
+      return q ? v : make_double2(v.x, 0.0);  // C2R ignores Im of the k_z = 0 coefficient
     };
-    // the exponent field's share of the factor l of a dz field (rounded up)
-    auto weight = [&](int h, int q) { return dz[h] && q > 1 ? (unsigned)(32 - __clz(q - 1)) << 20 : 0u; };
-    unsigned kmax[2] = {0u, 0u}, sum[2] = {0u, 0u};
     int E[2];
-    auto each = [&](auto f) {
-      if constexpr (NZRC > 0) {
-#pragma unroll
-        for (int k = 0; k < IT; k++)
-          if ((k + 1) * 32 <= NZRC / 3 + 1 || lane + 32 * k < NZ) f(k, lane + 32 * k);
-      } else {
-        for (int q = lane; q < NZ; q += 32) f(0, q);
-      }
-    };
-    if constexpr (NZRC > 0) {
-      each([&](int k, int q) {
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          g[h][k] = Gr[h][q];
-          if (q == 0) g[h][k].y = 0.0;
-        }
-      });
-    }
-    each([&](int k, int q) {
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const double2 v = value(h, k, q);
-        const unsigned key = max(fx_key(v.x), fx_key(v.y));
-        kmax[h] = max(kmax[h], key < 0x100000u || (dz[h] && q == 0) ? 0u : key + weight(h, q));
-      }
-    });
-#pragma unroll
-    for (int h = 0; h < 2; h++) kmax[h] = __reduce_max_sync(0xFFFFFFFFu, kmax[h]);
-    each([&](int k, int q) {
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const double2 v = value(h, k, q);
-        const unsigned w = weight(h, q), e = kmax[h] >> 20;
-        if (!(dz[h] && q == 0)) sum[h] += fx_mag(min(fx_key(v.x) + w, kmax[h]), e) + fx_mag(min(fx_key(v.y) + w, kmax[h]), e);
-      }
-    });
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      sum[h] = __reduce_add_sync(0xFFFFFFFFu, sum[h]);
-      E[h] = fx_exponent(kmax[h], sum[h]);
+      FxSum sum;
+      if (dz[h]) {
+#pragma unroll 1
+        for (int q = lane ? lane : 32; q < NZ; q += 32) {
+          const double2 v = load(h, q);
+          const unsigned w = q > 1 ? (unsigned)(32 - __clz(q - 1)) << 20 : 0u;
+          const unsigned kx = fx_key(v.x), ky = fx_key(v.y);
+          sum.add(kx < 0x100000u ? 0u : min(kx + w, 0x7FF00000u), ky < 0x100000u ? 0u : min(ky + w, 0x7FF00000u));
+        }
+      } else {
+#pragma unroll 1
+        for (int q = lane; q < NZ; q += 32) {
+          const double2 v = value(h, q);
+          sum.add(fx_key(v.x), fx_key(v.y));
+        }
+      }
+      E[h] = sum.warp_exponent();
       if (E[h] != FX_BAD) E[h] += 1;  // two-sided
       if (lane == 0) sE[rr * 12 + 2 * t + h] = E[h];
     }
-    each([&](int k, int q) {
-      cpx<fx> x[2];
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const double2 v = value(h, k, q);
-        if (dz[h]) x[h] = mk<fx>(-fx_from_times(v.y, q, E[h]), fx_from_times(v.x, q, E[h]));
-        else x[h] = mk<fx>(fx_from(v.x, E[h]), fx_from(v.y, E[h]));
+#pragma unroll 1
+    for (int q = lane; q < NZ; q += 32) {
+      const double2 v = value(0, q), w = value(1, q);
+      cpx<fx> x, y;
+      if (dz[1]) {  // pairs (dt u_z, dz u_r) and (dz u_theta, dz u_z)
+        x = dz[0] ? muli<fx, +1>(mk<fx>(fx_from_times(v.x, q, E[0]), fx_from_times(v.y, q, E[0])))
+                  : mk<fx>(fx_from(v.x, E[0]), fx_from(v.y, E[0]));
+        y = muli<fx, +1>(mk<fx>(fx_from_times(w.x, q, E[1]), fx_from_times(w.y, q, E[1])));
+      } else {
+        x = mk<fx>(fx_from(v.x, E[0]), fx_from(v.y, E[0]));
+        y = mk<fx>(fx_from(w.x, E[1]), fx_from(w.y, E[1]));
       }
-      Zt[at(q)] = mk<fx>(x[0].x - x[1].y, x[0].y + x[1].x);
-      if (q) Zt[at(NZR - q)] = mk<fx>(x[0].x + x[1].y, x[1].x - x[0].y);
-    });
-    for (int q = NZ + lane; q <= NZR - NZ; q += 32) Zt[at(q)] = mk<fx>(0, 0);
+      Zt[q] = mk<fx>(x.x - y.y, x.y + y.x);
+      if (q) Zt[NZR - q] = mk<fx>(x.x + y.y, y.x - x.y);
+    }
+    __syncwarp();  // the second field's slots have been read
+    for (int q = NZ + lane; q <= NZR - NZ; q += 32) Zt[q] = mk<fx>(0, 0);
   }
   __syncthreads();
-  constexpr int BS = NZRC > 0 ? line_pad(NZRC - 1) + 1 : 0;
+  constexpr int BS = NZRC > 0 ? line_pitch(NZRC) : 0;
   if constexpr (NZRC > 0)
     pass_fft<fx, +1, NZRC, RPB * 6, 1, BS, false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx);
   else
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
     double nr[RPB], nt[RPB], nz[RPB];
 #pragma unroll
     for (int rr = 0; rr < RPB; rr++) {
-      const cpx<fx>* Zr = Z + (size_t)rr * 6 * ZP + at(n);
+      const cpx<fx>* Zr = Z + (size_t)rr * 6 * ZP + n;
       const int* e = sE + rr * 12;
       double u[12];
       int top = 0;
@@ -334,12 +334,12 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
       kn[rr * 3 + 2] = max(kn[rr * 3 + 2], fx_key(nz[rr]));
     }
     if (RPB == 2) {
-      P[at(n)] = make_double2(nr[0], nt[0]);
-      P[ZP + at(n)] = make_double2(nr[RPB - 1], nt[RPB - 1]);
-      P[2 * ZP + at(n)] = make_double2(nz[0], nz[RPB - 1]);
+      P[n] = make_double2(nr[0], nt[0]);
+      P[ZP + n] = make_double2(nr[RPB - 1], nt[RPB - 1]);
+      P[2 * ZP + n] = make_double2(nz[0], nz[RPB - 1]);
     } else {
-      P[at(n)] = make_double2(nr[0], nt[0]);
-      P[ZP + at(n)] = make_double2(nz[0], 0.0);
+      P[n] = make_double2(nr[0], nt[0]);
+      P[ZP + n] = make_double2(nz[0], 0.0);
     }
   }
 #pragma unroll
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
   for (int n = threadIdx.x; n < NZR; n += NTH) {
 #pragma unroll
     for (int s = 0; s < NFWD; s++) {
-      const double2 v = P[s * ZP + at(n)];
+      const double2 v = P[s * ZP + n];
 #pragma unroll
       for (int e = 0; e < RPB * 3; e++)
         if (s_of(e) == s) sn[e] += fx_mag(fx_key(p_of(e) ? v.y : v.x), skey[e] >> 20);
@@ -372,16 +372,16 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
   __syncthreads();
   int EN[RPB * 3];
 #pragma unroll
-  for (int e = 0; e < RPB * 3; e++) EN[e] = fx_exponent(skey[e], ssum[e]);
+  for (int e = 0; e < RPB * 3; e++) EN[e] = fx_exponent((int)(skey[e] >> 20), ssum[e]);
   for (int n = threadIdx.x; n < NZR; n += NTH) {
 #pragma unroll
     for (int s = 0; s < NFWD; s++) {
-      const double2 v = P[s * ZP + at(n)];
+      const double2 v = P[s * ZP + n];
       cpx<fx> x = mk<fx>(0, 0);
 #pragma unroll
       for (int e = 0; e < RPB * 3; e++)
         if (s_of(e) == s) (p_of(e) ? x.y : x.x) = fx_from(p_of(e) ? v.y : v.x, EN[e]);
-      Z[s * ZP + at(n)] = x;
+      Z[s * ZP + n] = x;
     }
   }
   __syncthreads();
@@ -395,9 +395,9 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
     const int q = idx % NQ, e = idx / NQ, c = e % 3, rr = e / 3, j = j0 + rr;
     if (j >= NTP) continue;
     const cpx<fx>* X = Z + (size_t)s_of(e) * ZP;
-    const cpx<fx> xq = X[at(q)], xm = X[at(q ? NZR - q : 0)];
+    const cpx<fx> xq = X[q], xm = X[q ? NZR - q : 0];
     const cpx<fx> v = p_of(e) ? mk<fx>(xq.y + xm.y, xm.x - xq.x) : mk<fx>(xq.x + xm.x, xq.y - xm.y);
-    const int E = fx_exponent(skey[e], ssum[e]);
+    const int E = fx_exponent((int)(skey[e] >> 20), ssum[e]);
     const size_t h = (((size_t)c * NR + i) * NTP + j) * NZ + q;
     if (NSP_IN_BOUNDS(tb, h, (size_t)3 * NR * NTP * NZ, BC_Z_OUT)) H[h] = fx_value(v, E == FX_BAD ? E : E - 1);
   }
@@ -490,7 +490,7 @@ static void launch_theta_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, const d
 
 template <int NZRC, int RPB>
 static void launch_z_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, bool standalone, cudaStream_t st, int nm) {
-  const size_t sm = sizeof(cpx<fx>) * 6 * RPB * (NZRC > 0 ? line_pad(NZRC - 1) + 1 : tb.NZR);
+  const size_t sm = sizeof(cpx<fx>) * 6 * RPB * (NZRC > 0 ? line_pitch(NZRC) : tb.NZR);
   fx_z<NZRC, RPB><<<dim3((tb.NTP + RPB - 1) / RPB, tb.NR, nm), z_threads(NZRC), sm, st>>>(tb, bf, dctl, standalone ? 1 : 0);
 }
 
