@@ -9,11 +9,14 @@
 // are corrector iterations of the members that have not converged (the others
 // skip their blocks), so each member keeps the reference's own iteration count
 // (integrate, mod_integrate.cu:112-130) without any device-to-host round trip.
+#include <cuda.h>
 #include <sys/stat.h>
 
 #include <cmath>
 #include <algorithm>
 #include <cstdarg>
+#include <cstddef>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -85,9 +88,9 @@ struct nsp_ctx {
   // nsp_set_strict: a step whose corrector loop stopped at maxit with err > tol makes
   // nsp_step / nsp_step_host return NSP_ERR_MAXIT.
   bool strict = false;
-  // Pinned host copy of the step history, then the members' status words, the fault
-  // flag and the members' unconverged-step counts: read back after the steps with
-  // asynchronous copies and one synchronisation.
+  // Pinned host copy of the control block's end: the fault flag, the step count, the members'
+  // unconverged-step counts and status words, the step history -- read back after the steps
+  // with one copy and one synchronisation.
   int* pin = nullptr;
   std::vector<void*> allocs;
   std::string err;
@@ -679,14 +682,20 @@ int nsp_create(const nsp_params* members, int n_members, int precision, int devi
   h.tol = members[0].tol;
   h.hist_cap = 1024;
   int rc;
+  // The control block and, right behind it, what a stepping call clears and reads back.
+  static_assert(offsetof(Ctl, step) == offsetof(Ctl, fault) + sizeof(int) && offsetof(Ctl, step) + sizeof(int) == sizeof(Ctl),
+                "fault and step end the control block");
+  unsigned char* ctl = nullptr;
+  if ((rc = dalloc(c, &ctl, sizeof(Ctl) + sizeof(int) * n_members * ((size_t)h.hist_cap + 2)))) return rc;
+  c->dctl = reinterpret_cast<Ctl*>(ctl);
+  h.unconv = reinterpret_cast<int*>(ctl + sizeof(Ctl));
+  h.status = h.unconv + n_members;
+  h.hist = h.status + n_members;
   if ((rc = dalloc(c, &h.phase, sizeof(int) * n_members))) return rc;
   if ((rc = dalloc(c, &h.ite, sizeof(int) * n_members))) return rc;
-  if ((rc = dalloc(c, &h.status, sizeof(int) * n_members))) return rc;
   if ((rc = dalloc(c, &h.num, sizeof(unsigned long long) * n_members))) return rc;
   if ((rc = dalloc(c, &h.den, sizeof(unsigned long long) * n_members))) return rc;
   if ((rc = dalloc(c, &h.err, sizeof(double) * n_members))) return rc;
-  if ((rc = dalloc(c, &h.hist, sizeof(int) * n_members * (size_t)h.hist_cap))) return rc;
-  if ((rc = dalloc(c, &h.unconv, sizeof(int) * n_members))) return rc;
   CK(cudaMemset(h.unconv, 0, sizeof(int) * n_members));
   CK(cudaMemset(h.phase, 0, sizeof(int) * n_members));
   CK(cudaMemset(h.ite, 0, sizeof(int) * n_members));
@@ -694,14 +703,13 @@ int nsp_create(const nsp_params* members, int n_members, int precision, int devi
   CK(cudaMemset(h.num, 0, sizeof(unsigned long long) * n_members));
   CK(cudaMemset(h.den, 0, sizeof(unsigned long long) * n_members));
   CK(cudaMemset(h.err, 0, sizeof(double) * n_members));
-  if ((rc = dalloc(c, &c->dctl, sizeof(Ctl)))) return rc;
   CK(cudaMemcpy(c->dctl, &h, sizeof(Ctl), cudaMemcpyHostToDevice));
   // Bounds record of the bounds-checked build (nsp_bounds.cuh), shared by every group.
   unsigned long long* bc = nullptr;
   if ((rc = dalloc(c, &bc, 4 * sizeof(unsigned long long)))) return rc;
   CK(cudaMemset(bc, 0, 4 * sizeof(unsigned long long)));
   for (auto& g : c->groups) g.tb.bc = bc;
-  CK(cudaMallocHost(&c->pin, sizeof(int) * ((size_t)(h.hist_cap + 2) * n_members + 1)));
+  CK(cudaMallocHost(&c->pin, sizeof(int) * ((size_t)(h.hist_cap + 2) * n_members + 2)));
   return NSP_OK;
 }
 
@@ -961,26 +969,78 @@ int nsp_get_state_host(nsp_ctx* c, int m, double* ur, double* ut, double* uz) {
   return copy_states(c, m, dst, false);
 }
 
+// Whether a kernel may take [p, p + bytes) as an array of complex values: aligned, in one
+// allocation of the context's device and inside it.  Anything else goes through cudaMemcpy,
+// which copies what it can (other devices, 8-byte alignment) and reports what it cannot.
+static bool plain_device_array(const nsp_ctx* c, const void* p, size_t bytes) {
+  if (reinterpret_cast<uintptr_t>(p) % alignof(double2)) return false;
+  using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static const Range range = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      return (Range) nullptr;
+    }
+    return (Range)f;
+  }();
+  cudaPointerAttributes at;
+  if (!range || cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeDevice || at.device != c->device) {
+    cudaGetLastError();
+    return false;
+  }
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr q = reinterpret_cast<CUdeviceptr>(p);
+  return range(&base, &size, q) == CUDA_SUCCESS && q >= base && q - base <= size && bytes <= size - (q - base);
+}
+
+// One member's components between the caller's device arrays `user` and the state buffers: one
+// launch for the three.
+static int hand_over(nsp_ctx* c, int m, const void* const (&user)[3], bool to_state) {
+  const long long n = c->groups[c->grp[m]].tb.S;
+  const size_t bytes = sizeof(double2) * (size_t)n;
+  CK(cudaSetDevice(c->device));
+  double2* state[3];
+  bool plain = true;
+  for (int k = 0; k < 3; k++) {
+    state[k] = state_ptr(c, m, k);
+    plain = plain && plain_device_array(c, user[k], bytes);
+  }
+  if (plain) {
+    const double2* src[3];
+    double2* dst[3];
+    for (int k = 0; k < 3; k++) {
+      double2* u = static_cast<double2*>(const_cast<void*>(user[k]));
+      src[k] = to_state ? u : state[k];
+      dst[k] = to_state ? state[k] : u;
+    }
+    launch_copy3(src, dst, n, to_state ? c->hctl.status + c->internal[m] : nullptr, c->st);
+    CK(cudaGetLastError());
+  } else {
+    if (to_state)
+      if (int rc = clear_status(c, m)) return rc;
+    for (int k = 0; k < 3; k++) {
+      if (to_state) CK(cudaMemcpyAsync(state[k], user[k], bytes, cudaMemcpyDeviceToDevice, c->st));
+      else CK(cudaMemcpyAsync(const_cast<void*>(user[k]), state[k], bytes, cudaMemcpyDeviceToDevice, c->st));
+    }
+  }
+  CK(cudaStreamSynchronize(c->st));
+  return NSP_OK;
+}
+
 int nsp_set_state_device(nsp_ctx* c, int m, const void* ur, const void* ut, const void* uz) {
   if (int rc = check_member(c, m)) return rc;
   if (!ur || !ut || !uz) return fail(c, NSP_ERR_ARG, "null state pointer");
-  size_t bytes = sizeof(double2) * (size_t)c->groups[c->grp[m]].tb.S;
-  const void* src[3] = {ur, ut, uz};
   c->mirror_ok = false;
-  if (int rc = clear_status(c, m)) return rc;
-  for (int k = 0; k < 3; k++) CK(cudaMemcpyAsync(state_ptr(c, m, k), src[k], bytes, cudaMemcpyDeviceToDevice, c->st));
-  CK(cudaStreamSynchronize(c->st));
-  return NSP_OK;
+  return hand_over(c, m, {ur, ut, uz}, true);
 }
 
 int nsp_get_state_device(nsp_ctx* c, int m, void* ur, void* ut, void* uz) {
   if (int rc = check_member(c, m)) return rc;
   if (!ur || !ut || !uz) return fail(c, NSP_ERR_ARG, "null state pointer");
-  size_t bytes = sizeof(double2) * (size_t)c->groups[c->grp[m]].tb.S;
-  void* dst[3] = {ur, ut, uz};
-  for (int k = 0; k < 3; k++) CK(cudaMemcpyAsync(dst[k], state_ptr(c, m, k), bytes, cudaMemcpyDeviceToDevice, c->st));
-  CK(cudaStreamSynchronize(c->st));
-  return NSP_OK;
+  return hand_over(c, m, {ur, ut, uz}, false);
 }
 
 // One step of every member whose phase is 0 at its start (members at -1 sit it out):
@@ -1058,37 +1118,37 @@ static long long kernels_per_pass(const nsp_ctx* c) {
   return (c->precision == NSP_MIXED && !c->use_graph ? 5LL : 4LL) * (long long)c->groups.size() + 1;
 }
 
-// The step history of the last `batch` steps into the pinned buffer; with `final` also
-// the members' status words, the fault flag and the unconverged-step counts.  One
-// synchronisation of the stream.
-static int read_control(nsp_ctx* c, int batch, bool final) {
-  const int nm = c->nmem;
-  const size_t tail = (size_t)c->hctl.hist_cap * nm;
-  if (batch > 0)
-    CK(cudaMemcpyAsync(c->pin, c->hctl.hist, sizeof(int) * (size_t)batch * nm, cudaMemcpyDeviceToHost, c->st));
-  if (final) {
-    CK(cudaMemcpyAsync(c->pin + tail, c->hctl.status, sizeof(int) * nm, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(c->pin + tail + nm, &c->dctl->fault, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(c->pin + tail + nm + 1, c->hctl.unconv, sizeof(int) * nm, cudaMemcpyDeviceToHost, c->st));
-  }
+// The fault flag, the members' unconverged-step counts and status words and the history of
+// the last `batch` steps into the pinned buffer: one copy, one synchronisation of the stream.
+static int read_control(nsp_ctx* c, int batch) {
+  CK(cudaMemcpyAsync(c->pin, &c->dctl->fault, sizeof(int) * (2 + (size_t)(2 + batch) * c->nmem), cudaMemcpyDeviceToHost,
+                     c->st));
   CK(cudaStreamSynchronize(c->st));
   return NSP_OK;
 }
+static const int* pin_unconv(const nsp_ctx* c) { return c->pin + 2; }
+static const int* pin_status(const nsp_ctx* c) { return c->pin + 2 + c->nmem; }
+static const int* pin_hist(const nsp_ctx* c) { return c->pin + 2 + 2 * (size_t)c->nmem; }
 
-// After a final read_control: a device-side wait that ran out, then non-finite members.
+// Clears the step count and, at a call's start, the unconverged-step counts behind it.
+static int begin_steps(nsp_ctx* c, bool first) {
+  CK(cudaMemsetAsync(&c->dctl->step, 0, sizeof(int) * (first ? 1 + (size_t)c->nmem : 1), c->st));
+  return NSP_OK;
+}
+
+// After read_control: a device-side wait that ran out, then non-finite members.
 static int control_verdict(nsp_ctx* c) {
   const int nm = c->nmem;
-  const int* tail = c->pin + (size_t)c->hctl.hist_cap * nm;
-  if (tail[nm]) {
+  if (c->pin[0]) {
     CK(cudaMemsetAsync(&c->dctl->fault, 0, sizeof(int), c->st));
     return fail(c, NSP_ERR_DEVICE, "a device-side wait ran out; the call's results are invalid");
   }
   for (int m = 0; m < nm; m++)
-    if (tail[c->internal[m]] & NSP_ERR_NONFINITE)
+    if (pin_status(c)[c->internal[m]] & NSP_ERR_NONFINITE)
       return fail(c, NSP_ERR_NONFINITE, "member %d: non-finite velocity or convergence measure", m);
   if (c->strict)
     for (int m = 0; m < nm; m++)
-      if (const int n = tail[nm + 1 + c->internal[m]])
+      if (const int n = pin_unconv(c)[c->internal[m]])
         return fail(c, NSP_ERR_MAXIT, "member %d: %d step(s) stopped at maxit = %d without convergence", m, n,
                     c->hctl.maxit);
   return NSP_OK;
@@ -1109,17 +1169,16 @@ int nsp_step(nsp_ctx* c, int nsteps, int* iters_out) {
   if (c->precision == NSP_MIXED && nsteps > 0 && !c->mirror_ok)
     for (auto& g : c->groups) launch_mirror(g.tb, g.bf.U[c->parity], g.bf.U32[c->parity], g.bf.DR32[c->parity], c->st);
   c->mirror_ok = false;
-  if (nsteps > 0) CK(cudaMemsetAsync(c->hctl.unconv, 0, sizeof(int) * nm, c->st));
   if (nsteps == 0)
-    if (int rc = read_control(c, 0, true)) return rc;
+    if (int rc = read_control(c, 0)) return rc;
   for (int done = 0; done < nsteps;) {
     int chunk = std::min(cap, nsteps - done);
-    CK(cudaMemsetAsync(&c->dctl->step, 0, sizeof(int), c->st));
+    if (int rc = begin_steps(c, done == 0)) return rc;
     for (int s = 0; s < chunk; s++)
       if (int rc = run_step(c)) return rc;
     CK(cudaGetLastError());
-    if (int rc = read_control(c, chunk, done + chunk == nsteps)) return rc;
-    const int* hist = c->pin;
+    if (int rc = read_control(c, chunk)) return rc;
+    const int* hist = pin_hist(c);
     for (int s = 0; s < chunk; s++) {
       int mx = 0;
       for (int m = 0; m < nm; m++) mx = std::max(mx, hist[(size_t)s * nm + m]);
@@ -1204,7 +1263,6 @@ int nsp_step_host(nsp_ctx* c, int nsteps, const double* in, double* out, int* it
     c->ev_done.push_back(e2);
   }
   if (int rc = clear_status(c, NSP_ALL_MEMBERS)) return rc;  // every state comes from `in`
-  CK(cudaMemsetAsync(c->hctl.unconv, 0, sizeof(int) * nm, c->st));
   // Copies in may start only once earlier work on the state is done.
   CK(cudaEventRecord(c->ev_done[0], c->st));
   CK(cudaStreamWaitEvent(c->cp_in, c->ev_done[0], 0));
@@ -1213,7 +1271,7 @@ int nsp_step_host(nsp_ctx* c, int nsteps, const double* in, double* out, int* it
   long long launches = 0;
   for (int done = 0; done < nsteps;) {
     const int batch = std::min(cap, nsteps - done);
-    CK(cudaMemsetAsync(&c->dctl->step, 0, sizeof(int), c->st));
+    if (int rc = begin_steps(c, done == 0)) return rc;
     std::vector<char> chunked(batch, 0);
     for (int s = 0; s < batch; s++) {
       const bool first = done + s == 0, last = done + s == nsteps - 1;
@@ -1261,9 +1319,9 @@ int nsp_step_host(nsp_ctx* c, int nsteps, const double* in, double* out, int* it
       CK(cudaGetLastError());
       c->parity ^= 1;
     }
-    if (int rc = read_control(c, batch, done + batch == nsteps)) return rc;
+    if (int rc = read_control(c, batch)) return rc;
     for (int s = 0; s < batch; s++) {
-      const int* row = c->pin + (size_t)s * nm;
+      const int* row = pin_hist(c) + (size_t)s * nm;
       if (chunked[s]) {
         for (int k = 0; k < K; k++)
           launches += (1 + *std::max_element(row + c->chunk_lo[k], row + c->chunk_lo[k + 1])) * per_iter;

@@ -117,7 +117,6 @@ enum { MEAN_V = 0, MEAN_W, MEAN_U, MEAN_WP, MEAN_UP, MEAN_N };
 // p > 0 = corrector iteration p pending, -1 = converged for this step.
 struct Ctl {
   int parity;          // U[parity] holds the state u^n, U[parity^1] the iterate
-  int step;            // steps completed in the current nsp_step call
   int any;             // host-visible copy of the loop condition
   int nmem;
   int maxit;
@@ -132,11 +131,15 @@ struct Ctl {
   int* unconv;         // [nmem]: steps of the current call whose corrector loop stopped at
                        // maxit with err > tol (the reference moves on silently)
   int hist_cap;
-  int fault;           // nonzero: a device-side wait ran out and a kernel abandoned its work
   int hold;            // nonzero: a completed step keeps parity and step count (chunked
                        // steps: members advance chunk by chunk, then finish_step flips once)
   int inject;          // test hook (nsp_debug_inject): bit 0 -- the tensor-core transforms'
                        // operand-image barrier is never arrived on, so their bounded wait runs out
+  int pad;
+  // What a stepping call clears and reads back lies together: these two words, then (in the same
+  // allocation) unconv, status and hist -- one clear from `step`, one copy from `fault`.
+  int fault;           // nonzero: a device-side wait ran out and a kernel abandoned its work
+  int step;            // steps completed in the current nsp_step call
 };
 
 // Kernel launchers (nsp_transform.cu, nsp_linear.cu).
@@ -155,6 +158,9 @@ void launch_converge(Ctl* dctl, int nmem, unsigned long long cond_handle, int us
 // Completes a step taken in member chunks: parity flip and step count (converge_k's
 // completion work, held back while the chunks ran).
 void launch_finish_step(Ctl* dctl, cudaStream_t st);
+// Copies three components of n complex values each in one launch (16-byte aligned device
+// arrays); status: a member's status word to clear, or null.
+void launch_copy3(const double2* const (&src)[3], double2* const (&dst)[3], long long n, int* status, cudaStream_t st);
 void launch_lusolve(const Tables& tb, int kind, const double2* rhs, double2* sol, cudaStream_t st);
 void launch_fp64_peak(double* out, int blocks, int threads, int iters, cudaStream_t st);
 // max |div u| over the interior rows -> out[0], over the wall row -> out[1] (ordered bits);

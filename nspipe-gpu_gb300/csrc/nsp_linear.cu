@@ -1411,6 +1411,33 @@ void launch_converge(Ctl* dctl, int nmem, unsigned long long cond_handle, int us
   converge_k<<<1, 256, 0, st>>>(dctl, (cudaGraphConditionalHandle)cond_handle, use_cond);
 }
 
+// State hand-over of one member between device arrays: one launch instead of three copies (and
+// a clear), each of which costs a launch and a gap of ~2 us -- the size of the copies themselves
+// at NR=48 x 32 x 64 modes.  Four values in flight per thread.
+struct Copy3 {
+  const double2* src[3];
+  double2* dst[3];
+};
+__global__ void __launch_bounds__(256) copy3_k(Copy3 c, long long n, int* status) {
+  const double2* __restrict__ s = blockIdx.y == 0 ? c.src[0] : blockIdx.y == 1 ? c.src[1] : c.src[2];
+  double2* __restrict__ d = blockIdx.y == 0 ? c.dst[0] : blockIdx.y == 1 ? c.dst[1] : c.dst[2];
+  const long long h0 = blockIdx.x * 1024LL + threadIdx.x;
+  double2 v[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (h0 + 256 * k < n) v[k] = s[h0 + 256 * k];
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (h0 + 256 * k < n) d[h0 + 256 * k] = v[k];
+  if (status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0;
+}
+
+void launch_copy3(const double2* const (&src)[3], double2* const (&dst)[3], long long n, int* status, cudaStream_t st) {
+  Copy3 c;
+  for (int k = 0; k < 3; k++) c.src[k] = src[k], c.dst[k] = dst[k];
+  copy3_k<<<dim3((unsigned)((n + 1023) / 1024), 3), 256, 0, st>>>(c, n, status);
+}
+
 void launch_finish_step(Ctl* dctl, cudaStream_t st) { finish_step_k<<<1, 1, 0, st>>>(dctl); }
 
 void launch_lusolve(const Tables& tb, int kind, const double2* rhs, double2* sol, cudaStream_t st) {
