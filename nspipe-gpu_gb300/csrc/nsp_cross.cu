@@ -36,26 +36,44 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
 #pragma unroll
   for (int k = 0; k < KZ; k++) ms[k] = 0.0;
   for (int mu0 = 0; mu0 <= NT / 2; mu0 += NB) {
-    for (int b = threadIdx.x >> 5; b < NB; b += NTH / 32) {
+    const int nb = min(NB, NT / 2 + 1 - mu0);
+    // both lines of a pair copied asynchronously into the line they become (fx_z)
+    auto plus = [&](int mu) { return row + (size_t)mu * NZ; };
+    auto minus = [&](int mu) { return row + (size_t)(mu ? NT - mu : 0) * NZ; };  // (mu = NT/2: the same line, unused)
+    auto raw2 = [&](int q) { return q < NZ - 2 ? NZ + q : NZR - NZ + 2 + q; };
+    if constexpr (NZRC > 0) {
+      for (int b = threadIdx.x >> 5; b < nb; b += NTH / 32) {
+        cpx<fx>* Zt = Z + (size_t)b * ZP;
+        const double2 *P = plus(mu0 + b), *M = minus(mu0 + b);
+        for (int q = lane; q < NZ; q += 32) {
+          cp_async16(Zt + q, P + q);
+          cp_async16(Zt + raw2(q), M + q);
+        }
+      }
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncwarp();
+    }
+    for (int b = threadIdx.x >> 5; b < nb; b += NTH / 32) {
       const int mu = mu0 + b;
       cpx<fx>* Zt = Z + (size_t)b * ZP;
-      if (mu > NT / 2) {
-        for (int q = lane; q < NZR; q += 32) Zt[q] = mk<fx>(0, 0);
-        continue;
-      }
-      const double2* P = row + (size_t)mu * NZ;
-      const double2* M = row + (size_t)(mu ? NT - mu : 0) * NZ;  // (mu = NT/2: the same line, unused)
+      const double2* raw = reinterpret_cast<const double2*>(Zt);
+      const double2 *P = plus(mu), *M = minus(mu);
+      auto at_p = [&](int q) { return NZRC > 0 ? raw[q] : P[q]; };
+      auto at_m = [&](int q) { return NZRC > 0 ? raw[raw2(q)] : M[q]; };
       const bool pair = mu < NT / 2;
       FxSum sum;
+#pragma unroll 1
       for (int q = lane; q < NZ; q += 32) {
-        const double2 a = P[q], m = M[q];
+        const double2 a = at_p(q), m = at_m(q);
         sum.add(fx_key(a.x), fx_key(a.y));
         if (pair) sum.add(fx_key(m.x), fx_key(m.y));
       }
       const int E = sum.warp_exponent();
       if (lane == 0) sE[b] = E;
+#pragma unroll 1
       for (int q = lane; q < NZ; q += 32) {
-        const double2 a = P[q], m = M[q];
+        const double2 a = at_p(q), m = at_m(q);
         const cpx<fx> x = mk<fx>(fx_from(a.x, E), fx_from(a.y, E));
         const cpx<fx> y = pair ? mk<fx>(fx_from(m.x, E), -fx_from(m.y, E)) : mk<fx>(0, 0);
         if (q) {
@@ -65,22 +83,22 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
           Zt[0] = mk<fx>(fx_half(x.x + y.x), fx_half(x.y + y.y));
         }
       }
+      __syncwarp();  // the second line's slots have been read
       for (int q = NZ + lane; q <= NZR - NZ; q += 32) Zt[q] = mk<fx>(0, 0);
     }
     __syncthreads();
     if constexpr (NZRC > 0)
-      pass_fft<fx, +1, NZRC, NB, 1, line_pitch(NZRC), false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx);
+      pass_fft<fx, +1, NZRC, NB, 1, line_pitch(NZRC), false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx, nb);
     else
-      fft_batch<fx, +1, MAXRZ, false>(Z, tb.pz, NB, 1, NZR, tb.tw_zx);
-    const int nb = min(NB, NT / 2 + 1 - mu0);
+      fft_batch<fx, +1, MAXRZ, false>(Z, tb.pz, nb, 1, NZR, tb.tw_zx);
 #pragma unroll
     for (int k = 0; k < KZ; k++) {
       const int n = threadIdx.x + k * NTH;
       if (n < NZR)
         for (int b = 0; b < nb; b++) {
           const double2 v = fx_value(Z[(size_t)b * ZP + n], sE[b]);
-          if (mu0 + b == 0) ms[k] = v.x * v.x;
-          else ms[k] += 2.0 * (v.x * v.x + v.y * v.y);
+          if (mu0 + b == 0) ms[k] = 0.5 * (v.x * v.x);
+          else ms[k] = fma(v.x, v.x, fma(v.y, v.y, ms[k]));
         }
     }
     __syncthreads();
@@ -89,7 +107,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
 #pragma unroll
   for (int k = 0; k < KZ; k++) {
     const int n = threadIdx.x + k * NTH;
-    if (n < NZR) o[n] = ms[k];
+    if (n < NZR) o[n] = 2.0 * ms[k];
   }
 }
 

@@ -327,19 +327,22 @@ __host__ __device__ constexpr int line_res_store(int ns, int p) {
   return ns * p % 16 == 0 ? (ns < 16 ? ns : 16) : ns * p == 8 ? 8 + ns : 16;
 }
 
-// One Stockham pass of radix P over NB transforms of length N (see fft_stage_ct), in place:
+// One Stockham pass of radix P over NB transforms (contiguous lines: the first nb) of length N
+// (see fft_stage_ct), in place:
 // element e of transform t at t BS + e ES (COLS: neighbouring threads on neighbouring
 // transforms) or at t BS + e
 // (line_pad(e) between passes).  Elements [Z0, Z1] are known to be zero on the way in
 // (first pass), elements [D0, D1] not needed on the way out (last pass); empty if Z1 < Z0.
 template <typename T, int SIGN, int N, int NB, int ES, int BS, bool COLS, int NTH, int P, int NS, int Z0, int Z1, int D0, int D1>
-__device__ __forceinline__ void fft_pass(cpx<T>* buf, const typename vec2<T>::type* __restrict__ tw) {
+__device__ __forceinline__ void fft_pass(cpx<T>* buf, const typename vec2<T>::type* __restrict__ tw, int nb) {
   constexpr int NBF = N / P, TOTAL = NB * NBF, R = (TOTAL + NTH - 1) / NTH, TSTR = N / (NS * P);
+  const int total = COLS ? TOTAL : nb * NBF;
+  const bool full = (COLS || nb == NB) && TOTAL % NTH == 0;  // (constant where nb is)
   cpx<T> v[R][P];
 #pragma unroll
   for (int rr = 0; rr < R; rr++) {
     const int b = threadIdx.x + rr * NTH;
-    if (TOTAL % NTH == 0 || b < TOTAL) {
+    if (full || b < total) {
       const int t = COLS ? b % NB : b / NBF, j = COLS ? b / NB : b - t * NBF;
 #pragma unroll
       for (int q = 0; q < P; q++) {
@@ -355,7 +358,7 @@ __device__ __forceinline__ void fft_pass(cpx<T>* buf, const typename vec2<T>::ty
 #pragma unroll
   for (int rr = 0; rr < R; rr++) {
     const int b = threadIdx.x + rr * NTH;
-    if (TOTAL % NTH == 0 || b < TOTAL) {
+    if (full || b < total) {
       const int t = COLS ? b % NB : b / NBF, j = COLS ? b / NB : b - t * NBF;
       const int k = (NS == 1) ? 0 : j % NS;
       if (NS > 1) {
@@ -377,11 +380,11 @@ __device__ __forceinline__ void fft_pass(cpx<T>* buf, const typename vec2<T>::ty
 }
 
 template <typename T, int SIGN, int N, int NB, int ES, int BS, bool COLS, int NTH, int Z0, int Z1, int D0, int D1, int S = 0, int NS = 1>
-__device__ __forceinline__ void pass_fft(cpx<T>* buf, const typename vec2<T>::type* __restrict__ tw) {
+__device__ __forceinline__ void pass_fft(cpx<T>* buf, const typename vec2<T>::type* __restrict__ tw, int nb = NB) {
   constexpr int P = pass_radix(N, S, COLS);
   if constexpr (P > 0) {
-    fft_pass<T, SIGN, N, NB, ES, BS, COLS, NTH, P, NS, Z0, Z1, D0, D1>(buf, tw);
-    pass_fft<T, SIGN, N, NB, ES, BS, COLS, NTH, Z0, Z1, D0, D1, S + 1, NS * P>(buf, tw);
+    fft_pass<T, SIGN, N, NB, ES, BS, COLS, NTH, P, NS, Z0, Z1, D0, D1>(buf, tw, nb);
+    pass_fft<T, SIGN, N, NB, ES, BS, COLS, NTH, Z0, Z1, D0, D1, S + 1, NS * P>(buf, tw, nb);
   }
 }
 
