@@ -325,7 +325,7 @@ int reset_control(nsp_ctx* c) {
 // The z-stage kernel of each group (radix-stage or one of the two-pass splits compiled
 // for its length and precision), timed like the linear pass: z stage alone on the
 // group's buffers, best of 3 after a warm-up.  Cached per shape and precision,
-// "z1:NRxNTxNZ:pP", not per member count: the kernels differ in rounding, and members
+// "z2:NRxNTxNZ:pP", not per member count: the kernels differ in rounding, and members
 // of one shape give the same bits whatever ensemble they are stepped in.
 int autotune_z(nsp_ctx* c, std::map<std::string, int>& cache, bool* dirty) {
   const bool mixed = c->precision == NSP_MIXED;
@@ -338,7 +338,7 @@ int autotune_z(nsp_ctx* c, std::map<std::string, int>& cache, bool* dirty) {
     const int nv = z_variants(g.tb.NZR, g.tb.NTP, mixed);
     if (nv == 0) continue;
     char key[128];
-    snprintf(key, sizeof key, "z1:%dx%dx%d:p%d", g.tb.NR, g.tb.NT, g.tb.NZ, c->precision);
+    snprintf(key, sizeof key, "z2:%dx%dx%d:p%d", g.tb.NR, g.tb.NT, g.tb.NZ, c->precision);
     auto it = cache.find(key);
     if (it != cache.end() && it->second >= 0 && it->second <= nv) {
       g.tb.z_variant = it->second;

@@ -16,13 +16,19 @@ namespace nsp {
 
 __host__ __device__ __forceinline__ uint32_t f64_to_f32_bits(uint64_t b) {
   const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
-  const uint32_t sign = hi & 0x80000000u, e = (hi >> 20) & 0x7FFu;
-  if (e < 897u) return sign;  // below 2^-126: zero, double denormals, float denormal range
-  if (e == 0x7FFu) return sign | ((((hi & 0xFFFFFu) | lo) != 0u) ? 0x7FC00000u : 0x7F800000u);  // NaN, Inf
-  if (e > 1150u) return sign | 0x7F800000u;  // 2^128 and beyond: Inf
-  uint32_t f = ((e - 896u) << 23) | ((hi & 0xFFFFFu) << 3) | (lo >> 29);  // exponent rebias 1023 -> 127
-  const uint32_t rest = lo & 0x1FFFFFFFu;                                  // the 29 dropped mantissa bits
-  f += (rest > 0x10000000u) || (rest == 0x10000000u && (f & 1u));          // ties to even; may carry to Inf
+  const uint32_t sign = hi & 0x80000000u, x = ((hi >> 20) & 0x7FFu) - 897u;
+  // In range: 9 bits of the exponent and 23 of the mantissa by one funnel shift, the rebias
+  // 1023 -> 127 (-896 = -384 in 9 bits) and the rounding of the 29 dropped bits (ties to even; a
+  // carry may go to Inf) as additions.
+  uint32_t f = ((hi << 3) | (lo >> 29)) + 0x40000000u;
+  f += ((lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (f & 1u)) >> 29;
+  if (x > 253u) {
+    f = 0u;                      // below 2^-126: zero, double denormals, float denormal range
+    if ((int32_t)x > 253) {      // 2^128 and beyond: Inf, or NaN
+      const bool nan = x == 0x7FFu - 897u && ((hi & 0xFFFFFu) | lo) != 0u;
+      f = nan ? 0x7FC00000u : 0x7F800000u;
+    }
+  }
   return sign | f;
 }
 

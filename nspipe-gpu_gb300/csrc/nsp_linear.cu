@@ -283,6 +283,11 @@ __device__ __forceinline__ void solve_line_ring(V* X, int ld, const V* __restric
   __syncwarp(pair);
 }
 
+// First row of the 7 that stored row i of a stencil table spans: entry j belongs to row
+// base + j, with zeros where the stencil is cut short at the axis (its last entries) or the
+// wall (its first), so that the mixed passes' loops have a fixed length and no bounds.
+__device__ __forceinline__ int stencil_base(int i, int NR) { return min(max(i - IW, 0), NR - STEN); }
+
 // The low half of a line slot holds an FP32 pair in the increment passes.
 __device__ __forceinline__ float2& f32slot(double2* a, int e) { return reinterpret_cast<float2*>(a)[2 * e]; }
 // The mixed passes hold a line slot as two double-float parts (re.hi, re.lo, im.hi,
@@ -295,6 +300,15 @@ __device__ __forceinline__ void put_df(double2* a, int e, float x, float y) { df
 __device__ __forceinline__ float2 split_df(double x) {
   const float hi = f64_to_f32(x);
   return make_float2(hi, f64_to_f32(x - f32_to_f64(hi)));
+}
+__device__ __forceinline__ float2 split_df(double x, float hi) {  // hi = fl32(x) known
+  return make_float2(hi, f64_to_f32(x - f32_to_f64(hi)));
+}
+// fl32 of a double-float value: its high part, flushed like f64_to_f32 below 2^-126.
+__device__ __forceinline__ float df_f32(float hi) {
+  float f;
+  asm("mul.ftz.f32 %0, %1, 0f3F800000;" : "=f"(f) : "f"(hi));
+  return f;
 }
 __device__ __forceinline__ void put_df(double2* a, int e, double2 v) {
   const float2 x = split_df(v.x), y = split_df(v.y);
@@ -474,9 +488,12 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
         // per value adds u^n/dt.  The mean mode (k = 0) stays in FP64: its Laplacian is
         // steady, so FP32 rounding there would add up step after step.
         float2 fr = make_float2(0.f, 0.f), ft = fr, fz = fr;
-        for (int j = 0; j < len; j++) {
-          const float a = __ldg(Luc32 + lo + j), b = __ldg(Luc32 + le + j);
-          const int e = (left + j) * LM + mm;
+        const int cb = stencil_base(i, NR) * LM + mm;
+        const float *La = Luc32 + (1 - par_m) * STEN * NR + STEN * i, *Lb = Luc32 + par_m * STEN * NR + STEN * i;
+#pragma unroll
+        for (int j = 0; j < STEN; j++) {
+          const float a = __ldg(La + j), b = __ldg(Lb + j);
+          const int e = cb + j * LM;
           const float2 vr = T32[e], vt = T32[LN + e], vz = T32[2 * LN + e];
           fr.x = fmaf(a, vr.x, fr.x); fr.y = fmaf(a, vr.y, fr.y);
           ft.x = fmaf(a, vt.x, ft.x); ft.y = fmaf(a, vt.y, ft.y);
@@ -516,7 +533,8 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
           // widening on the integer pipe (the hardware conversion issues on the FP64 pipe)
           const double2 u = Un[c * S + h];
           if constexpr (DFS) {  // u^n/(2dt) + g in double-float: u^n split, the product and the sum exact
-            const float2 ux = split_df(u.x), uy = split_df(u.y);
+            // u^n's high part is its FP32 mirror (the same rounding), here in the tile
+            const float2 ux = split_df(u.x, T32[c * LN + p].x), uy = split_df(u.y, T32[c * LN + p].y);
             float sx = 0.f, tx = 0.f, sy = 0.f, ty = 0.f;
             df_add_prod(sx, tx, hidt_df, dfloat{ux.x, ux.y});
             df_add_prod(sy, ty, hidt_df, dfloat{uy.x, uy.y});
@@ -675,11 +693,12 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
     if constexpr (INC) {  // FP32 on the increment, into double-float for the solve
       float sx = 0.f, sy = 0.f;
       if (k < NTNZ && i < NR - 1) {
-        const int left = max(0, i - IW), right = min(i + IW, NR - 1), len = right + 1 - left, i0 = i + IW - right;
-        const float* Dr = tb.Ddiv32 + (1 - spar[mm]) * STEN * NR + STEN * i + i0;
-        for (int j = 0; j < len; j++) {
+        const int cb = stencil_base(i, NR) * LM + mm;
+        const float* Dr = tb.Ddiv32 + (1 - spar[mm]) * STEN * NR + STEN * i;
+#pragma unroll
+        for (int j = 0; j < STEN; j++) {
           const float de = __ldg(Dr + j);
-          const float2 a = f32slot(R, (left + j) * LM + mm);
+          const float2 a = f32slot(R, cb + j * LM);
           sx = fmaf(de, a.x, sx);
           sy = fmaf(de, a.y, sy);
         }
@@ -693,11 +712,12 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
     } else if constexpr (DFS) {  // mixed predictor: the same stencil in double-float
       float sx = 0.f, tx = 0.f, sy = 0.f, ty = 0.f;
       if (k < NTNZ && i < NR - 1) {
-        const int left = max(0, i - IW), right = min(i + IW, NR - 1), len = right + 1 - left, i0 = i + IW - right;
-        const float2* Dr = tb.Ddivdf + (1 - spar[mm]) * STEN * NR + STEN * i + i0;
-        for (int j = 0; j < len; j++) {
+        const int cb = stencil_base(i, NR) * LM + mm;
+        const float2* Dr = tb.Ddivdf + (1 - spar[mm]) * STEN * NR + STEN * i;
+#pragma unroll
+        for (int j = 0; j < STEN; j++) {
           const dfloat de = ld_df(Dr + j);
-          const float4 a = dfslot(R, (left + j) * LM + mm);
+          const float4 a = dfslot(R, cb + j * LM);
           df_add_prod(sx, tx, de, df_re(a));
           df_add_prod(sy, ty, de, df_im(a));
         }
@@ -788,12 +808,13 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
     double2 up = c2(0, 0), um = c2(0, 0), rz = c2(0, 0);
     if constexpr (INC) {  // FP32 on the increment; each thread reads its own slots and the P taps
       if (i < NR - 1) {
-        const int left = max(0, i - IW), right = min(i + IW, NR - 1), len = right + 1 - left, i0 = i + IW - right;
-        const float* Dr = tb.D32 + spar[mm] * STEN * NR + STEN * i + i0;
+        const int cb = stencil_base(i, NR) * LM + mm;
+        const float* Dr = tb.D32 + spar[mm] * STEN * NR + STEN * i;
         float2 rr = f32slot(R, p);
-        for (int j = 0; j < len; j++) {
+#pragma unroll
+        for (int j = 0; j < STEN; j++) {
           const float de = __ldg(Dr + j);
-          const float2 a = f32slot(P, (left + j) * LM + mm);
+          const float2 a = f32slot(P, cb + j * LM);
           rr.x = fmaf(-de, a.x, rr.x);
           rr.y = fmaf(-de, a.y, rr.y);
         }
@@ -811,13 +832,14 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       const dfloat z{0.f, 0.f};
       dfloat upx = z, upy = z, umx = z, umy = z, rzx = z, rzy = z;
       if (i < NR - 1) {
-        const int left = max(0, i - IW), right = min(i + IW, NR - 1), len = right + 1 - left, i0 = i + IW - right;
-        const float2* Dr = tb.Ddf + spar[mm] * STEN * NR + STEN * i + i0;
+        const int cb = stencil_base(i, NR) * LM + mm;
+        const float2* Dr = tb.Ddf + spar[mm] * STEN * NR + STEN * i;
         const float4 r0 = dfslot(R, p);
         float sx = r0.x, tx = r0.y, sy = r0.z, ty = r0.w;  // rr - d_r p
-        for (int j = 0; j < len; j++) {
+#pragma unroll
+        for (int j = 0; j < STEN; j++) {
           const dfloat de = ld_df(Dr + j);
-          const float4 a = dfslot(P, (left + j) * LM + mm);
+          const float4 a = dfslot(P, cb + j * LM);
           df_sub_prod(sx, tx, de, df_re(a));
           df_sub_prod(sy, ty, de, df_im(a));
         }
@@ -1120,7 +1142,13 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
         nonfin |= ((unsigned)__double2hiint(v.x) & EX) == EX || ((unsigned)__double2hiint(v.y) & EX) == EX;
         Ui[c * S + h] = v;
         if (Ui32) {
-          const float2 f = make_float2(f64_to_f32(v.x), f64_to_f32(v.y));  // integer-pipe rounding
+          float2 f;
+          if constexpr (DFS && !INC) {  // the high parts, still in the slot
+            const float4 d = dfslot(R, c * LN + p);
+            f = make_float2(df_f32(d.x), df_f32(d.z));
+          } else {
+            f = make_float2(f64_to_f32(v.x), f64_to_f32(v.y));  // integer-pipe rounding
+          }
           Ui32[c * S + h] = f;
           reinterpret_cast<float2*>(R + c * LN + p)[0] = f;  // FP32 copy for the d_r mirror below
         }
@@ -1147,14 +1175,22 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
     for (int p = tid; p < LN; p += nth) {
       const int i = p / LM, mm = p - i * LM, k = k0 + mm;
       if (k >= NTNZ) continue;
-      const int left = max(0, i - IW), right = min(i + IW, NR - 1), len = right + 1 - left, i0 = i + IW - right;
+      const int cb = stencil_base(i, NR) * LM + mm;
       const size_t h = (size_t)i * NTNZ + k;
       if (!NSP_IN_BOUNDS(tb, h, S, BC_LIN_POINT)) continue;
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const int tab = abs(spar[mm] - (c < 2 ? 1 : 0));
-        const float* Dr = tb.D32 + tab * STEN * NR + STEN * i + i0;
-        Udr32[c * S + h] = dr32_line(Dr, left, len, [&](int row) { return F[2 * (c * LN + row * LM + mm)]; });
+        const float* Dr = tb.D32 + tab * STEN * NR + STEN * i;
+        float vx = 0.f, vy = 0.f;  // (dr32_line's terms; the added ones are zero)
+#pragma unroll
+        for (int j = 0; j < STEN; j++) {
+          const float de = __ldg(Dr + j);
+          const float2 a = F[2 * (c * LN + cb + j * LM)];
+          vx += de * a.x;
+          vy += de * a.y;
+        }
+        Udr32[c * S + h] = make_float2(vx, vy);
       }
     }
   }

@@ -41,7 +41,7 @@ constexpr int MAXR = 4;   // register rounds of the run-time FFT
 // Theta columns per block: 32 while that gives a pass about as many butterflies as threads.
 constexpr int theta_cols(int ntp) { return ntp == 0 || ntp > 108 ? 16 : 32; }
 constexpr int TTH = 256;  // threads of the theta kernels
-constexpr int ZTH = 256;  // threads of the z kernel
+constexpr int ZTH = 256;  // threads of the run-time z kernel
 constexpr int Z2TH = 192; // threads of the two-pass z kernel (its passes run 192, 144, 384, 48, 36, 384 tasks)
 
 template <typename T> __device__ __forceinline__ const typename vec2<T>::type* tw_t(const Tables& tb);
@@ -138,58 +138,81 @@ __global__ void __launch_bounds__(TTH) nl_theta_inv(Tables tb, Bufs bf, const Ct
 // ---------------------------------------------------------------- z stage
 // Field order of the 12 physical arrays: u_r,u_t,u_z, dr u_r,dr u_t,dr u_z,
 // dt u_r,dt u_t,dt u_z, dz u_r,dz u_t,dz u_z.  Pair t holds fields (2t, 2t+1).
+//
+// In place: a warp writes a pair's packed Hermitian spectrum into its line, the passes
+// (nsp_fft.cuh) keep a thread's butterflies in registers between their loads and stores, so a
+// block holds 6 RPB lines and no second buffer.  That is what large lengths need: at 768 points
+// the two-pass kernel's two buffers leave one block of 192 threads on an SM (225 ns per member
+// and mode at NR=48 x 32, this kernel 162).  Below, the two-pass kernel's fewer trips through
+// shared memory win (192 points: 115 against 140; 576: 176 and 185); the autotuner chooses.
+// Threads about the butterflies of a pass; blocks per SM that the registers are limited for
+// (768 points: 192 x 5 162, 288 x 4 226, 384 x 2 with two rows 162).
+constexpr int zp_threads(int n) { return n == 0 ? 256 : n == 432 ? 288 : n >= 96 ? 192 : 96; }
+constexpr int zp_blocks(int n) { return n == 0 ? 1 : n == 432 ? 4 : n >= 96 ? 5 : 8; }
 template <typename T, int NZRC, int RPB>
-__global__ void __launch_bounds__(ZTH) nl_z(Tables tb, Bufs bf, const Ctl* ctl, int standalone) {
+__global__ void __launch_bounds__(zp_threads(NZRC), zp_blocks(NZRC)) nl_z(Tables tb, Bufs bf, const Ctl* ctl, int standalone) {
+  constexpr int NTH = zp_threads(NZRC);
   const int mloc = blockIdx.z, i = blockIdx.y, j0 = blockIdx.x * RPB;
   if (!standalone && ctl->phase[tb.mem0 + mloc] < 0) return;
   extern __shared__ __align__(16) unsigned char smraw[];
-  cpx<T>* Z = reinterpret_cast<cpx<T>*>(smraw);  // [RPB*6][NZR]
-  const int NR = tb.NR, NZ = tb.NZ, NTP = tb.NTP;
-  const int NZR = NZRC > 0 ? NZRC : tb.NZR;
+  cpx<T>* Z = reinterpret_cast<cpx<T>*>(smraw);  // [RPB*6] lines of ZP
+  const int NR = tb.NR, NTP = tb.NTP;
+  const int NZR = NZRC > 0 ? NZRC : tb.NZR, NZ = NZRC > 0 ? NZRC / 3 + 1 : tb.NZ;
+  const int ZP = NZRC > 0 ? line_pad(NZRC - 1) + 1 : NZR;
   const cpx<T>* G = reinterpret_cast<const cpx<T>*>(bf.G) + (size_t)mloc * 9 * NR * NTP * NZ;
   cpx<T>* H = reinterpret_cast<cpx<T>*>(bf.H) + (size_t)mloc * 3 * NR * NTP * NZ;
   const T kzs = tb_kzs<T>(tb);
+  const int lane = threadIdx.x & 31;
   // Hermitian-extended spectra, two real fields per complex transform.
-  for (int idx = threadIdx.x; idx < RPB * 6 * NZR; idx += ZTH) {
-    int q = idx % NZR, t = (idx / NZR) % 6, rr = idx / (6 * NZR);
-    int j = j0 + rr;
-    cpx<T> z = mk<T>(0, 0);
-    int qq = -1;
-    bool cj = false;
-    if (q < NZ) qq = q;
-    else if (q > NZR - NZ) { qq = NZR - q; cj = true; }
-    if (j < NTP && qq >= 0) {
-      cpx<T> ab[2];
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        int fld = 2 * t + h;
-        int src = fld < 9 ? fld : fld - 9;  // dz u_c comes from the u_c columns
-        const size_t gi = (((size_t)src * NR + i) * NTP + j) * NZ + qq;
-        cpx<T> g = NSP_IN_BOUNDS(tb, gi, (size_t)9 * NR * NTP * NZ, BC_Z_IN) ? G[gi] : mk<T>(0, 0);
-        if (fld >= 9) {
-          T kz = kzs * (T)qq;
-          g = mk<T>(-kz * g.y, kz * g.x);
-        }
-        if (qq == 0) g.y = (T)0;  // C2R ignores Im of the k_z = 0 coefficient
-        if (cj) g.y = -g.y;
-        ab[h] = g;
-      }
-      z = mk<T>(ab[0].x - ab[1].y, ab[0].y + ab[1].x);
+  for (int task = threadIdx.x >> 5; task < RPB * 6; task += NTH / 32) {
+    const int t = task % 6, rr = task / 6, j = j0 + rr;
+    cpx<T>* Zt = Z + (size_t)task * ZP;
+    if (j >= NTP || !NSP_IN_BOUNDS(tb, ((size_t)i * NTP + j) * NZ + NZ - 1, (size_t)NR * NTP * NZ, BC_Z_IN)) {
+      for (int q = lane; q < NZR; q += 32) Zt[q] = mk<T>(0, 0);
+      continue;
     }
-    Z[(size_t)(rr * 6 + t) * NZR + q] = z;
+    const int fa = 2 * t, fb = 2 * t + 1;  // dz u_c comes from the u_c columns
+    const cpx<T>* Ga = G + (((size_t)(fa < 9 ? fa : fa - 9) * NR + i) * NTP + j) * NZ;
+    const cpx<T>* Gb = G + (((size_t)(fb < 9 ? fb : fb - 9) * NR + i) * NTP + j) * NZ;
+    auto put = [&](int q, cpx<T> a, cpx<T> b) {
+      const T kz = kzs * (T)q;
+      if (fa >= 9) a = mk<T>(-kz * a.y, kz * a.x);
+      if (fb >= 9) b = mk<T>(-kz * b.y, kz * b.x);
+      if (q == 0) a.y = b.y = (T)0;  // C2R ignores Im of the k_z = 0 coefficient
+      Zt[q] = mk<T>(a.x - b.y, a.y + b.x);
+      if (q) Zt[NZR - q] = mk<T>(a.x + b.y, b.x - a.y);
+    };
+    constexpr int U = 4;  // loads in flight per lane and field
+    for (int q0 = 0; q0 < NZ; q0 += 32 * U) {
+      cpx<T> a[U], b[U];
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        const int q = q0 + 32 * k + lane;
+        if (q < NZ) a[k] = Ga[q], b[k] = Gb[q];
+      }
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        const int q = q0 + 32 * k + lane;
+        if (q < NZ) put(q, a[k], b[k]);
+      }
+    }
+    for (int q = NZ + lane; q <= NZR - NZ; q += 32) Zt[q] = mk<T>(0, 0);
   }
   __syncthreads();
-  if constexpr (NZRC > 0) fft_ct<T, +1, NZRC, RPB * 6, 1, NZRC, false, ZTH>(Z, tw_z<T>(tb));
-  else fft_batch<T, +1, MAXR, false>(Z, tb.pz, RPB * 6, 1, NZR, tw_z<T>(tb));
+  constexpr int NFWD = (RPB == 2) ? 3 : 2;
+  if constexpr (NZRC > 0)
+    pass_fft<T, +1, NZRC, RPB * 6, 1, line_pad(NZRC - 1) + 1, false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tw_z<T>(tb));
+  else
+    fft_batch<T, +1, MAXR, false>(Z, tb.pz, RPB * 6, 1, NZR, tw_z<T>(tb));
   // -(u.grad)u (calcNonlinear_k), packed for the forward transforms:
   // RPB 2: slot0 = (Nr0, Nt0), slot1 = (Nr1, Nt1), slot2 = (Nz0, Nz1); RPB 1: slot0 = (Nr, Nt), slot1 = (Nz, 0).
   const T rinv = tb_rinv<T>(tb, i);
-  for (int n = threadIdx.x; n < NZR; n += ZTH) {
+  for (int n = threadIdx.x; n < NZR; n += NTH) {
     T nr[RPB], nt[RPB], nz[RPB];
 #pragma unroll
     for (int rr = 0; rr < RPB; rr++) {
-      const cpx<T>* Zr = Z + (size_t)rr * 6 * NZR + n;
-      cpx<T> a0 = Zr[0], a1 = Zr[NZR], a2 = Zr[2 * NZR], a3 = Zr[3 * NZR], a4 = Zr[4 * NZR], a5 = Zr[5 * NZR];
+      const cpx<T>* Zr = Z + (size_t)rr * 6 * ZP + n;
+      cpx<T> a0 = Zr[0], a1 = Zr[ZP], a2 = Zr[2 * ZP], a3 = Zr[3 * ZP], a4 = Zr[4 * ZP], a5 = Zr[5 * ZP];
       T ur = a0.x, ut = a0.y, uz = a1.x;
       T drr = a1.y, drt = a2.x, drz = a2.y, dtr = a3.x, dtt = a3.y, dtz = a4.x, dzr = a4.y, dzt = a5.x, dzz = a5.y;
       T utr = ut * rinv;
@@ -199,31 +222,31 @@ __global__ void __launch_bounds__(ZTH) nl_z(Tables tb, Bufs bf, const Ctl* ctl, 
     }
     if (RPB == 2) {
       Z[n] = mk<T>(nr[0], nt[0]);
-      Z[NZR + n] = mk<T>(nr[RPB - 1], nt[RPB - 1]);
-      Z[2 * NZR + n] = mk<T>(nz[0], nz[RPB - 1]);
+      Z[ZP + n] = mk<T>(nr[RPB - 1], nt[RPB - 1]);
+      Z[2 * ZP + n] = mk<T>(nz[0], nz[RPB - 1]);
     } else {
       Z[n] = mk<T>(nr[0], nt[0]);
-      Z[NZR + n] = mk<T>(nz[0], (T)0);
+      Z[ZP + n] = mk<T>(nz[0], (T)0);
     }
   }
   __syncthreads();
-  constexpr int NFWD = (RPB == 2) ? 3 : 2;
-  if constexpr (NZRC > 0) fft_ct<T, -1, NZRC, NFWD, 1, NZRC, false, ZTH>(Z, tw_z<T>(tb));
-  else fft_batch<T, -1, MAXR, false>(Z, tb.pz, NFWD, 1, NZR, tw_z<T>(tb));
+  if constexpr (NZRC > 0)
+    pass_fft<T, -1, NZRC, NFWD, 1, line_pad(NZRC - 1) + 1, false, NTH, 0, -1, NZRC / 3, 2 * NZRC / 3>(Z, tw_z<T>(tb));
+  else
+    fft_batch<T, -1, MAXR, false>(Z, tb.pz, NFWD, 1, NZR, tw_z<T>(tb));
   // Unpack: x = a + i b  ->  A_q = (X_q + conj X_{-q})/2,  B_q = (X_q - conj X_{-q})/(2i).
   const int NQ = NZ - 1;
-  for (int idx = threadIdx.x; idx < RPB * 3 * NQ; idx += ZTH) {
-    int q = idx % NQ, c = (idx / NQ) % 3, rr = idx / (3 * NQ);
-    int j = j0 + rr;
+  for (int idx = threadIdx.x; idx < RPB * 3 * NQ; idx += NTH) {
+    const int q = idx % NQ, c = (idx / NQ) % 3, rr = idx / (3 * NQ), j = j0 + rr;
     if (j >= NTP) continue;
     int slot;
     bool takeB;
     if (c < 2) { slot = rr; takeB = (c == 1); }
     else { slot = (RPB == 2) ? 2 : 1; takeB = (RPB == 2) && rr == 1; }
-    const cpx<T>* X = Z + (size_t)slot * NZR;
-    cpx<T> xq = X[q], xm = X[(NZR - q) % NZR];
-    cpx<T> v = takeB ? mk<T>((T)0.5 * (xq.y + xm.y), (T)-0.5 * (xq.x - xm.x))
-                     : mk<T>((T)0.5 * (xq.x + xm.x), (T)0.5 * (xq.y - xm.y));
+    const cpx<T>* X = Z + (size_t)slot * ZP;
+    const cpx<T> xq = X[q], xm = X[q ? NZR - q : 0];
+    const cpx<T> v = takeB ? mk<T>((T)0.5 * (xq.y + xm.y), (T)-0.5 * (xq.x - xm.x))
+                           : mk<T>((T)0.5 * (xq.x + xm.x), (T)0.5 * (xq.y - xm.y));
     if (NSP_IN_BOUNDS(tb, (((size_t)c * NR + i) * NTP + j) * NZ + q, (size_t)3 * NR * NTP * NZ, BC_Z_OUT))
       H[(((size_t)c * NR + i) * NTP + j) * NZ + q] = v;
   }
@@ -534,9 +557,9 @@ static void launch_theta(const Tables& tb, const Bufs& bf, Ctl* dctl, const doub
 
 template <typename T, int NZRC, int RPB>
 static void launch_z(const Tables& tb, const Bufs& bf, Ctl* dctl, bool standalone, cudaStream_t st, int nm) {
-  size_t sm = sizeof(cpx<T>) * 6 * RPB * tb.NZR;
+  size_t sm = sizeof(cpx<T>) * 6 * RPB * (NZRC > 0 ? line_pad(NZRC - 1) + 1 : tb.NZR);
   dim3 g((tb.NTP + RPB - 1) / RPB, tb.NR, nm);
-  nl_z<T, NZRC, RPB><<<g, ZTH, sm, st>>>(tb, bf, dctl, standalone ? 1 : 0);
+  nl_z<T, NZRC, RPB><<<g, zp_threads(NZRC), sm, st>>>(tb, bf, dctl, standalone ? 1 : 0);
 }
 
 template <typename T, int NZRC, int N1, int N2, int R>
@@ -551,16 +574,18 @@ static void launch_z2(const Tables& tb, const Bufs& bf, Ctl* dctl, bool standalo
 }
 
 #define NSP_NTP_LIST(X) X(12) X(18) X(24) X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(192)
-#define NSP_NZR_LIST(X) X(24, 2) X(48, 2) X(96, 2) X(192, 2) X(384, 2) X(576, 1) X(768, 1)
+#define NSP_NZR_LIST(X) X(24, 2) X(36, 2) X(48, 2) X(54, 2) X(72, 2) X(96, 2) X(108, 2) X(144, 2) X(162, 2) \
+  X(192, 2) X(216, 2) X(288, 2) X(384, 1) X(432, 2) X(576, 1) X(768, 1)
 // Two-pass z stage: (NZR, N1, N2, rows per block); the setup-time autotuner picks among
-// the splits and the radix-stage kernel per shape.  Every 2^a 3^b length up to 432 that a
-// register pass of at most 24 points splits is here: the run-time kernel, bound by its index
+// the splits and the in-place passes per shape (which win at 432 and 768 points, so those have no
+// split).  Every other 2^a 3^b length up to 576 that a register pass of at most 24 points splits
+// is here: the run-time kernel, bound by its index
 // arithmetic, takes 1066 us where the 18 x 9 split takes 89 (7 members of NR=61, 36 x 54
 // modes); its theta transforms (NTP = 54) 274 and 85 us where the compiled ones take 80 and 27.
 #define NSP_Z2_LIST(X) X(24, 4, 6, 2) X(36, 6, 6, 2) X(48, 8, 6, 2) X(54, 9, 6, 2) X(72, 12, 6, 2) \
   X(108, 9, 12, 2) X(108, 12, 9, 2) X(144, 12, 12, 2) X(162, 9, 18, 2) X(162, 18, 9, 2) X(216, 18, 12, 2) \
-  X(288, 16, 18, 2) X(288, 12, 24, 2) X(432, 18, 24, 2) X(432, 24, 18, 2) X(96, 8, 12, 2) X(96, 12, 8, 2) X(192, 16, 12, 2) \
-  X(192, 12, 16, 2) X(384, 16, 24, 2) X(384, 24, 16, 2) X(576, 24, 24, 2) X(768, 32, 24, 2) X(768, 24, 32, 2)
+  X(288, 16, 18, 2) X(288, 12, 24, 2) X(96, 8, 12, 2) X(96, 12, 8, 2) X(192, 16, 12, 2) \
+  X(192, 12, 16, 2) X(384, 16, 24, 2) X(384, 24, 16, 2) X(576, 24, 24, 2)
 
 int z_variants(int NZR, int NTP, bool fp32) {
   int n = 0;
@@ -580,9 +605,9 @@ int z_default_variant(int NZR, int NTP, bool fp32) {
 
 std::string z_variant_name(int NZR, int NTP, bool fp32, int v) {
   if (!fp32) return "radix, 64-bit fixed point";
-  if (v <= 0) return "radix";
+  if (v <= 0) return "in-place passes";
   int k = 0;
-  std::string s = "radix";
+  std::string s = "in-place passes";
 #define NSP_Z2_NAME(len, a, b, r) \
   if (NZR == len && NTP % r == 0 && ++k == v) s = "two-pass " #a "x" #b;
   NSP_Z2_LIST(NSP_Z2_NAME)
