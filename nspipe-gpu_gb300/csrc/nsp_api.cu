@@ -192,8 +192,8 @@ Tables member_view(const Group& g, int slot) {
   t.fac += (size_t)ps * 4 * t.NR * NFAC * t.NTNZ;
   t.V += (size_t)ps * 3 * t.S;
   if (t.V32) t.V32 += (size_t)ps * 3 * t.S;
-  if (t.facdf) t.facdf += (size_t)ps * 4 * t.NR * NFAC * t.NTNZ;
-  if (t.fac32) t.fac32 += (size_t)ps * 4 * t.NR * NFAC * t.NTNZ;
+  if (t.facdf) t.facdf += (size_t)ps * 4 * t.NR * NPACK * t.NTNZ;
+  if (t.fac32) t.fac32 += (size_t)ps * 4 * t.NR * NPACK * t.NTNZ;
   if (t.Vdf) t.Vdf += (size_t)ps * 2 * 3 * t.S;
   t.Luc += (size_t)ps * 2 * STEN * t.NR;
   t.Luc32 += (size_t)ps * 2 * STEN * t.NR;
@@ -387,7 +387,7 @@ int autotune(nsp_ctx* c) {
   CK(cudaEventCreate(&e1));
   for (auto& g : c->groups) {
     char key[128];
-    snprintf(key, sizeof key, "v2:%dx%dx%d:m%d:p%d", g.tb.NR, g.tb.NT, g.tb.NZ, g.tb.nmem, c->precision);
+    snprintf(key, sizeof key, "v3:%dx%dx%d:m%d:p%d", g.tb.NR, g.tb.NT, g.tb.NZ, g.tb.nmem, c->precision);
     const std::string key_inc = std::string(key) + ":inc";
     auto it = cache.find(key), it_inc = cache.find(key_inc);
     const bool mixed = c->precision == NSP_MIXED;
@@ -799,13 +799,14 @@ int nsp_setup(nsp_ctx* c) {
     if (c->precision == NSP_MIXED) {
       // the increment passes' FP32 correction profiles; the double-float factors, correction
       // profiles and stencils of the linear passes
+      const size_t pack_n = fac_n / NFAC * NPACK;
       float2 *v32 = nullptr, *fdf = nullptr, *vdf = nullptr;
       float* f32 = nullptr;
-      if ((rc = dalloc(c, &v32, sizeof(float2) * V_n)) || (rc = dalloc(c, &fdf, sizeof(float2) * fac_n)) ||
-          (rc = dalloc(c, &vdf, sizeof(float2) * 2 * V_n)) || (rc = dalloc(c, &f32, sizeof(float) * fac_n)))
+      if ((rc = dalloc(c, &v32, sizeof(float2) * V_n)) || (rc = dalloc(c, &fdf, sizeof(float2) * pack_n)) ||
+          (rc = dalloc(c, &vdf, sizeof(float2) * 2 * V_n)) || (rc = dalloc(c, &f32, sizeof(float) * pack_n)))
         return rc;
       launch_to_f32(tb.V, v32, (long long)V_n, c->st);
-      launch_split_fac(tb.fac, fdf, f32, (long long)fac_n, (int)NTNZ, c->st);
+      launch_split_fac(tb.fac, fdf, f32, (long long)(fac_n / NFAC), (int)NTNZ, c->st);
       launch_split_df(reinterpret_cast<const double*>(tb.V), vdf, 2 * (long long)V_n, c->st);
       CK(cudaGetLastError());
       tb.V32 = v32;

@@ -70,7 +70,11 @@ template <typename T, int SIGN, int P> __device__ __forceinline__ void dft(cpx<T
   }
 }
 
-// Groups of asynchronous global -> shared copies (cp.async) and their waits.
+// 16-byte asynchronous copies global -> shared (cp.async), groups of copies and their waits.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }

@@ -214,11 +214,6 @@ constexpr int z_blocks(int n) {
 
 // Values per line in shared memory: the gaps between passes, at least two behind the line.
 constexpr int line_pitch(int n) { return line_pad(n - 1) + 1 > n + 2 ? line_pad(n - 1) + 1 : n + 2; }
-// 16-byte asynchronous copies global -> shared, their groups and waits.
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
 // Compiled z lengths and theta rows per block: two (three packed forward transforms for both)
 // while the six lines of each leave three blocks on an SM.
 #define NSP_NZR_LIST(X) X(24, 2) X(36, 2) X(48, 2) X(54, 2) X(72, 2) X(96, 2) X(108, 2) X(144, 2) X(162, 2) \

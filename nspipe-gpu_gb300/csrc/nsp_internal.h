@@ -13,6 +13,7 @@ constexpr double PI2 = 6.283185307179586;  // the reference's 2*pi literal (head
 constexpr int STEN = 7;                     // radial stencil width (head.h:44)
 constexpr int IW = 3;                       // half stencil (head.h:45)
 constexpr int NFAC = 7;                     // stored factor entries per row: L(i-3..i-1), 1/U_ii, U(i+1..i+3)
+constexpr int NPACK = 8;                    // the same in the mixed form's tables: L(i-3..i-1), 0, U(i+3..i+1), 1/U_ii
 constexpr int MAXPLAN = 12;                 // radix stages of one transform length
 
 // FFT plan for one length: radices applied in order (Stockham, natural order out).
@@ -53,7 +54,8 @@ struct Tables {
   const double* fac;   // [4][NR][7][NTNZ]: banded LU factors of u+, u-, u_z, p
   const double2* V;    // [3][NR][NTNZ]: influence-matrix correction profiles (+, -, z)
   const float2* V32;   // mixed form: the same in FP32 (the corrector increments' correction)
-  const float2* facdf;  // mixed form: fac as double-float pairs (hi, lo), backward entries divided by U_ii
+  const float2* facdf;  // mixed form: fac as double-float pairs (hi, lo), [4][NR][NTNZ][NPACK], backward entries
+                        // divided by U_ii
   const float* fac32;   // mixed form: the same in FP32 (the increment passes' Helmholtz solves)
   const float2* Vdf;    // mixed form: V as double-float pairs, real and imaginary part of each entry
   const float2* Ddf;    // mixed form: D, Ddiv and 1/r as double-float pairs (the predictor's stencils)

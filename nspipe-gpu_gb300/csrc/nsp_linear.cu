@@ -104,9 +104,11 @@ __device__ __forceinline__ dfloat ldf(const dfloat* p) {
 // real, so the real and imaginary parts are independent solves and two threads can
 // share a line), V = dfloat one part in double-float with the factors F = dfloat.
 // Factor rows are fetched four at a time so that their L2 latencies overlap.
-template <typename V, typename F>
+// PACK: the mixed form's tables, whose rows hold a mode's factors together (split_fac_k).
+template <bool PACK, typename V, typename F>
 __device__ __forceinline__ void solve_line(V* X, int ld, const F* __restrict__ f, int NTNZ, int NR) {
-  const size_t rs = (size_t)NFAC * NTNZ;  // row stride of the factor table
+  const size_t rs = (size_t)(PACK ? NPACK : NFAC) * NTNZ;  // row stride of the factor table
+  auto at = [NTNZ](const F* fr, int e) { return PACK ? fr + (e < 3 ? e : 10 - e) : fr + (size_t)e * NTNZ; };
   V xm1{}, xm2{}, xm3{};
   int i = 0;
   for (; i + 4 <= NR; i += 4) {
@@ -115,7 +117,7 @@ __device__ __forceinline__ void solve_line(V* X, int ld, const F* __restrict__ f
 #pragma unroll
     for (int r = 0; r < 4; r++) {
       const F* fr = f + (i + r) * rs;
-      l[r][0] = ldf(fr); l[r][1] = ldf(fr + NTNZ); l[r][2] = ldf(fr + 2 * NTNZ);
+      l[r][0] = ldf(at(fr, 0)); l[r][1] = ldf(at(fr, 1)); l[r][2] = ldf(at(fr, 2));
       b[r] = X[(i + r) * ld];
     }
 #pragma unroll
@@ -126,7 +128,7 @@ __device__ __forceinline__ void solve_line(V* X, int ld, const F* __restrict__ f
   }
   for (; i < NR; i++) {
     const F* fr = f + i * rs;
-    F l[3] = {ldf(fr), ldf(fr + NTNZ), ldf(fr + 2 * NTNZ)};
+    F l[3] = {ldf(at(fr, 0)), ldf(at(fr, 1)), ldf(at(fr, 2))};
     V x = X[i * ld];
     fwd_row(x, l, xm1, xm2, xm3);
     X[i * ld] = x;
@@ -139,8 +141,8 @@ __device__ __forceinline__ void solve_line(V* X, int ld, const F* __restrict__ f
 #pragma unroll
     for (int r = 0; r < 4; r++) {
       const F* fr = f + (i - r) * rs;
-      u[r][0] = ldf(fr + 6 * NTNZ); u[r][1] = ldf(fr + 5 * NTNZ);
-      u[r][2] = ldf(fr + 4 * NTNZ); u[r][3] = ldf(fr + 3 * NTNZ);
+      u[r][0] = ldf(at(fr, 6)); u[r][1] = ldf(at(fr, 5));
+      u[r][2] = ldf(at(fr, 4)); u[r][3] = ldf(at(fr, 3));
       b[r] = X[(i - r) * ld];
     }
 #pragma unroll
@@ -151,21 +153,17 @@ __device__ __forceinline__ void solve_line(V* X, int ld, const F* __restrict__ f
   }
   for (; i >= 0; i--) {
     const F* fr = f + i * rs;
-    F u[4] = {ldf(fr + 6 * NTNZ), ldf(fr + 5 * NTNZ), ldf(fr + 4 * NTNZ), ldf(fr + 3 * NTNZ)};
+    F u[4] = {ldf(at(fr, 6)), ldf(at(fr, 5)), ldf(at(fr, 4)), ldf(at(fr, 3))};
     V x = X[i * ld];
     bwd_row(x, u, xp1, xp2, xp3);
     X[i * ld] = x;
   }
 }
 
-// 8-byte asynchronous copies global -> shared (cp.async), their groups and waits.
+// 8- and 16-byte asynchronous copies global -> shared (cp.async).
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
 
@@ -186,33 +184,55 @@ inline size_t ring_extra(int NR, int LM) {
   return tile > pl + rings ? tile - pl : rings;
 }
 
-// solve_line<V, V> (V = dfloat: double-float; V = float: FP32, the increment pass's
+// solve_line<true, V, V> (V = dfloat: double-float; V = float: FP32, the increment pass's
 // Helmholtz solves) with the factor rows staged through a shared-memory ring:
 // the copies of batch b + RB - 1 are in flight while batch b computes, so the rows
-// wait on shared memory instead of L2.  The two threads of a line (part 0 and 1, adjacent
-// lanes, both calling) share the copies -- part 0 fetches slots 0-1, part 1 slots 2-3 --
-// and meet at __syncwarp(pair) after each wait and before a slot is refilled.  Slots:
-// forward L(i-3), L(i-2), L(i-1); backward U(i+3), U(i+2), U(i+1), 1/U_ii.  Rows past the
-// last full batch read the table directly.  RB: ring depth in batches; RS: element
-// stride of the ring (2: the free upper halves of line slots that hold FP32 pairs).
+// wait on shared memory instead of L2.  A row's four factors of a mode lie together in the
+// table and in the ring (forward L(i-3), L(i-2), L(i-1), unused; backward U(i+3), U(i+2),
+// U(i+1), 1/U_ii): one 16-byte copy and one or two vector loads per thread and row, where
+// factors apart by mode took two copies and four loads with an address each -- the solves are
+// bound by their instructions (predictor / corrector pass of 28 pipes of three shapes: 2394 /
+// 1717 -> 2299 / 1649 us).  The two
+// threads of a line (part 0 and 1, adjacent lanes, both calling) share the copies -- halves of
+// a double-float row, alternate FP32 rows -- and meet at __syncwarp(pair) after each wait and
+// before a slot is refilled.  Rows past the last full batch read the table directly.  RB: ring
+// depth in batches; RS: element stride of the ring (2: the free upper halves of line slots
+// that hold FP32 pairs, filled in 8-byte copies).
 template <int LM, int RB, int RS, typename V>
 __device__ __forceinline__ void solve_line_ring(V* X, int ld, const V* __restrict__ f, int NTNZ, int NR,
                                                 V* ring, int mm, int part, unsigned pair) {
-  const size_t rs = (size_t)NFAC * NTNZ;
+  static_assert(RS == 1 || sizeof(V) == 8, "the strided ring holds double-float factors");
+  const size_t rs = (size_t)NPACK * NTNZ;
   const int nb = NR / 4;
-  auto at = [&](int b, int e) { return ring + (((b % RB) * 16 + e) * LM + mm) * RS; };
+  auto at = [&](int b, int r, int e) {
+    return RS == 1 ? ring + (((b % RB) * 4 + r) * LM + mm) * 4 + e : ring + (((b % RB) * 16 + r * 4 + e) * LM + mm) * RS;
+  };
   auto issue = [&](int b, bool fwd) {
+    const V* src = f + (fwd ? 4 * b : NR - 1 - 4 * b) * rs + (fwd ? 0 : 4);
 #pragma unroll
     for (int r = 0; r < 4; r++) {
-      const int row = fwd ? 4 * b + r : NR - 1 - 4 * b - r;
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        const int slot = 2 * part + q, e = fwd ? slot : 6 - slot;
-        if (!fwd || slot < 3) {
-          if constexpr (sizeof(V) == 8) cp_async8(at(b, r * 4 + slot), f + row * rs + (size_t)e * NTNZ);
-          else cp_async4(at(b, r * 4 + slot), f + row * rs + (size_t)e * NTNZ);
-        }
+      if constexpr (sizeof(V) == 4) {
+        if ((r & 1) == part) cp_async16(at(b, r, 0), src);
+      } else if constexpr (RS == 1) {
+        cp_async16(at(b, r, 2 * part), src + 2 * part);
+      } else {
+        cp_async8(at(b, r, 2 * part), src + 2 * part);
+        if (!fwd || part == 0) cp_async8(at(b, r, 2 * part + 1), src + 2 * part + 1);
       }
+      src = fwd ? src + rs : src - rs;
+    }
+  };
+  // a row's four factors from the ring
+  auto load = [&](int b, int r, V (&l)[4]) {
+    if constexpr (sizeof(V) == 4) {
+      const float4 v = *reinterpret_cast<const float4*>(at(b, r, 0));
+      l[0] = v.x; l[1] = v.y; l[2] = v.z; l[3] = v.w;
+    } else if constexpr (RS == 1) {
+      const float4 v = *reinterpret_cast<const float4*>(at(b, r, 0)), w = *reinterpret_cast<const float4*>(at(b, r, 2));
+      l[0] = V{v.x, v.y}; l[1] = V{v.z, v.w}; l[2] = V{w.x, w.y}; l[3] = V{w.z, w.w};
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++) l[j] = *at(b, r, j);
     }
   };
   V xm1{}, xm2{}, xm3{};
@@ -226,11 +246,10 @@ __device__ __forceinline__ void solve_line_ring(V* X, int ld, const V* __restric
     cp_async_commit();
     cp_async_wait<RB - 1>();
     __syncwarp(pair);
-    V l[4][3], x[4];
+    V l[4][4], x[4];
 #pragma unroll
     for (int r = 0; r < 4; r++) {
-#pragma unroll
-      for (int j = 0; j < 3; j++) l[r][j] = *at(b, r * 4 + j);
+      load(b, r, l[r]);
       x[r] = X[(4 * b + r) * ld];
     }
 #pragma unroll
@@ -242,7 +261,7 @@ __device__ __forceinline__ void solve_line_ring(V* X, int ld, const V* __restric
   }
   for (int i = 4 * nb; i < NR; i++) {
     const V* fr = f + i * rs;
-    V l[3] = {ldf(fr), ldf(fr + NTNZ), ldf(fr + 2 * NTNZ)};
+    V l[3] = {ldf(fr), ldf(fr + 1), ldf(fr + 2)};
     V x = X[i * ld];
     fwd_row(x, l, xm1, xm2, xm3);
     X[i * ld] = x;
@@ -261,8 +280,7 @@ __device__ __forceinline__ void solve_line_ring(V* X, int ld, const V* __restric
     V u[4][4], x[4];
 #pragma unroll
     for (int r = 0; r < 4; r++) {
-#pragma unroll
-      for (int j = 0; j < 4; j++) u[r][j] = *at(b, r * 4 + j);
+      load(b, r, u[r]);
       x[r] = X[(NR - 1 - 4 * b - r) * ld];
     }
 #pragma unroll
@@ -274,7 +292,7 @@ __device__ __forceinline__ void solve_line_ring(V* X, int ld, const V* __restric
   }
   for (int i = NR - 1 - 4 * nb; i >= 0; i--) {
     const V* fr = f + i * rs;
-    V u[4] = {ldf(fr + 6 * NTNZ), ldf(fr + 5 * NTNZ), ldf(fr + 4 * NTNZ), ldf(fr + 3 * NTNZ)};
+    V u[4] = {ldf(fr + 4), ldf(fr + 5), ldf(fr + 6), ldf(fr + 7)};
     V x = X[i * ld];
     bwd_row(x, u, xp1, xp2, xp3);
     X[i * ld] = x;
@@ -755,6 +773,9 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
   // (two threads per mode line: real and imaginary parts; every lane of the warp busy)
   // The last factor a solve reads of kind c, mode k: row NR-1, entry 6.
   auto fac_ok = [&](int c, int k) {
+    if (DFS)
+      return NSP_IN_BOUNDS(tb, (((size_t)c * NR + NR - 1) * NTNZ + k) * NPACK + NPACK - 1, (size_t)4 * NR * NPACK * NTNZ,
+                           BC_LIN_FACTOR);
     return NSP_IN_BOUNDS(tb, ((size_t)c * NR + NR - 1) * NFAC * NTNZ + 6 * (size_t)NTNZ + k,
                          (size_t)4 * NR * NFAC * NTNZ, BC_LIN_FACTOR);
   };
@@ -771,12 +792,12 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
     }
   }
   // Mixed form: the pressure solve in double-float (nsp_df.cuh), the factors split the same way.
-  const dfloat* facdf = reinterpret_cast<const dfloat*>(tb.facdf) + (size_t)ps * 4 * NR * NFAC * NTNZ;
+  const dfloat* facdf = reinterpret_cast<const dfloat*>(tb.facdf) + (size_t)ps * 4 * NR * NPACK * NTNZ;
   if (tid < 2 * LM) {
     const int mm = tid >> 1, part = tid & 1;
     if (k0 + mm < NTNZ && fac_ok(3, k0 + mm)) {
       dfloat* X = reinterpret_cast<dfloat*>(P + mm) + part;
-      const dfloat* fp = facdf + 3 * (size_t)NR * NFAC * NTNZ + k0 + mm;
+      const dfloat* fp = facdf + (3 * (size_t)NR * NTNZ + k0 + mm) * NPACK;
       const unsigned pair = 3u << ((tid & 31) & ~1);
       if constexpr (INC) {
         // the increment pass's lines hold FP32 pairs here: a deep ring in their slots'
@@ -788,7 +809,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       } else if constexpr (DFS)
         solve_line_ring<LM, RING_B, 1>(X, 2 * LM, fp, NTNZ, NR, ringD, mm, part, pair);
       else
-        solve_line(reinterpret_cast<double*>(P + mm) + part, 2 * LM, fac + 3 * (size_t)NR * NFAC * NTNZ + k0 + mm,
+        solve_line<false>(reinterpret_cast<double*>(P + mm) + part, 2 * LM, fac + 3 * (size_t)NR * NFAC * NTNZ + k0 + mm,
                    NTNZ, NR);
     }
   }
@@ -896,15 +917,15 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       if constexpr (INC)  // FP32 on the hi parts (lo stays 0): an increment of a well-conditioned operator;
                           // FP32 factors, so twice the batches in a ring of the same bytes
         solve_line_ring<LM, 2 * RING_B, 1>(reinterpret_cast<float*>(R + c * LN + mm) + 2 * part, 4 * LM,
-                            tb.fac32 + (size_t)ps * 4 * NR * NFAC * NTNZ + (size_t)c * NR * NFAC * NTNZ + k0 + mm,
+                            tb.fac32 + (((size_t)ps * 4 + c) * NR * NTNZ + k0 + mm) * NPACK,
                             NTNZ, NR, reinterpret_cast<float*>(ringF) + (size_t)c * 2 * RING_B * 16 * LM, mm, part,
                             3u << ((tid & 31) & ~1));
       else if constexpr (DFS)
         solve_line_ring<LM, RING_B, 1>(reinterpret_cast<dfloat*>(R + c * LN + mm) + part, 2 * LM,
-                            facdf + (size_t)c * NR * NFAC * NTNZ + k0 + mm, NTNZ, NR,
+                            facdf + ((size_t)c * NR * NTNZ + k0 + mm) * NPACK, NTNZ, NR,
                             ringF + (size_t)c * RING_B * 16 * LM, mm, part, 3u << ((tid & 31) & ~1));
       else
-        solve_line(reinterpret_cast<double*>(R + c * LN + mm) + part, 2 * LM,
+        solve_line<false>(reinterpret_cast<double*>(R + c * LN + mm) + part, 2 * LM,
                    fac + (size_t)c * NR * NFAC * NTNZ + k0 + mm, NTNZ, NR);
     }
   }
@@ -1350,7 +1371,7 @@ __global__ void lusolve_k(Tables tb, int kind, const double2* rhs, double2* sol)
   if (kind < 4) {
     if (k >= tb.NTNZ) return;
     for (int i = 0; i < tb.NR; i++) sol[(size_t)i * tb.NTNZ + k] = rhs[(size_t)i * tb.NTNZ + k];
-    solve_line(sol + k, tb.NTNZ, tb.fac + fo + k, tb.NTNZ, tb.NR);
+    solve_line<false>(sol + k, tb.NTNZ, tb.fac + fo + k, tb.NTNZ, tb.NR);
     return;
   }
   const int part = k & 1;
@@ -1365,7 +1386,8 @@ __global__ void lusolve_k(Tables tb, int kind, const double2* rhs, double2* sol)
     const float hi = f64_to_f32(x);
     X[h] = dfloat{hi, f64_to_f32(x - f32_to_f64(hi))};
   }
-  solve_line(X + 2 * (size_t)k, 2 * tb.NTNZ, reinterpret_cast<const dfloat*>(tb.facdf) + fo + k, tb.NTNZ, tb.NR);
+  solve_line<true>(X + 2 * (size_t)k, 2 * tb.NTNZ,
+                   reinterpret_cast<const dfloat*>(tb.facdf) + ((size_t)(kind & 3) * tb.NR * tb.NTNZ + k) * NPACK, tb.NTNZ, tb.NR);
   for (int i = 0; i < tb.NR; i++) {
     const size_t h = 2 * ((size_t)i * tb.NTNZ + k);
     const dfloat v = X[h];

@@ -791,19 +791,24 @@ void launch_split_df(const double* src, float2* dst, long long n, cudaStream_t s
   split_df_k<<<blocks, 256, 0, st>>>(src, dst, n);
 }
 
-// The banded-LU factor tables [kk][NR][NFAC][NTNZ] in double-float and FP32 for the
-// mixed form's solves, with the backward entries U(i, i+j) (entries 4..6) pre-divided by
-// U_ii (times entry 3, 1/U_ii): a backward row is then x_i = y_i / U_ii - sum U'_ij x_j,
-// the division applied to y_i off the row-to-row dependency chain.
+// The banded-LU factor tables [kk][NR][NFAC][NTNZ] in double-float and FP32 for the mixed
+// form's solves, [kk][NR][NTNZ][NPACK]: a row's factors of a mode together, in the order the
+// solves use them (L(i-3), L(i-2), L(i-1), 0, U(i+3), U(i+2), U(i+1), 1/U_ii).  The backward
+// entries U(i, i+j) are pre-divided by U_ii: a backward row is then x_i = y_i / U_ii -
+// sum U'_ij x_j, the division applied to y_i off the row-to-row dependency chain.  n: rows
+// times modes.
 __global__ void split_fac_k(const double* __restrict__ fac, float2* __restrict__ dfo, float* __restrict__ f32o,
                             long long n, int NTNZ) {
   for (long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x; h < n; h += (long long)gridDim.x * blockDim.x) {
-    const long long k = h % NTNZ, re = h / NTNZ, e = re % NFAC;
-    double x = fac[h];
-    if (e >= 4) x *= fac[(re - e + 3) * NTNZ + k];
-    const float hi = f64_to_f32(x);
-    dfo[h] = make_float2(hi, f64_to_f32(x - f32_to_f64(hi)));
-    f32o[h] = hi;
+    const double* f = fac + h / NTNZ * NFAC * NTNZ + h % NTNZ;
+    const double d = f[3 * (long long)NTNZ];
+#pragma unroll
+    for (int e = 0; e < NPACK; e++) {
+      const double x = e < 3 ? f[(long long)e * NTNZ] : e == 3 ? 0.0 : e < 7 ? f[(long long)(10 - e) * NTNZ] * d : d;
+      const float hi = f64_to_f32(x);
+      dfo[h * NPACK + e] = make_float2(hi, f64_to_f32(x - f32_to_f64(hi)));
+      f32o[h * NPACK + e] = hi;
+    }
   }
 }
 
