@@ -160,15 +160,10 @@ __device__ __forceinline__ void solve_line(V* X, int ld, const F* __restrict__ f
   }
 }
 
-// 8- and 16-byte asynchronous copies global -> shared (cp.async).
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
 
 // Depth of the factor ring of the double-float solves, in batches of four rows, and of
-// the increment pass's pressure ring, which lives in its lines' free upper halves.
+// the increment pass's pressure ring, which lives in the half of its lines that FP32 leaves free.
 constexpr int RING_B = 3;
 constexpr int RING_DEEP = 8;
 // Shared memory of one kind's ring: [RING_B][4 rows][4 slots][LM] double-float factors.
@@ -196,16 +191,14 @@ inline size_t ring_extra(int NR, int LM) {
 // threads of a line (part 0 and 1, adjacent lanes, both calling) share the copies -- halves of
 // a double-float row, alternate FP32 rows -- and meet at __syncwarp(pair) after each wait and
 // before a slot is refilled.  Rows past the last full batch read the table directly.  RB: ring
-// depth in batches; RS: element stride of the ring (2: the free upper halves of line slots
-// that hold FP32 pairs, filled in 8-byte copies).
-template <int LM, int RB, int RS, typename V>
+// depth in batches.
+template <int LM, int RB, typename V>
 __device__ __forceinline__ void solve_line_ring(V* X, int ld, const V* __restrict__ f, int NTNZ, int NR,
                                                 V* ring, int mm, int part, unsigned pair) {
-  static_assert(RS == 1 || sizeof(V) == 8, "the strided ring holds double-float factors");
   const size_t rs = (size_t)NPACK * NTNZ;
   const int nb = NR / 4;
   auto at = [&](int b, int r, int e) {
-    return RS == 1 ? ring + (((b % RB) * 4 + r) * LM + mm) * 4 + e : ring + (((b % RB) * 16 + r * 4 + e) * LM + mm) * RS;
+    return ring + (((b % RB) * 4 + r) * LM + mm) * 4 + e;
   };
   auto issue = [&](int b, bool fwd) {
     const V* src = f + (fwd ? 4 * b : NR - 1 - 4 * b) * rs + (fwd ? 0 : 4);
@@ -213,11 +206,8 @@ __device__ __forceinline__ void solve_line_ring(V* X, int ld, const V* __restric
     for (int r = 0; r < 4; r++) {
       if constexpr (sizeof(V) == 4) {
         if ((r & 1) == part) cp_async16(at(b, r, 0), src);
-      } else if constexpr (RS == 1) {
-        cp_async16(at(b, r, 2 * part), src + 2 * part);
       } else {
-        cp_async8(at(b, r, 2 * part), src + 2 * part);
-        if (!fwd || part == 0) cp_async8(at(b, r, 2 * part + 1), src + 2 * part + 1);
+        cp_async16(at(b, r, 2 * part), src + 2 * part);
       }
       src = fwd ? src + rs : src - rs;
     }
@@ -227,12 +217,9 @@ __device__ __forceinline__ void solve_line_ring(V* X, int ld, const V* __restric
     if constexpr (sizeof(V) == 4) {
       const float4 v = *reinterpret_cast<const float4*>(at(b, r, 0));
       l[0] = v.x; l[1] = v.y; l[2] = v.z; l[3] = v.w;
-    } else if constexpr (RS == 1) {
+    } else {
       const float4 v = *reinterpret_cast<const float4*>(at(b, r, 0)), w = *reinterpret_cast<const float4*>(at(b, r, 2));
       l[0] = V{v.x, v.y}; l[1] = V{v.z, v.w}; l[2] = V{w.x, w.y}; l[3] = V{w.z, w.w};
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; j++) l[j] = *at(b, r, j);
     }
   };
   V xm1{}, xm2{}, xm3{};
@@ -306,8 +293,6 @@ __device__ __forceinline__ void solve_line_ring(V* X, int ld, const V* __restric
 // wall (its first), so that the mixed passes' loops have a fixed length and no bounds.
 __device__ __forceinline__ int stencil_base(int i, int NR) { return min(max(i - IW, 0), NR - STEN); }
 
-// The low half of a line slot holds an FP32 pair in the increment passes.
-__device__ __forceinline__ float2& f32slot(double2* a, int e) { return reinterpret_cast<float2*>(a)[2 * e]; }
 // The mixed passes hold a line slot as two double-float parts (re.hi, re.lo, im.hi,
 // im.lo) -- the predictor from its right-hand side to its correction, the increment
 // passes around their banded solves: the same 16 bytes, so a solve addresses one part
@@ -386,6 +371,14 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
   extern __shared__ double2 sm[];
   double2* R = sm;           // [3][NR][LM] right-hand side, then the new velocity
   double2* P = sm + 3 * LN;  // [NR][LM] divergence, then the pressure
+  // Increment passes: the lines hold FP32 pairs, 8-byte values in the first half of R's space (no
+  // bank conflicts: 16-byte slots with FP32 halves made two wavefronts of every access); the
+  // second half holds the pressure solve's factor ring, then the pressure increment in FP32.
+  // (Corrector pass of 64 members of NR=48 x 32 x 64 modes 698 -> 628 us, of 28 uneven pipes 1649
+  // -> 1511.)
+  float2* R2 = reinterpret_cast<float2*>(sm);  // [3][NR][LM]
+  float2* P2 = R2 + 3 * LN;                    // [NR][LM]
+  float2* T32 = reinterpret_cast<float2*>(P);  // mixed predictor: [3][NR][LM], see below
   // DFS: the solves' factor rings (solve_line_ring), the pressure's after the lines, the
   // Helmholtz solves' from the pressure line on (dead by then)
   dfloat* ringD = reinterpret_cast<dfloat*>(sm + 4 * LN);
@@ -472,9 +465,8 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
     const float2* Un32 = U32n ? U32n + (size_t)mloc * 3 * S : nullptr;  // mixed form: FP32 mirror of u^n
     const float* Luc32 = tb.Luc32 + (size_t)ps * 2 * STEN * NR;
     dfloat hidt_df{0.f, 0.f};
-    // mixed: the block's tile of the FP32 mirror of u^n, [3][NR][LM], in the pressure line
+    // mixed: the block's tile T32 of the FP32 mirror of u^n, [3][NR][LM], in the pressure line
     // and ring space (free until stage C), loaded coalesced; the stencil reads it there.
-    float2* T32 = reinterpret_cast<float2*>(P);
     if constexpr (DFS) {
       const float2 a = split_df(hidt);
       hidt_df = dfloat{a.x, a.y};
@@ -618,7 +610,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       }
     }
   } else if constexpr (INC) {
-    // B'. N_i - N_{i-1} in FP32, into the FP32 halves of the line slots; RHSW32 takes N_i.
+    // B'. N_i - N_{i-1} in FP32, into the FP32 lines; RHSW32 takes N_i.
     // N_i is the transforms' output plus the mean-flow terms (nsp_state.cuh), from u_i's
     // FP32 mirror -- the transforms' input, at this block's own points -- and the mean
     // flow the theta-inverse recorded.  Both are stored as FP32 numbers (the transforms'
@@ -670,7 +662,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
             if (ok) Rw32[c * S + h] = make_float2(nx, ny);
             d = make_float2(nx - q[u][c].x, ny - q[u][c].y);
           }
-          f32slot(R, c * LN + p) = d;  // zero where k >= NTNZ
+          R2[c * LN + p] = d;  // zero where k >= NTNZ
         }
       }
     }
@@ -716,12 +708,12 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
 #pragma unroll
         for (int j = 0; j < STEN; j++) {
           const float de = __ldg(Dr + j);
-          const float2 a = f32slot(R, cb + j * LM);
+          const float2 a = R2[cb + j * LM];
           sx = fmaf(de, a.x, sx);
           sy = fmaf(de, a.y, sy);
         }
         const float kti = skt32[mm] * tb.rinv32[i], kz = skz32[mm];
-        const float2 rt = f32slot(R, LN + p), rz = f32slot(R, 2 * LN + p);
+        const float2 rt = R2[LN + p], rz = R2[2 * LN + p];
         sx -= kti * rt.y; sy += kti * rt.x;
         sx -= kz * rz.y; sy += kz * rz.x;
       }
@@ -800,24 +792,23 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       const dfloat* fp = facdf + (3 * (size_t)NR * NTNZ + k0 + mm) * NPACK;
       const unsigned pair = 3u << ((tid & 31) & ~1);
       if constexpr (INC) {
-        // the increment pass's lines hold FP32 pairs here: a deep ring in their slots'
-        // free upper halves (3 NR LM entries, RING_DEEP x 16 LM needed)
+        // a deep ring in the lines' free half (3 NR LM entries, RING_DEEP x 16 LM needed)
         if (3 * NR >= 16 * RING_DEEP)
-          solve_line_ring<LM, RING_DEEP, 2>(X, 2 * LM, fp, NTNZ, NR, reinterpret_cast<dfloat*>(R) + 1, mm, part, pair);
+          solve_line_ring<LM, RING_DEEP>(X, 2 * LM, fp, NTNZ, NR, reinterpret_cast<dfloat*>(P2), mm, part, pair);
         else
-          solve_line_ring<LM, RING_B, 1>(X, 2 * LM, fp, NTNZ, NR, ringD, mm, part, pair);
+          solve_line_ring<LM, RING_B>(X, 2 * LM, fp, NTNZ, NR, ringD, mm, part, pair);
       } else if constexpr (DFS)
-        solve_line_ring<LM, RING_B, 1>(X, 2 * LM, fp, NTNZ, NR, ringD, mm, part, pair);
+        solve_line_ring<LM, RING_B>(X, 2 * LM, fp, NTNZ, NR, ringD, mm, part, pair);
       else
         solve_line<false>(reinterpret_cast<double*>(P + mm) + part, 2 * LM, fac + 3 * (size_t)NR * NFAC * NTNZ + k0 + mm,
                    NTNZ, NR);
     }
   }
   __syncthreads();
-  if constexpr (INC) {  // the pressure increment to FP32 (hi = fl(hi + lo)), in place
+  if constexpr (INC) {  // the pressure increment to FP32 (hi = fl(hi + lo))
     for (int p = tid; p < LN; p += nth) {
       const float4 a = dfslot(P, p);
-      f32slot(P, p) = make_float2(a.x, a.z);
+      P2[p] = make_float2(a.x, a.z);
     }
     __syncthreads();
   }
@@ -831,24 +822,26 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       if (i < NR - 1) {
         const int cb = stencil_base(i, NR) * LM + mm;
         const float* Dr = tb.D32 + spar[mm] * STEN * NR + STEN * i;
-        float2 rr = f32slot(R, p);
+        float2 rr = R2[p];
 #pragma unroll
         for (int j = 0; j < STEN; j++) {
           const float de = __ldg(Dr + j);
-          const float2 a = f32slot(P, cb + j * LM);
+          const float2 a = P2[cb + j * LM];
           rr.x = fmaf(-de, a.x, rr.x);
           rr.y = fmaf(-de, a.y, rr.y);
         }
         const float kti = skt32[mm] * tb.rinv32[i], kz = skz32[mm];
-        const float2 pp = f32slot(P, p);
-        float2 rt = f32slot(R, LN + p), fz = f32slot(R, 2 * LN + p);
+        const float2 pp = P2[p];
+        float2 rt = R2[LN + p], fz = R2[2 * LN + p];
         rt.x += kti * pp.y; rt.y -= kti * pp.x;
         fz.x += kz * pp.y; fz.y -= kz * pp.x;
-        put_df(R, p, rr.x - rt.y, rr.y + rt.x);
-        put_df(R, LN + p, rr.x + rt.y, rr.y - rt.x);
-        put_df(R, 2 * LN + p, fz.x, fz.y);
-        continue;
+        R2[p] = make_float2(rr.x - rt.y, rr.y + rt.x);
+        R2[LN + p] = make_float2(rr.x + rt.y, rr.y - rt.x);
+        R2[2 * LN + p] = fz;
+      } else {
+        R2[p] = R2[LN + p] = R2[2 * LN + p] = make_float2(0.f, 0.f);
       }
+      continue;
     } else if constexpr (DFS) {  // mixed predictor: the same in double-float
       const dfloat z{0.f, 0.f};
       dfloat upx = z, upy = z, umx = z, umy = z, rzx = z, rzy = z;
@@ -914,14 +907,14 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
     const int tf = tid - F0;
     const int c = tf / (2 * LM), rem = tf - c * 2 * LM, mm = rem >> 1, part = rem & 1;
     if (k0 + mm < NTNZ && fac_ok(c, k0 + mm)) {
-      if constexpr (INC)  // FP32 on the hi parts (lo stays 0): an increment of a well-conditioned operator;
-                          // FP32 factors, so twice the batches in a ring of the same bytes
-        solve_line_ring<LM, 2 * RING_B, 1>(reinterpret_cast<float*>(R + c * LN + mm) + 2 * part, 4 * LM,
+      if constexpr (INC)  // FP32: an increment of a well-conditioned operator; FP32 factors, so
+                          // twice the batches in a ring of the same bytes
+        solve_line_ring<LM, 2 * RING_B>(reinterpret_cast<float*>(R2 + c * LN + mm) + part, 2 * LM,
                             tb.fac32 + (((size_t)ps * 4 + c) * NR * NTNZ + k0 + mm) * NPACK,
                             NTNZ, NR, reinterpret_cast<float*>(ringF) + (size_t)c * 2 * RING_B * 16 * LM, mm, part,
                             3u << ((tid & 31) & ~1));
       else if constexpr (DFS)
-        solve_line_ring<LM, RING_B, 1>(reinterpret_cast<dfloat*>(R + c * LN + mm) + part, 2 * LM,
+        solve_line_ring<LM, RING_B>(reinterpret_cast<dfloat*>(R + c * LN + mm) + part, 2 * LM,
                             facdf + ((size_t)c * NR * NTNZ + k0 + mm) * NPACK, NTNZ, NR,
                             ringF + (size_t)c * RING_B * 16 * LM, mm, part, 3u << ((tid & 31) & ~1));
       else
@@ -944,14 +937,14 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
         float2 urw = make_float2(0.f, 0.f), utw = urw;
         for (int j = 0; j <= IW; j++) {
           const int row = NR - 1 - IW + j;
-          const float4 a = dfslot(R, row * LM + mm), b = dfslot(R, LN + row * LM + mm);
-          const float2 ur = make_float2(0.5f * (a.x + b.x), 0.5f * (a.z + b.z));
+          const float2 a = R2[row * LM + mm], b = R2[LN + row * LM + mm];
+          const float2 ur = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y + b.y));
           const float de = __ldg(Dw + j);
           sx = fmaf(de, ur.x, sx);
           sy = fmaf(de, ur.y, sy);
-          if (j == IW) { urw = ur; utw = make_float2(0.5f * (a.z - b.z), -0.5f * (a.x - b.x)); }
+          if (j == IW) { urw = ur; utw = make_float2(0.5f * (a.y - b.y), -0.5f * (a.x - b.x)); }
         }
-        const float uzx = dfslot(R, 2 * LN + (NR - 1) * LM + mm).x, uzy = dfslot(R, 2 * LN + (NR - 1) * LM + mm).z;
+        const float uzx = R2[2 * LN + (NR - 1) * LM + mm].x, uzy = R2[2 * LN + (NR - 1) * LM + mm].y;
         const float kt = skt32[mm], kz = skz32[mm];
         sx += urw.x; sy += urw.y;
         sx += -kt * utw.y; sy += kt * utw.x;
@@ -1016,7 +1009,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
 
   // G2. u += (-div_wall) V (both at half scale), back to full-scale r/theta, mode (0,0) constraints.
   // Increment passes: in FP32 on the increment (the solves' results, their hi parts), into
-  // the FP32 halves of the slots -- the increment needs FP32's relative precision, the update
+  // the FP32 lines -- the increment needs FP32's relative precision, the update
   // of u in stage I stays FP64.  The mixed predictor: in double-float.
   if constexpr (INC) {
     const float2* Vp32 = tb.V32 + (size_t)ps * 3 * S;
@@ -1025,8 +1018,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       if (k >= NTNZ) continue;
       const size_t hv = (size_t)i * NTNZ + k;
       if (!NSP_IN_BOUNDS(tb, hv, S, BC_LIN_POINT)) continue;
-      const float4 a = dfslot(R, p), b = dfslot(R, LN + p), z = dfslot(R, 2 * LN + p);  // FP32: the hi parts
-      float2 up = make_float2(a.x, a.z), um = make_float2(b.x, b.z), uz = make_float2(z.x, z.z);
+      float2 up = R2[p], um = R2[LN + p], uz = R2[2 * LN + p];
       const float2 dv = dvs32[mm], v0 = Vp32[hv], v1 = Vp32[S + hv], v2 = Vp32[2 * S + hv];
       up.x += dv.x * v0.x - dv.y * v0.y; up.y += dv.x * v0.y + dv.y * v0.x;
       um.x += dv.x * v1.x - dv.y * v1.y; um.y += dv.x * v1.y + dv.y * v1.x;
@@ -1035,7 +1027,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       float2 ut = make_float2(up.y - um.y, -(up.x - um.x));
       uz = make_float2(uz.x + uz.x, uz.y + uz.y);
       if (k == 0) { ur = make_float2(0.f, 0.f); ut.y = 0.f; uz.y = 0.f; }
-      f32slot(R, p) = ur; f32slot(R, LN + p) = ut; f32slot(R, 2 * LN + p) = uz;
+      R2[p] = ur; R2[LN + p] = ut; R2[2 * LN + p] = uz;
     }
   } else if constexpr (DFS) {  // mixed predictor: the same in double-float, with V split likewise
     const float4* Vd = reinterpret_cast<const float4*>(tb.Vdf) + (size_t)ps * 3 * S;
@@ -1094,9 +1086,9 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
   if (k0 == 0 && tid == 0) {
     double Q = 0.0;
     if constexpr (INC) {
-      for (int i = 0; i < NR; i++) Q += tb.rdr[i] * f32_to_f64(f32slot(R, 2 * LN + i * LM).x);
+      for (int i = 0; i < NR; i++) Q += tb.rdr[i] * f32_to_f64(R2[2 * LN + i * LM].x);
       const double corr = -Q / Qc;
-      for (int i = 0; i < NR; i++) f32slot(R, 2 * LN + i * LM).x += f64_to_f32(corr * ucp[i]);
+      for (int i = 0; i < NR; i++) R2[2 * LN + i * LM].x += f64_to_f32(corr * ucp[i]);
     } else if constexpr (DFS) {  // the mixed predictor's double-float line, summed and corrected in FP64
       for (int i = 0; i < NR; i++) Q += tb.rdr[i] * df_value(R, 2 * LN + i * LM).x;
       const double corr = (tb.Qdes - Q) / Qc;
@@ -1146,7 +1138,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
         double2 v;
         if constexpr (INC) {
           // |increment|^2 and |u_i|^2 in FP32 (the measure only decides err > tol)
-          const float2 f = f32slot(R, c * LN + p);
+          const float2 f = R2[c * LN + p];
           const float ox = f64_to_f32(o[u][c].x), oy = f64_to_f32(o[u][c].y);
           lnum32 = max(lnum32, __float_as_uint(fmaf(f.x, f.x, f.y * f.y)));
           lden32 = max(lden32, __float_as_uint(fmaf(ox, ox, oy * oy)));
@@ -1171,7 +1163,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
             f = make_float2(f64_to_f32(v.x), f64_to_f32(v.y));  // integer-pipe rounding
           }
           Ui32[c * S + h] = f;
-          reinterpret_cast<float2*>(R + c * LN + p)[0] = f;  // FP32 copy for the d_r mirror below
+          (INC ? R2 : T32)[c * LN + p] = f;  // FP32 copy for the d_r mirror below
         }
       }
     }
@@ -1192,7 +1184,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
   // J. mixed form: d_r of the new FP32 mirror (the theta-inverse's d_r u fields), with
   // the transform kernels' stencil, so that they read one value instead of 7 levels.
   if (Udr32) {
-    const float2* F = reinterpret_cast<const float2*>(R);  // FP32 value of line entry e at F[2e]
+    const float2* F = INC ? R2 : T32;  // (the predictor's in the tile's space: the pressure line and rings are dead)
     for (int p = tid; p < LN; p += nth) {
       const int i = p / LM, mm = p - i * LM, k = k0 + mm;
       if (k >= NTNZ) continue;
@@ -1207,7 +1199,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
 #pragma unroll
         for (int j = 0; j < STEN; j++) {
           const float de = __ldg(Dr + j);
-          const float2 a = F[2 * (c * LN + cb + j * LM)];
+          const float2 a = F[c * LN + cb + j * LM];
           vx += de * a.x;
           vy += de * a.y;
         }
