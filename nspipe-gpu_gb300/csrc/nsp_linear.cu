@@ -416,7 +416,12 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
   const double* Luc = tb.Luc + (size_t)ps * 2 * STEN * NR;
   const double* ucp = tb.uc + (size_t)ps * NR;
   const double c_ex = tb.sscal[4 * ps], Qc = tb.sscal[4 * ps + 2];
-  const int tid = threadIdx.x, nth = blockDim.x;
+  const int tid = threadIdx.x, nth = DFS && !INC ? NTH : blockDim.x;
+  // Mixed predictor: a thread's points p = tid + q NTH lie in one mode column wherever the block
+  // is whole rows (16 pipes of 48 x 32 x 64: 1.058 -> 1.040 ms; the increment pass has no registers
+  // left for it, 628 -> 651 us).
+  constexpr bool COLUMN = DFS && !INC && NTH % LM == 0;
+  const int mm0 = tid % LM;
   if (tid == 0) bad = 0;
   if (tid < LM) {  // wavenumbers once per block instead of per point
     int k = k0 + tid, it = k / NZ, l = k - it * NZ, m = it < NT / 2 ? it : it - NT;
@@ -477,7 +482,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       __syncthreads();
     }
     for (int p = tid; p < LN; p += nth) {
-      int i = p / LM, mm = p - i * LM, k = k0 + mm;
+      int i = p / LM, mm = COLUMN ? mm0 : p - i * LM, k = k0 + mm;
       if (k >= NTNZ) {
         for (int c = 0; c < 3; c++) R[c * LN + p] = c2(0, 0);
         continue;
@@ -634,7 +639,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       }
 #pragma unroll
       for (int u = 0; u < UB; u++) {
-        const int p = pb + u * nth, i = p / LM, mm = p - i * LM, k = k0 + mm;
+        const int p = pb + u * nth, i = p / LM, mm = COLUMN ? mm0 : p - i * LM, k = k0 + mm;
         if (p >= LN) continue;
         const bool ok = k < NTNZ && (!kBoundsCheck || (size_t)i * NTNZ + k < (size_t)S);
         const size_t h = (size_t)i * NTNZ + k;
@@ -698,7 +703,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
 
   // C. divergence of rhs into P; wall row = 0 (write_bcon).
   for (int p = tid; p < LN; p += nth) {
-    int i = p / LM, mm = p - i * LM, k = k0 + mm;
+    int i = p / LM, mm = COLUMN ? mm0 : p - i * LM, k = k0 + mm;
     double2 d = c2(0, 0);
     if constexpr (INC) {  // FP32 on the increment, into double-float for the solve
       float sx = 0.f, sy = 0.f;
@@ -815,7 +820,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
 
   // E. rhs -= grad p, r/theta -> +/-, wall rows = 0.
   for (int p = tid; p < LN; p += nth) {
-    int i = p / LM, mm = p - i * LM, k = k0 + mm;
+    int i = p / LM, mm = COLUMN ? mm0 : p - i * LM, k = k0 + mm;
     if (k >= NTNZ) continue;
     double2 up = c2(0, 0), um = c2(0, 0), rz = c2(0, 0);
     if constexpr (INC) {  // FP32 on the increment; each thread reads its own slots and the P taps
@@ -1014,7 +1019,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
   if constexpr (INC) {
     const float2* Vp32 = tb.V32 + (size_t)ps * 3 * S;
     for (int p = tid; p < LN; p += nth) {
-      const int i = p / LM, mm = p - i * LM, k = k0 + mm;
+      const int i = p / LM, mm = COLUMN ? mm0 : p - i * LM, k = k0 + mm;
       if (k >= NTNZ) continue;
       const size_t hv = (size_t)i * NTNZ + k;
       if (!NSP_IN_BOUNDS(tb, hv, S, BC_LIN_POINT)) continue;
@@ -1032,7 +1037,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
   } else if constexpr (DFS) {  // mixed predictor: the same in double-float, with V split likewise
     const float4* Vd = reinterpret_cast<const float4*>(tb.Vdf) + (size_t)ps * 3 * S;
     for (int p = tid; p < LN; p += nth) {
-      const int i = p / LM, mm = p - i * LM, k = k0 + mm;
+      const int i = p / LM, mm = COLUMN ? mm0 : p - i * LM, k = k0 + mm;
       if (k >= NTNZ) continue;
       const size_t hv = (size_t)i * NTNZ + k;
       if (!NSP_IN_BOUNDS(tb, hv, S, BC_LIN_POINT)) continue;
@@ -1063,7 +1068,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
       put_df(R, p, urx, ury); put_df(R, LN + p, utx, uty); put_df(R, 2 * LN + p, uzx, uzy);
     }
   } else for (int p = tid; p < LN; p += nth) {
-    int i = p / LM, mm = p - i * LM, k = k0 + mm;
+    int i = p / LM, mm = COLUMN ? mm0 : p - i * LM, k = k0 + mm;
     if (k >= NTNZ) continue;
     double2 up = R[p], um = R[LN + p], uz = R[2 * LN + p];
     double2 dv = dvs[mm];
@@ -1186,7 +1191,7 @@ __global__ void __launch_bounds__(NTH, NTH >= 1024 ? 1 : ((1024 / NTH) < 2 ? 2 :
   if (Udr32) {
     const float2* F = INC ? R2 : T32;  // (the predictor's in the tile's space: the pressure line and rings are dead)
     for (int p = tid; p < LN; p += nth) {
-      const int i = p / LM, mm = p - i * LM, k = k0 + mm;
+      const int i = p / LM, mm = COLUMN ? mm0 : p - i * LM, k = k0 + mm;
       if (k >= NTNZ) continue;
       const int cb = stencil_base(i, NR) * LM + mm;
       const size_t h = (size_t)i * NTNZ + k;
