@@ -818,10 +818,11 @@ int nsp_setup(nsp_ctx* c) {
         return rc;
     }
     std::vector<double2> wt = twiddles(tb.NTP), wz = twiddles(tb.NZR);
-    if ((rc = upload(c, &tb.tw_t, wt)) || (rc = upload(c, &tb.tw_z, wz)) || (rc = upload(c, &tb.tw_t32, to_f32(wt))) ||
-        (rc = upload(c, &tb.tw_z32, to_f32(wz))) || (rc = upload(c, &tb.tw_tx, fx_twiddles(tb.NTP))) ||
-        (rc = upload(c, &tb.tw_zx, fx_twiddles(tb.NZR))))
-      return rc;
+    if ((rc = upload(c, &tb.tw_t32, to_f32(wt))) || (rc = upload(c, &tb.tw_z32, to_f32(wz)))) return rc;
+    std::vector<int4> wx = fx_twiddles(tb.NTP), wzx = fx_twiddles(tb.NZR);
+    wx.insert(wx.end(), wzx.begin(), wzx.end());
+    if ((rc = upload(c, &tb.tw_tx, wx))) return rc;
+    tb.tw_zx = tb.tw_tx + tb.NTP;
     make_plan(tb.NTP, tb.pt);
     make_plan(tb.NZR, tb.pz);
     tb.kts = PI2 / p.LT;

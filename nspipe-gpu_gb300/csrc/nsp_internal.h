@@ -61,10 +61,8 @@ struct Tables {
   const float2* Ddf;    // mixed form: D, Ddiv and 1/r as double-float pairs (the predictor's stencils)
   const float2* Ddivdf;
   const float2* rinvdf;
-  const double2* tw_t; // [NTP] exp(-2 pi i e/NTP), FP64
-  const double2* tw_z; // [NZR]
-  const float2* tw_t32;
-  const float2* tw_z32;
+  const float2* tw_t32;  // [NTP] exp(-2 pi i e/NTP)
+  const float2* tw_z32;  // [NZR]
   const int4* tw_tx;   // the same twiddles as 62-bit fractions (nsp_fx.cuh)
   const int4* tw_zx;
   FftPlan pt, pz;

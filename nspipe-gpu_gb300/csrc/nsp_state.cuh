@@ -19,33 +19,25 @@ __device__ __forceinline__ const double2* member_source(const Tables& tb, const 
   return (which ? bf.U[1] : bf.U[0]) + (size_t)mloc * 3 * tb.S;  // (a select keeps bf out of local memory)
 }
 
-// Scalars and 1/r of the tables in the working precision (FP32 copies for T = float).
-template <typename T> __device__ __forceinline__ T tb_kts(const Tables& tb) {
-  if constexpr (sizeof(T) == 4) return tb.kts32; else return tb.kts;
-}
-template <typename T> __device__ __forceinline__ T tb_kzs(const Tables& tb) {
-  if constexpr (sizeof(T) == 4) return tb.kzs32; else return tb.kzs;
-}
-template <typename T> __device__ __forceinline__ T tb_inv_norm(const Tables& tb) {
-  if constexpr (sizeof(T) == 4) return tb.inv_norm32; else return tb.inv_norm;
-}
-template <typename T> __device__ __forceinline__ T tb_rinv(const Tables& tb, int i) {
-  if constexpr (sizeof(T) == 4) return tb.rinv32[i]; else return tb.rinv[i];
-}
+// Scalars, 1/r and the derivative rows of the tables in the working precision (the FP32 copies:
+// the FP64 form's transforms read the FP64 ones themselves, nsp_transform_fx.cu).
+template <typename T> __device__ __forceinline__ T tb_kts(const Tables& tb);
+template <> __device__ __forceinline__ float tb_kts<float>(const Tables& tb) { return tb.kts32; }
+template <typename T> __device__ __forceinline__ T tb_kzs(const Tables& tb);
+template <> __device__ __forceinline__ float tb_kzs<float>(const Tables& tb) { return tb.kzs32; }
+template <typename T> __device__ __forceinline__ T tb_inv_norm(const Tables& tb);
+template <> __device__ __forceinline__ float tb_inv_norm<float>(const Tables& tb) { return tb.inv_norm32; }
+template <typename T> __device__ __forceinline__ T tb_rinv(const Tables& tb, int i);
+template <> __device__ __forceinline__ float tb_rinv<float>(const Tables& tb, int i) { return tb.rinv32[i]; }
+template <typename T> __device__ __forceinline__ const T* dtab(const Tables& tb);
+template <> __device__ __forceinline__ const float* dtab<float>(const Tables& tb) { return tb.D32; }
 
-// Transform input in the working precision: the FP64 state, or its FP32 mirror.
+// Transform input in the working precision: the state's FP32 mirror.
 template <typename T> struct StateIn;
-template <> struct StateIn<double> {
-  const double2* p;
-  __device__ __forceinline__ cpx<double> ld(size_t h) const { double2 a = p[h]; return mk<double>(a.x, a.y); }
-};
 template <> struct StateIn<float> {
   const float2* p;
   __device__ __forceinline__ cpx<float> ld(size_t h) const { float2 a = __ldg(p + h); return mk<float>(a.x, a.y); }
 };
-template <typename T> __device__ __forceinline__ const T* dtab(const Tables& tb);
-template <> __device__ __forceinline__ const double* dtab<double>(const Tables& tb) { return tb.D; }
-template <> __device__ __forceinline__ const float* dtab<float>(const Tables& tb) { return tb.D32; }
 
 template <typename T>
 __device__ __forceinline__ StateIn<T> member_input(const Tables& tb, const Bufs& bf, const Ctl* ctl, int mloc,
@@ -56,8 +48,7 @@ __device__ __forceinline__ StateIn<T> member_input(const Tables& tb, const Bufs&
     int ph = ctl->phase[tb.mem0 + mloc];
     which = (ph == 0) ? ctl->parity : (ctl->parity ^ 1);
   }
-  if constexpr (sizeof(T) == 8) s.p = src ? src : (which ? bf.U[1] : bf.U[0]) + (size_t)mloc * 3 * tb.S;
-  else s.p = src ? src32 : (which ? bf.U32[1] : bf.U32[0]) + (size_t)mloc * 3 * tb.S;
+  s.p = src ? src32 : (which ? bf.U32[1] : bf.U32[0]) + (size_t)mloc * 3 * tb.S;
   return s;
 }
 

@@ -546,17 +546,20 @@ std::vector<int4> fx_twiddles(int n) {
     h = (int)(x >> 32) - (l >> 31);
   };
   std::vector<int4> w(n);
+  struct Angle {  // cosine and sine of (pi/2) rest / n, each rest evaluated once (128-bit long doubles are slow)
+    bool set = false;
+    long double c, s;
+  };
+  std::vector<Angle> first(n / 2 + 1);
   for (int e = 0; e < n; e++) {
-    const int q = (int)(4LL * e / n);                          // quarter turn
-    const long long rest = 4LL * e - (long long)q * n;         // angle within it: (pi/2) rest / n
-    long double c, s;                                          // of that angle
-    if (2 * rest <= n) {
-      c = cosl(PI_L * 0.5L * (long double)rest / (long double)n);
-      s = sinl(PI_L * 0.5L * (long double)rest / (long double)n);
-    } else {
-      s = cosl(PI_L * 0.5L * (long double)(n - rest) / (long double)n);
-      c = sinl(PI_L * 0.5L * (long double)(n - rest) / (long double)n);
+    const int q = (int)(4LL * e / n);                      // quarter turn
+    const int rest = (int)(4LL * e - (long long)q * n);    // angle within it: (pi/2) rest / n
+    Angle& a = first[2 * rest <= n ? rest : n - rest];
+    if (!a.set) {
+      const long double x = PI_L * 0.5L * (long double)(2 * rest <= n ? rest : n - rest) / (long double)n;
+      a = Angle{true, cosl(x), sinl(x)};
     }
+    const long double c = 2 * rest <= n ? a.c : a.s, s = 2 * rest <= n ? a.s : a.c;
     const long double re[4] = {c, -s, -c, s}, im[4] = {-s, -c, s, c};
     int4& o = w[e];
     halves(re[q], o.x, o.y);
