@@ -1280,51 +1280,75 @@ __global__ void finish_step_k(Ctl* ctl) {
 // Divergence diagnostic of one member's state (div_k / divWall_k, mod_radialFD.cu:34-96):
 // |d_r u_r + u_r/r + i m u_theta / r + i k_z u_z| per point, maximum over the interior
 // rows into out[0] and over the wall row into out[1] (ordered bits, atomicMax).
-__global__ void diag_div_k(Tables tb, const double2* __restrict__ U, unsigned long long* out) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// Bound by the FP64 pipe (some 23 operations per point).  A thread takes DIV_ROWS rows of a
+// mode with the 7 rows of its stencil in registers: whole columns per thread, every tap loaded
+// again and the maxima compared in FP64 left the pipe waiting (64 pipes of 48 x 32 x 64: 370 us,
+// now 300; 6 to 24 rows a thread are within 4% of one another).
+constexpr int DIV_ROWS = 12, DIV_TH = 128;
+__global__ void __launch_bounds__(DIV_TH) diag_div_k(Tables tb, const double2* __restrict__ U, unsigned long long* out) {
+  __shared__ unsigned long long top[2][DIV_TH / 32];
+  const int k = blockIdx.x * DIV_TH + threadIdx.x;
   const int NR = tb.NR, NT = tb.NT, NZ = tb.NZ, NTNZ = tb.NTNZ;
+  const int row0 = blockIdx.y * DIV_ROWS, row1 = min(row0 + DIV_ROWS, NR);
   const long long S = tb.S;
   U += (size_t)blockIdx.z * 3 * S;  // member blockIdx.z of a batched launch
   out += 2 * blockIdx.z;
-  double mi = 0.0, mw = 0.0;
+  unsigned long long mi = 0, mw = 0;  // bits of the largest squares: they order like the values
   if (k < NTNZ) {
     const int it = k / NZ, l = k - it * NZ, m = it < NT / 2 ? it : it - NT;
     const double kt = tb.kts * (double)m, kz = tb.kzs * (double)l;
     const int tab = abs((abs(m) % 2) - 1);
-    for (int i = 0; i < NR; i++) {
-      const int left = max(0, i - IW), right = min(i + IW, NR - 1), len = right + 1 - left, i0 = i + IW - right;
-      const double* Dr = tb.D + tab * STEN * NR + STEN * i + i0;
+    int base = stencil_base(row0, NR);
+    double2 w[STEN];  // u_r of rows base ..
+#pragma unroll
+    for (int j = 0; j < STEN; j++) w[j] = U[(size_t)(base + j) * NTNZ + k];
+    for (int i = row0; i < row1; i++) {
+      if (stencil_base(i, NR) > base) {
+        base++;
+#pragma unroll
+        for (int j = 0; j < STEN - 1; j++) w[j] = w[j + 1];
+        w[STEN - 1] = U[(size_t)(base + STEN - 1) * NTNZ + k];
+      }
+      const int j0 = max(0, i - IW) - base, j1 = min(i + IW, NR - 1) - base;  // cut short at axis and wall
+      const double* Dr = tb.D + tab * STEN * NR + STEN * i;
       double sx = 0.0, sy = 0.0;
-      for (int j = 0; j < len; j++) {
-        const double2 a = U[(size_t)(left + j) * NTNZ + k];
-        sx += Dr[j] * a.x;
-        sy += Dr[j] * a.y;
+#pragma unroll
+      for (int j = 0; j < STEN; j++) {
+        if (j < j0 || j > j1) continue;
+        sx += Dr[j] * w[j].x;
+        sy += Dr[j] * w[j].y;
       }
       const size_t h = (size_t)i * NTNZ + k;
       const double ri = tb.rinv[i], kti = kt * ri;
       const double2 ur = U[h], ut = U[S + h], uz = U[2 * S + h];
       sx += ur.x * ri - kti * ut.y - kz * uz.y;
       sy += ur.y * ri + kti * ut.x + kz * uz.x;
-      // the square root is monotone and correctly rounded: taken once, of the maximum
-      const double a = sx * sx + sy * sy;
-      if (i < NR - 1) mi = fmax(mi, a);
-      else mw = fmax(mw, a);
+      const unsigned long long a = (unsigned long long)__double_as_longlong(sx * sx + sy * sy);
+      if (a > 0x7FF0000000000000ull) continue;  // NaN
+      if (i < NR - 1) mi = max(mi, a);
+      else mw = max(mw, a);
     }
-    mi = sqrt(mi);
-    mw = sqrt(mw);
   }
   for (int o = 16; o > 0; o >>= 1) {
-    mi = fmax(mi, __shfl_xor_sync(0xffffffffu, mi, o));
-    mw = fmax(mw, __shfl_xor_sync(0xffffffffu, mw, o));
+    mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, o));
+    mw = max(mw, __shfl_xor_sync(0xffffffffu, mw, o));
   }
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(out, (unsigned long long)__double_as_longlong(mi));
-    atomicMax(out + 1, (unsigned long long)__double_as_longlong(mw));
+    top[0][threadIdx.x >> 5] = mi;
+    top[1][threadIdx.x >> 5] = mw;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    unsigned long long a = 0;
+    for (int v = 0; v < DIV_TH / 32; v++) a = max(a, top[threadIdx.x][v]);
+    // the square root is monotone and correctly rounded: taken once, of the maximum
+    if (a) atomicMax(out + threadIdx.x, (unsigned long long)__double_as_longlong(sqrt(__longlong_as_double((long long)a))));
   }
 }
 
 void launch_diag_div(const Tables& tb, const double2* U, unsigned long long* out, cudaStream_t st, int nmem) {
-  diag_div_k<<<dim3((tb.NTNZ + 127) / 128, 1, nmem), 128, 0, st>>>(tb, U, out);
+  const dim3 grid((tb.NTNZ + DIV_TH - 1) / DIV_TH, (tb.NR + DIV_ROWS - 1) / DIV_ROWS, nmem);
+  diag_div_k<<<grid, DIV_TH, 0, st>>>(tb, U, out);
 }
 
 // Re u_z(m=0, k_z=0)(r_i) of nmem consecutive members -> out[member][NR].
