@@ -109,7 +109,9 @@ int nsp_save_state(nsp_ctx* ctx, int member, const char* file_r, const char* fil
  * member = NSP_ALL_MEMBERS: each pointer then holds that component of every member,
  * back to back in member order (one synchronisation for the whole ensemble). */
 #define NSP_ALL_MEMBERS (-1)
-/* Setting a member's state clears its status (NSP_ERR_NONFINITE of an earlier state). */
+/* Setting a member's state clears its status (NSP_ERR_NONFINITE of an earlier state).
+ * The arrays of a set may be the same or overlap.  Where those of nsp_get_state_device do, the
+ * components are written in the order u_r, u_theta, u_z. */
 int nsp_set_state_host(nsp_ctx* ctx, int member, const double* ur, const double* ut, const double* uz);
 int nsp_get_state_host(nsp_ctx* ctx, int member, double* ur, double* ut, double* uz);
 int nsp_set_state_device(nsp_ctx* ctx, int member, const void* ur, const void* ut, const void* uz);

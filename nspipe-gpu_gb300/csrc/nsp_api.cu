@@ -998,8 +998,15 @@ static bool plain_device_array(const nsp_ctx* c, const void* p, size_t bytes) {
   return range(&base, &size, q) == CUDA_SUCCESS && q >= base && q - base <= size && bytes <= size - (q - base);
 }
 
+// Whether two arrays of `bytes` bytes share any of them.
+static bool overlap(const void* a, const void* b, size_t bytes) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return (x < y ? y - x : x - y) < bytes;
+}
+
 // One member's components between the caller's device arrays `user` and the state buffers: one
-// launch for the three.
+// launch for the three.  Destinations that overlap (one scratch array for the components a
+// caller does not want) take the copies, in the order u_r, u_theta, u_z: the last one stands.
 static int hand_over(nsp_ctx* c, int m, const void* const (&user)[3], bool to_state) {
   const long long n = c->groups[c->grp[m]].tb.S;
   const size_t bytes = sizeof(double2) * (size_t)n;
@@ -1010,6 +1017,9 @@ static int hand_over(nsp_ctx* c, int m, const void* const (&user)[3], bool to_st
     state[k] = state_ptr(c, m, k);
     plain = plain && plain_device_array(c, user[k], bytes);
   }
+  if (!to_state)
+    plain = plain && !overlap(user[0], user[1], bytes) && !overlap(user[0], user[2], bytes) &&
+            !overlap(user[1], user[2], bytes);
   if (plain) {
     const double2* src[3];
     double2* dst[3];

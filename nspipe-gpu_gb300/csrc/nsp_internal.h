@@ -159,7 +159,7 @@ void launch_converge(Ctl* dctl, int nmem, unsigned long long cond_handle, int us
 // completion work, held back while the chunks ran).
 void launch_finish_step(Ctl* dctl, cudaStream_t st);
 // Copies three components of n complex values each in one launch (16-byte aligned device
-// arrays); status: a member's status word to clear, or null.
+// arrays, the destinations apart from one another); status: a member's status word to clear, or null.
 void launch_copy3(const double2* const (&src)[3], double2* const (&dst)[3], long long n, int* status, cudaStream_t st);
 void launch_lusolve(const Tables& tb, int kind, const double2* rhs, double2* sol, cudaStream_t st);
 void launch_fp64_peak(double* out, int blocks, int threads, int iters, cudaStream_t st);

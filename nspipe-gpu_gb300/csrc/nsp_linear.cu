@@ -1492,7 +1492,7 @@ void launch_converge(Ctl* dctl, int nmem, unsigned long long cond_handle, int us
 
 // State hand-over of one member between device arrays: one launch instead of three copies (and
 // a clear), each of which costs a launch and a gap of ~2 us -- the size of the copies themselves
-// at NR=48 x 32 x 64 modes.  Four values in flight per thread.
+// at NR=48 x 32 x 64 modes.  Four values in flight per thread.  The destinations are apart.
 struct Copy3 {
   const double2* src[3];
   double2* dst[3];
