@@ -21,7 +21,10 @@
 //             1.2e-16 .. 3.3e-16 for decaying and 1.5e-16 .. 4.0e-16 for white spectra of
 //             32 x 65 to 128 x 257 modes, 2.7e-16 .. 6.4e-16 and 1.3e-15 .. 3.6e-15 with the
 //             FP64 transforms it replaced;
-//   Inf, NaN  a line that holds one gives NaN (its E is FX_BAD), as its FP64 transform would.
+//   range     FP64's: the unit goes down to 2^-1075 and results to subnormal numbers (the field of
+//             0 at both conversions costs 0.3 .. 0.8% of a step of this form);
+//   Inf, NaN  a line that holds one, or whose bound passes 2^1023, gives NaN (its E is FX_BAD), as
+//             its FP64 transform would with Inf.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -41,11 +44,12 @@ __device__ __forceinline__ unsigned fx_mag(unsigned k, unsigned emax) {
 }
 
 // The line's exponent E from its largest exponent field and its sum of magnitudes (fx_mag
-// units): the sum is below 2^E.  Clamped so that zero and subnormal lines convert to 0 and
-// fx_to needs no range checks; a line that sums to 2^1000 or more counts as infinite.
+// units): the sum is below 2^E.  Clamped at a unit of 2^-1075, below the smallest FP64 number's,
+// so that a line follows its values down to subnormal ones; a line whose bound exceeds 2^1023
+// (results up to 2^1024) counts as infinite.
 __device__ __forceinline__ int fx_exponent(int emax, unsigned sum) {
-  const int E = max(emax - 1043 + (32 - __clz((int)sum)), -900);
-  return emax >= 0x7FF || E > 1000 ? FX_BAD : E;
+  const int E = max(emax - 1043 + (32 - __clz((int)sum)), -1014);
+  return emax >= 0x7FF || E > 1023 ? FX_BAD : E;
 }
 
 // Largest exponent field and sum of magnitudes of a line in one pass: the sum is kept in units
@@ -71,10 +75,11 @@ struct FxSum {
 // roundings of a floating-point sum do.)
 __device__ __forceinline__ fx fx_from(double x, int E) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const unsigned mh = (hi & 0xFFFFFu) | 0x100000u;
+  const unsigned e = (hi >> 20) & 0x7FFu, nz = min(e, 1u);  // (zero and subnormal: 0.m at exponent 1)
+  const unsigned mh = (hi & 0xFFFFFu) + (nz << 20);
   // 1.m left-aligned below the sign bit, then shifted right by r >= 2
   const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, 10) << 32) | (lo << 10);
-  const int r = E + 1085 - FX_BITS - (int)((hi >> 20) & 0x7FFu);
+  const int r = E + 1084 - FX_BITS - (int)e + (int)nz;
   const fx v = (fx)(((m >> min(r - 1, 63)) + 1) >> 1);
   const fx s = (fx)((int)hi >> 31);
   return (v ^ s) - s;
@@ -82,21 +87,23 @@ __device__ __forceinline__ fx fx_from(double x, int E) {
 // The same for x q, q < 2^9 a whole number: the product is formed exactly.
 __device__ __forceinline__ fx fx_from_times(double x, unsigned q, int E) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const unsigned mh = (hi & 0xFFFFFu) | 0x100000u;
+  const unsigned e = (hi >> 20) & 0x7FFu, nz = min(e, 1u);
+  const unsigned mh = (hi & 0xFFFFFu) + (nz << 20);
   const int z = __clz((int)q) - 22;  // q 2^z in [2^9, 2^10): the product in [2^61, 2^63)
   const unsigned qz = q << z;
   const unsigned long long m = (unsigned long long)lo * qz + ((unsigned long long)(mh * qz) << 32);
-  const int r = E + 1075 - FX_BITS - (int)((hi >> 20) & 0x7FFu) + z;
+  const int r = E + 1074 - FX_BITS - (int)e + (int)nz + z;
   const fx v = q ? (fx)(((m >> min(r - 1, 63)) + 1) >> 1) : 0;
   const fx s = (fx)((int)hi >> 31);
   return (v ^ s) - s;
 }
 
-// v 2^e rounded to nearest, |v| < 2^62, e = E - FX_BITS of a line (so the result is normal).
+// v 2^e rounded to nearest, |v| < 2^62, e = E - FX_BITS of a line (or one less: a halved result).
+// The leading bit goes to 62, or to where a result below 2^-1022 has it with an exponent field of 0.
 __device__ __forceinline__ double fx_to(fx v, int e) {
   const int s = (int)(v >> 63);
   const unsigned long long a = (unsigned long long)((v ^ (fx)s) - (fx)s);
-  const int z = __clzll((long long)a) - 1;  // leading bit to 62: rounding carries into 63 at most
+  const int z = min(__clzll((long long)a) - 1, e + 1084);  // (rounding carries into 63 at most)
   const unsigned long long q = ((a << (z & 63)) + 0x200u) >> 10;
   const unsigned hi = (unsigned)(q >> 32) + ((unsigned)(1084 + e - z) << 20);
   return __hiloint2double((int)(a ? hi | ((unsigned)s & 0x80000000u) : 0u), (int)q);

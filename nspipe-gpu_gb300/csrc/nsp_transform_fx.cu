@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
           const double2 v = load(h, q);
           const unsigned w = q > 1 ? (unsigned)(32 - __clz(q - 1)) << 20 : 0u;
           const unsigned kx = fx_key(v.x), ky = fx_key(v.y);
-          sum.add(kx < 0x100000u ? 0u : min(kx + w, 0x7FF00000u), ky < 0x100000u ? 0u : min(ky + w, 0x7FF00000u));
+          sum.add(min(max(kx, 0x100000u) + w, 0x7FF00000u), min(max(ky, 0x100000u) + w, 0x7FF00000u));
         }
       } else {
 #pragma unroll 1
