@@ -25,6 +25,7 @@ template <int NZRC, int RPB>
 __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tables tb, const double2* __restrict__ U,
                                                                             double* __restrict__ part) {
   constexpr int NTH = z_threads(NZRC), NB = RPB * 6, KZ = NZRC > 0 ? (NZRC + NTH - 1) / NTH : 4;
+  static_assert(NZRC > 0 || 6 * (KZ * NTH / 4) >= RT_TASKS, "points of a run-time length (radices up to 4)");
   const int i = blockIdx.x, c = blockIdx.y, lane = threadIdx.x & 31;
   extern __shared__ __align__(16) unsigned char smraw[];
   cpx<fx>* Z = reinterpret_cast<cpx<fx>*>(smraw);  // [NB] lines of ZP
@@ -138,11 +139,11 @@ void launch_diag_cross(const Tables& tb, const double2* U, double* part, double*
     const int nm = std::min(nmem - m0, 65535);
     const double2* Um = U + (size_t)m0 * 3 * tb.S;
     switch (tb.NZR) {
-#define NSP_CASE_C(n, r) \
-  case n: launch_cross_t<n, r>(tb, Um, part, st, nm); break;
+#define NSP_CASE_C(n) \
+  case n: launch_cross_t<n, z_rows(n)>(tb, Um, part, st, nm); break;
       NSP_NZR_LIST(NSP_CASE_C)
 #undef NSP_CASE_C
-      default: launch_cross_t<0, 1>(tb, Um, part, st, nm);
+      default: launch_cross_t<0, z_rows(0)>(tb, Um, part, st, nm);
     }
     cross_sum_k<<<dim3((tb.NZR + 127) / 128, nm), 128, 0, st>>>(tb, part, out);
     part += (size_t)nm * 3 * tb.NR * tb.NZR;
@@ -151,9 +152,9 @@ void launch_diag_cross(const Tables& tb, const double2* U, double* part, double*
 }
 
 void configure_cross_kernels() {
-#define NSP_CFG_C(n, r) cudaFuncSetAttribute(fx_cross<n, r>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+#define NSP_CFG_C(n) cudaFuncSetAttribute(fx_cross<n, z_rows(n)>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   NSP_NZR_LIST(NSP_CFG_C)
-  NSP_CFG_C(0, 1)
+  NSP_CFG_C(0)
 #undef NSP_CFG_C
 }
 

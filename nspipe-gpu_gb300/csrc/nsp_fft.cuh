@@ -258,6 +258,35 @@ __host__ __device__ constexpr int pass_radix(int n, int s, bool cols) {
   return 0;
 }
 
+// The compiled lengths, of both forms' kernels and of the cross sections: theta and z.  Any other
+// 2^a 3^b length takes the run-time plan (fft_batch), whose kernels all hold at least RT_TASKS
+// butterflies of 16 theta columns or of 6 z lines in registers (transform_supported refuses more).
+#define NSP_NTP_LIST(X) X(12) X(18) X(24) X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(192)
+#define NSP_NZR_LIST(X) X(24) X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(162) X(192) X(216) X(288) X(384) X(432) \
+  X(576) X(768)
+constexpr int RT_TASKS = 1024;
+constexpr bool ntp_compiled(int n) {
+#define NSP_IS(m) if (n == m) return true;
+  NSP_NTP_LIST(NSP_IS)
+  return false;
+}
+constexpr bool nzr_compiled(int n) {
+  NSP_NZR_LIST(NSP_IS)
+#undef NSP_IS
+  return false;
+}
+constexpr int pass_length(int n, bool cols) {
+  int m = 1;
+  for (int s = 0; s < 3 && pass_radix(n, s, cols) > 0; s++) m *= pass_radix(n, s, cols);
+  return m;
+}
+#define NSP_HAS_PLAN_T(n) static_assert(pass_length(n, true) == n, "radices of a compiled theta length");
+#define NSP_HAS_PLAN_Z(n) static_assert(pass_length(n, false) == n, "radices of a compiled z length");
+NSP_NTP_LIST(NSP_HAS_PLAN_T)
+NSP_NZR_LIST(NSP_HAS_PLAN_Z)
+#undef NSP_HAS_PLAN_T
+#undef NSP_HAS_PLAN_Z
+
 // Place of element e in a line of contiguous elements between passes: one gap per 16 so that
 // the strided stores of a first pass spread over the banks.  A transform's input and output
 // are without gaps.

@@ -221,9 +221,9 @@ constexpr int z_blocks(int n) {
 
 // Values per line in shared memory: the gaps between passes, at least two behind the line.
 constexpr int line_pitch(int n) { return line_pad(n - 1) + 1 > n + 2 ? line_pad(n - 1) + 1 : n + 2; }
-// Compiled z lengths and theta rows per block: two (three packed forward transforms for both)
-// while the six lines of each leave three blocks on an SM.
-#define NSP_NZR_LIST(X) X(24, 2) X(36, 2) X(48, 2) X(54, 2) X(72, 2) X(96, 2) X(108, 2) X(144, 2) X(162, 2) \
-  X(192, 2) X(216, 2) X(288, 2) X(384, 1) X(432, 1) X(576, 1) X(768, 1)
+// Theta rows per block: two (three packed forward transforms for both) while the six lines of
+// each leave three blocks on an SM.
+constexpr int z_rows(int n) { return n == 0 || n >= 384 ? 1 : 2; }
+static_assert(MAXRZ * z_threads(0) >= RT_TASKS, "register rounds of the run-time FFT");
 
 }  // namespace nsp

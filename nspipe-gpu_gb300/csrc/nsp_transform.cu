@@ -42,6 +42,7 @@ constexpr int MAXR = 4;   // register rounds of the run-time FFT
 constexpr int theta_cols(int ntp) { return ntp == 0 || ntp > 108 ? 16 : 32; }
 constexpr int TTH = 256;  // threads of the theta kernels
 constexpr int ZTH = 256;  // threads of the run-time z kernel
+static_assert(MAXR * TTH >= RT_TASKS && MAXR * ZTH >= RT_TASKS, "register rounds of the run-time FFT");
 constexpr int Z2TH = 192; // threads of the two-pass z kernel (its passes run 192, 144, 384, 48, 36, 384 tasks)
 
 template <typename T> __device__ __forceinline__ const typename vec2<T>::type* tw_t(const Tables& tb);
@@ -573,9 +574,8 @@ static void launch_z2(const Tables& tb, const Bufs& bf, Ctl* dctl, bool standalo
   nl_z2<T, NZRC, N1, N2, R><<<g, Z2TH, z2_smem<T, NZRC, N1, N2, R>(), st>>>(tb, bf, dctl, standalone ? 1 : 0);
 }
 
-#define NSP_NTP_LIST(X) X(12) X(18) X(24) X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(192)
-#define NSP_NZR_LIST(X) X(24, 2) X(36, 2) X(48, 2) X(54, 2) X(72, 2) X(96, 2) X(108, 2) X(144, 2) X(162, 2) \
-  X(192, 2) X(216, 2) X(288, 2) X(384, 1) X(432, 2) X(576, 1) X(768, 1)
+// Theta rows per block of the in-place z kernel.
+constexpr int zp_rows(int n) { return n == 0 || n == 384 || n >= 576 ? 1 : 2; }
 // Two-pass z stage: (NZR, N1, N2, rows per block); the setup-time autotuner picks among
 // the splits and the in-place passes per shape (which win at 432 and 768 points, so those have no
 // split).  Every other 2^a 3^b length up to 576 that a register pass of at most 24 points splits
@@ -646,11 +646,11 @@ static void launch_nl_t(const Tables& tb, const Bufs& bf, Ctl* dctl, const doubl
     }
     if (!done) {
       switch (tb.NZR) {
-#define NSP_CASE_Z(n, r) \
-  case n: launch_z<T, n, r>(tb, bf, dctl, src != nullptr, st, nm); break;
+#define NSP_CASE_Z(n) \
+  case n: launch_z<T, n, zp_rows(n)>(tb, bf, dctl, src != nullptr, st, nm); break;
         NSP_NZR_LIST(NSP_CASE_Z)
 #undef NSP_CASE_Z
-        default: launch_z<T, 0, 1>(tb, bf, dctl, src != nullptr, st, nm);
+        default: launch_z<T, 0, zp_rows(0)>(tb, bf, dctl, src != nullptr, st, nm);
       }
     }
   }
@@ -678,9 +678,9 @@ static void configure_t() {
   NSP_NTP_LIST(NSP_CFG_T)
   NSP_CFG_T(0)
 #undef NSP_CFG_T
-#define NSP_CFG_Z(n, r) cudaFuncSetAttribute(nl_z<T, n, r>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+#define NSP_CFG_Z(n) cudaFuncSetAttribute(nl_z<T, n, zp_rows(n)>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   NSP_NZR_LIST(NSP_CFG_Z)
-  NSP_CFG_Z(0, 1)
+  NSP_CFG_Z(0)
 #undef NSP_CFG_Z
 }
 
@@ -701,17 +701,10 @@ void configure_transform_kernels() {
 }
 
 bool transform_supported(int NTP, int NZR) {
-  bool ct_t = false, ct_z = false;
-#define NSP_HAS_T(n) ct_t |= (NTP == n);
-#define NSP_HAS_Z(n, r) ct_z |= (NZR == n);
-  NSP_NTP_LIST(NSP_HAS_T)
-  NSP_NZR_LIST(NSP_HAS_Z)
-#undef NSP_HAS_T
-#undef NSP_HAS_Z
   FftPlan pt, pz;
   make_plan(NTP, pt);
   make_plan(NZR, pz);
-  return (ct_t || max_butterflies(pt, 16) <= MAXR * TTH) && (ct_z || max_butterflies(pz, 6) <= MAXR * ZTH);
+  return (ntp_compiled(NTP) || max_butterflies(pt, 16) <= RT_TASKS) && (nzr_compiled(NZR) || max_butterflies(pz, 6) <= RT_TASKS);
 }
 
 void launch_nonlinear(const Tables& tb, const Bufs& bf, Ctl* dctl, bool mixed, const double2* src, double2* dst,

@@ -36,6 +36,7 @@ namespace {
 
 constexpr int MAXR = 4;   // register rounds of the run-time FFT along theta
 constexpr int TTH = 256;  // threads of the theta kernels
+static_assert(MAXR * TTH >= RT_TASKS, "register rounds of the run-time FFT");
 
 // Columns per block of the theta kernels: 32 (512-byte rows of G) while that leaves several
 // blocks' columns in shared memory, so that a pass has about as many butterflies as threads.
@@ -474,9 +475,6 @@ __global__ void __launch_bounds__(TTH) fx_theta_fwd(Tables tb, Bufs bf, const Ct
 }
 
 // ---------------------------------------------------------------- launcher
-#define NSP_NTP_LIST(X) X(12) X(18) X(24) X(36) X(48) X(54) X(72) X(96) X(108) X(144) X(192)
-
-
 template <int NTPC>
 static void launch_theta_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, const double2* src, double2* dst,
                             cudaStream_t st, int mask, int nm) {
@@ -509,11 +507,11 @@ void launch_nonlinear_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, const doub
   if (mask & 1) theta(1);
   if (mask & 2) {
     switch (tb.NZR) {
-#define NSP_CASE_Z(n, r) \
-  case n: launch_z_fx<n, r>(tb, bf, dctl, src != nullptr, st, nm); break;
+#define NSP_CASE_Z(n) \
+  case n: launch_z_fx<n, z_rows(n)>(tb, bf, dctl, src != nullptr, st, nm); break;
       NSP_NZR_LIST(NSP_CASE_Z)
 #undef NSP_CASE_Z
-      default: launch_z_fx<0, 1>(tb, bf, dctl, src != nullptr, st, nm);
+      default: launch_z_fx<0, z_rows(0)>(tb, bf, dctl, src != nullptr, st, nm);
     }
   }
   if (mask & 4) theta(4);
@@ -527,9 +525,9 @@ void configure_transform_fx_kernels() {
   NSP_NTP_LIST(NSP_CFG_T)
   NSP_CFG_T(0)
 #undef NSP_CFG_T
-#define NSP_CFG_Z(n, r) cudaFuncSetAttribute(fx_z<n, r>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+#define NSP_CFG_Z(n) cudaFuncSetAttribute(fx_z<n, z_rows(n)>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   NSP_NZR_LIST(NSP_CFG_Z)
-  NSP_CFG_Z(0, 1)
+  NSP_CFG_Z(0)
 #undef NSP_CFG_Z
 }
 
