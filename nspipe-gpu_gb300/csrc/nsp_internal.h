@@ -68,8 +68,8 @@ struct Tables {
   FftPlan pt, pz;
   int lin_variant;     // block shape of the linear pass (autotuned at setup)
   int lin_variant_inc; // mixed form: block shape of the increment (corrector) pass
-  int z_variant;       // z-stage kernel (autotuned at setup): 0 radix-stage, k >= 1 the k-th
-                       // two-pass N1 x N2 split compiled for the length and precision
+  int z_variant;       // z-stage kernel (autotuned at setup): 0 in place, k >= 1 the k-th
+                       // two-pass N1 x N2 split compiled for the length (mixed form)
   int nsets;           // operator parameter sets (distinct Re) of the group
   const int* mset;     // [nmem] parameter set of each member
   const double* sscal; // [nsets][4]: (1-d_im)/Re, 2/Re, Qc, Re

@@ -596,7 +596,7 @@ int z_variants(int NZR, int NTP, bool fp32) {
 }
 
 // The two-pass kernel where one is compiled for the length (the FP32 default, measured
-// faster than the radix-stage kernel on the bench shape), else the radix-stage kernel.
+// faster than the in-place kernel on the bench shape), else the in-place one.
 int z_default_variant(int NZR, int NTP, bool fp32) {
   const char* e = getenv("NSP_Z2");
   if (e && e[0] == '0') return 0;
@@ -604,10 +604,11 @@ int z_default_variant(int NZR, int NTP, bool fp32) {
 }
 
 std::string z_variant_name(int NZR, int NTP, bool fp32, int v) {
-  if (!fp32) return "radix, 64-bit fixed point";
-  if (v <= 0) return "in-place passes";
+  // variant 0: the compiled passes in place, or the run-time plan's radix stages
+  if (!fp32) return nzr_compiled(NZR) ? "passes, 64-bit fixed point" : "radix, 64-bit fixed point";
+  std::string s = nzr_compiled(NZR) ? "in-place passes" : "radix";
+  if (v <= 0) return s;
   int k = 0;
-  std::string s = "in-place passes";
 #define NSP_Z2_NAME(len, a, b, r) \
   if (NZR == len && NTP % r == 0 && ++k == v) s = "two-pass " #a "x" #b;
   NSP_Z2_LIST(NSP_Z2_NAME)
@@ -633,7 +634,7 @@ static void launch_nl_t(const Tables& tb, const Bufs& bf, Ctl* dctl, const doubl
   }
   if (mask & 2) {
     bool done = false;
-    // the group's z-stage variant: the k-th two-pass split of the length, or (0) radix
+    // the group's z-stage variant: the k-th two-pass split of the length, or (0) in place
     if (tb.z_variant > 0) {
       int k = 0;
 #define NSP_CASE_Z2(n, a, b, r)                                                      \
