@@ -1,7 +1,7 @@
-// nsp_bounds.cuh -- the bounds-checked build of the step kernels.
+// nsp_bounds.cuh -- the bounds-checked build of the step and diagnostic kernels.
 //
 // Compiled with -DNSP_BOUNDS_CHECK (nspipe-gpu_gb300/build.py --bounds-check, which
-// makes libnspipe_gb300_bc.so), every global-memory access of the step kernels whose
+// makes libnspipe_gb300_bc.so), every global-memory access of those kernels whose
 // index is computed from the launch geometry is checked against the extent of the
 // array (or member slab) it addresses.  An access outside it is skipped -- a load
 // reads zero, a store is dropped -- and counted in the context's bounds record
@@ -43,6 +43,8 @@ enum BoundsSite {
   BC_Z_OUT,            // z stage: H store
   BC_MIRROR,           // FP32 mirror of an outside state
   BC_CONVERGE,         // convergence bookkeeping: member index
+  BC_DIAG,             // diagnostics: state load
+  BC_CROSS,            // cross sections: mean-square and result stores
 };
 
 }  // namespace nsp

@@ -1,6 +1,7 @@
 // nsp_cross.cu -- the cross-section diagnostics, transforms in 64-bit fixed point (nsp_fx.cuh).
 #include <algorithm>
 
+#include "nsp_bounds.cuh"
 #include "nsp_fx.cuh"
 #include "nsp_internal.h"
 
@@ -41,9 +42,14 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
     // both lines of a pair copied asynchronously into the line they become (fx_z)
     auto plus = [&](int mu) { return row + (size_t)mu * NZ; };
     auto minus = [&](int mu) { return row + (size_t)(mu ? NT - mu : 0) * NZ; };  // (mu = NT/2: the same line, unused)
+    auto live = [&](int mu) {  // both lines inside the member's component
+      const int last = mu && mu < NT / 2 ? NT - mu : mu;
+      return NSP_IN_BOUNDS(tb, (size_t)i * tb.NTNZ + (size_t)last * NZ + NZ - 1, tb.S, BC_DIAG);
+    };
     auto raw2 = [&](int q) { return q < NZ - 2 ? NZ + q : NZR - NZ + 2 + q; };
     if constexpr (NZRC > 0) {
       for (int b = threadIdx.x >> 5; b < nb; b += NTH / 32) {
+        if (!live(mu0 + b)) continue;
         cpx<fx>* Zt = Z + (size_t)b * ZP;
         const double2 *P = plus(mu0 + b), *M = minus(mu0 + b);
         for (int q = lane; q < NZ; q += 32) {
@@ -58,6 +64,11 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
     for (int b = threadIdx.x >> 5; b < nb; b += NTH / 32) {
       const int mu = mu0 + b;
       cpx<fx>* Zt = Z + (size_t)b * ZP;
+      if (!live(mu)) {
+        for (int q = lane; q < NZR; q += 32) Zt[q] = mk<fx>(0, 0);
+        if (lane == 0) sE[b] = 0;
+        continue;
+      }
       const double2* raw = reinterpret_cast<const double2*>(Zt);
       const double2 *P = plus(mu), *M = minus(mu);
       auto at_p = [&](int q) { return NZRC > 0 ? raw[q] : P[q]; };
@@ -104,7 +115,9 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
     }
     __syncthreads();
   }
-  double* o = part + (((size_t)blockIdx.z * 3 + c) * tb.NR + i) * NZR;
+  const size_t o0 = (((size_t)blockIdx.z * 3 + c) * tb.NR + i) * NZR;
+  if (!NSP_IN_BOUNDS(tb, o0 + NZR - 1, (size_t)gridDim.z * 3 * tb.NR * NZR, BC_CROSS)) return;
+  double* o = part + o0;
 #pragma unroll
   for (int k = 0; k < KZ; k++) {
     const int n = threadIdx.x + k * NTH;
@@ -124,6 +137,7 @@ __global__ void cross_sum_k(Tables tb, const double* __restrict__ part, double* 
     q += w * s;
     u += w * p[(size_t)(2 * NR + i) * NZR];
   }
+  if (!NSP_IN_BOUNDS(tb, ((size_t)blockIdx.y * 2 + 1) * NZR + n, (size_t)gridDim.y * 2 * NZR, BC_CROSS)) return;
   out[((size_t)blockIdx.y * 2) * NZR + n] = q;
   out[((size_t)blockIdx.y * 2 + 1) * NZR + n] = u;
 }

@@ -1294,7 +1294,9 @@ __global__ void __launch_bounds__(DIV_TH) diag_div_k(Tables tb, const double2* _
   U += (size_t)blockIdx.z * 3 * S;  // member blockIdx.z of a batched launch
   out += 2 * blockIdx.z;
   unsigned long long mi = 0, mw = 0;  // bits of the largest squares: they order like the values
-  if (k < NTNZ) {
+  // the last row of the block's stencils, and the first
+  if (k < NTNZ && NSP_IN_BOUNDS(tb, (size_t)(stencil_base(row1 - 1, NR) + STEN - 1) * NTNZ + k, S, BC_DIAG) &&
+      NSP_IN_BOUNDS(tb, (long long)stencil_base(row0, NR) * NTNZ + k, S, BC_DIAG)) {
     const int it = k / NZ, l = k - it * NZ, m = it < NT / 2 ? it : it - NT;
     const double kt = tb.kts * (double)m, kz = tb.kzs * (double)l;
     const int tab = abs((abs(m) % 2) - 1);
@@ -1356,6 +1358,7 @@ __global__ void gather_mean_k(Tables tb, const double2* __restrict__ U, double* 
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nmem * tb.NR) return;
   const int m = q / tb.NR, i = q - m * tb.NR;
+  if (!NSP_IN_BOUNDS(tb, (size_t)i * tb.NTNZ, tb.S, BC_DIAG)) return;
   out[q] = U[((size_t)m * 3 + 2) * tb.S + (size_t)i * tb.NTNZ].x;
 }
 
