@@ -25,8 +25,9 @@ namespace nsp {
 template <int NZRC, int RPB>
 __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tables tb, const double2* __restrict__ U,
                                                                             double* __restrict__ part) {
-  constexpr int NTH = z_threads(NZRC), NB = RPB * 6, KZ = NZRC > 0 ? (NZRC + NTH - 1) / NTH : 4;
-  static_assert(NZRC > 0 || 6 * (KZ * NTH / 4) >= RT_TASKS, "points of a run-time length (radices up to 4)");
+  constexpr int ZTH = z_threads(NZRC), NB = RPB * 6, KZ = NZRC > 0 ? (NZRC + ZTH - 1) / ZTH : 4;
+  static_assert(NZRC > 0 || 6 * (KZ * ZTH / 4) >= RT_TASKS, "points of a run-time length (radices up to 4)");
+  const int NTH = NZRC > 0 ? ZTH : blockDim.x;
   const int i = blockIdx.x, c = blockIdx.y, lane = threadIdx.x & 31;
   extern __shared__ __align__(16) unsigned char smraw[];
   cpx<fx>* Z = reinterpret_cast<cpx<fx>*>(smraw);  // [NB] lines of ZP
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_cross(Tabl
     }
     __syncthreads();
     if constexpr (NZRC > 0)
-      pass_fft<fx, +1, NZRC, NB, 1, line_pitch(NZRC), false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx, nb);
+      pass_fft<fx, +1, NZRC, NB, 1, line_pitch(NZRC), false, ZTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx, nb);
     else
       fft_batch<fx, +1, MAXRZ, false>(Z, tb.pz, nb, 1, NZR, tb.tw_zx);
 #pragma unroll
@@ -132,10 +133,24 @@ __global__ void cross_sum_k(Tables tb, const double* __restrict__ part, double* 
   if (n >= NZR) return;
   const double* p = part + (size_t)blockIdx.y * 3 * NR * NZR + n;
   double q = 0.0, u = 0.0;
-  for (int i = 0; i < NR; i++) {
-    const double w = tb.rdr[i], s = p[(size_t)i * NZR] + p[(size_t)(NR + i) * NZR];
-    q += w * s;
-    u += w * p[(size_t)(2 * NR + i) * NZR];
+  constexpr int B = 8;  // rows whose loads are in flight together (one by one: a chain of NR latencies)
+  for (int i0 = 0; i0 < NR; i0 += B) {
+    double w[B], r[B], t[B], z[B];
+#pragma unroll
+    for (int k = 0; k < B; k++) {
+      const size_t i = min(i0 + k, NR - 1);
+      w[k] = tb.rdr[i];
+      r[k] = p[i * NZR];
+      t[k] = p[(NR + i) * NZR];
+      z[k] = p[(2 * NR + i) * NZR];
+    }
+#pragma unroll
+    for (int k = 0; k < B; k++) {
+      if (i0 + k < NR) {
+        q += w[k] * (r[k] + t[k]);
+        u += w[k] * z[k];
+      }
+    }
   }
   if (!NSP_IN_BOUNDS(tb, ((size_t)blockIdx.y * 2 + 1) * NZR + n, (size_t)gridDim.y * 2 * NZR, BC_CROSS)) return;
   out[((size_t)blockIdx.y * 2) * NZR + n] = q;
@@ -145,7 +160,7 @@ __global__ void cross_sum_k(Tables tb, const double* __restrict__ part, double* 
 template <int NZRC, int RPB>
 static void launch_cross_t(const Tables& tb, const double2* U, double* part, cudaStream_t st, int nmem) {
   const size_t sm = sizeof(cpx<fx>) * 6 * RPB * (NZRC > 0 ? line_pitch(NZRC) : tb.NZR);
-  fx_cross<NZRC, RPB><<<dim3(tb.NR, 3, nmem), z_threads(NZRC), sm, st>>>(tb, U, part);
+  fx_cross<NZRC, RPB><<<dim3(tb.NR, 3, nmem), NZRC > 0 ? z_threads(NZRC) : rt_z_threads(tb.NZR), sm, st>>>(tb, U, part);
 }
 
 void launch_diag_cross(const Tables& tb, const double2* U, double* part, double* out, cudaStream_t st, int nmem) {

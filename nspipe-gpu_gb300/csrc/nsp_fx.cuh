@@ -225,5 +225,12 @@ constexpr int line_pitch(int n) { return line_pad(n - 1) + 1 > n + 2 ? line_pad(
 // each leave three blocks on an SM.
 constexpr int z_rows(int n) { return n == 0 || n >= 384 ? 1 : 2; }
 static_assert(MAXRZ * z_threads(0) >= RT_TASKS, "register rounds of the run-time FFT");
+// Threads of a run-time length: a thread's 255 registers leave an SM one block of 192, and six
+// lines of up to 18 points are 18 to 54 butterflies, so those take blocks of 64 (64 members of
+// NR=48 x 4 x 2 modes, z stage: 867 -> 291 us, FP64 transforms 797; 64 of 18 x 6: 5185 -> 1767,
+// 5245; the cross sections of 64 of NR=96 x 4 x 2: 658 -> 300, direct sums 229).
+constexpr int RT_SHORT = 18;
+constexpr int rt_z_threads(int n) { return n <= RT_SHORT ? 64 : z_threads(0); }
+static_assert(MAXRZ * rt_z_threads(RT_SHORT) >= 6 * RT_SHORT / 2, "register rounds of the short run-time lengths");
 
 }  // namespace nsp

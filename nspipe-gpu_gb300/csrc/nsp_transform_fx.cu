@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(TTH) fx_theta_inv(Tables tb, Bufs bf, const Ct
 // warp takes a pair of a row: both half spectra's scales, then their packed Hermitian extension.
 template <int NZRC, int RPB>
 __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables tb, Bufs bf, const Ctl* ctl, int standalone) {
-  constexpr int NTH = z_threads(NZRC);
+  const int NTH = NZRC > 0 ? z_threads(NZRC) : blockDim.x;
   const int mloc = blockIdx.z, i = blockIdx.y, j0 = blockIdx.x * RPB;
   if (!standalone && ctl->phase[tb.mem0 + mloc] < 0) return;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
   __syncthreads();
   constexpr int BS = NZRC > 0 ? line_pitch(NZRC) : 0;
   if constexpr (NZRC > 0)
-    pass_fft<fx, +1, NZRC, RPB * 6, 1, BS, false, NTH, NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx);
+    pass_fft<fx, +1, NZRC, RPB * 6, 1, BS, false, z_threads(NZRC), NZRC / 3 + 1, 2 * NZRC / 3 - 1, 0, -1>(Z, tb.tw_zx);
   else
     fft_batch<fx, +1, MAXRZ, false>(Z, tb.pz, RPB * 6, 1, NZR, tb.tw_zx);
   // -(u.grad)u (calcNonlinear_k) in FP64, packed for the forward transforms:
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(z_threads(NZRC), z_blocks(NZRC)) fx_z(Tables t
   }
   __syncthreads();
   if constexpr (NZRC > 0)
-    pass_fft<fx, -1, NZRC, NFWD, 1, BS, false, NTH, 0, -1, NZRC / 3, 2 * NZRC / 3>(Z, tb.tw_zx);
+    pass_fft<fx, -1, NZRC, NFWD, 1, BS, false, z_threads(NZRC), 0, -1, NZRC / 3, 2 * NZRC / 3>(Z, tb.tw_zx);
   else
     fft_batch<fx, -1, MAXRZ, false>(Z, tb.pz, NFWD, 1, NZR, tb.tw_zx);
   // Unpack: x = a + i b  ->  A_q = (X_q + conj X_{-q})/2,  B_q = (X_q - conj X_{-q})/(2i).
@@ -489,7 +489,8 @@ static void launch_theta_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, const d
 template <int NZRC, int RPB>
 static void launch_z_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, bool standalone, cudaStream_t st, int nm) {
   const size_t sm = sizeof(cpx<fx>) * 6 * RPB * (NZRC > 0 ? line_pitch(NZRC) : tb.NZR);
-  fx_z<NZRC, RPB><<<dim3((tb.NTP + RPB - 1) / RPB, tb.NR, nm), z_threads(NZRC), sm, st>>>(tb, bf, dctl, standalone ? 1 : 0);
+  fx_z<NZRC, RPB><<<dim3((tb.NTP + RPB - 1) / RPB, tb.NR, nm), NZRC > 0 ? z_threads(NZRC) : rt_z_threads(tb.NZR), sm, st>>>(
+      tb, bf, dctl, standalone ? 1 : 0);
 }
 
 void launch_nonlinear_fx(const Tables& tb, const Bufs& bf, Ctl* dctl, const double2* src, double2* dst,
