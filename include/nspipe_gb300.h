@@ -45,8 +45,9 @@ extern "C" {
 
 #define NSP_FP64 0  /* plain form: FP64 (matches the reference); its FFTs in 64-bit fixed point, one scale
                              per transform line: a line's error is relative to its norm, as an FP64 FFT's
-                             is, and the nonlinear term's within 5e-16 of its norm at a level.  FP64's range;
-                             a line whose sum of magnitudes passes about 2^1023 gives NaN               */
+                             is, and the nonlinear term's some 1e-16 of its norm at a level (the rounding of the
+                             radial derivatives' FP64 sums apart).  FP64's range; a line whose sum of
+                             magnitudes passes about 2^1023 gives NaN                                  */
 #define NSP_MIXED 1 /* transforms + nonlinear product in FP32 (theta DFT 3xTF32); solves and corrections
                              in double-float (FP32 pairs) or FP32 on corrector increments; state in FP64 */
 

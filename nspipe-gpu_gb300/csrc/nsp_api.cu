@@ -322,8 +322,8 @@ int reset_control(nsp_ctx* c) {
   return NSP_OK;
 }
 
-// The z-stage kernel of each group (radix-stage or one of the two-pass splits compiled
-// for its length and precision), timed like the linear pass: z stage alone on the
+// The z-stage kernel of each group (in place, or in the mixed form one of the two-pass splits
+// compiled for its length), timed like the linear pass: z stage alone on the
 // group's buffers, best of 3 after a warm-up.  Cached per shape and precision,
 // "z2:NRxNTxNZ:pP", not per member count: the kernels differ in rounding, and members
 // of one shape give the same bits whatever ensemble they are stepped in.

@@ -241,9 +241,11 @@ template <typename T, int SIGN, int P> __device__ __forceinline__ void reg_dft(c
 
 // Radices of the compiled lengths: few passes over shared memory, with few enough complex
 // values in registers for the kernels' blocks per SM (nsp_fx.cuh: at 192 points 8 x 4 x 6 takes
-// 665, 16 x 12 733 ns per member and mode); 0: the length has no compiled transform.  (768:
-// 8 x 8 x 12 takes 3% less, but its rounding moves the step at which the unstable NR=96 run of
-// tests/test_gpu_c1_diag.py leaves single corrector passes.)
+// 665, 16 x 12 733 ns per member and mode); 0: the length has no compiled transform.  768, one plan
+// for both forms: 16 x 8 x 6 takes 88 us in the mixed z stage of a pipe of 48 x 64 x 256 modes and
+// 450 in the FP64 form's, 8 x 8 x 12 96 and 435 with an error some 4% lower; the rounding of the
+// first leaves the unstable NR=96 run of tests/test_gpu_c1_diag.py in single corrector passes as long
+// as the reference's.
 // Columns (the theta transforms) have no padding and more lines: two passes where three would do.
 __host__ __device__ constexpr int pass_radix(int n, int s, bool cols) {
   if (cols && n == 192) return s == 0 ? 16 : s == 1 ? 12 : 0;

@@ -101,9 +101,6 @@ __device__ __forceinline__ bool mean_field(int f) { return f == 1 || f == 2 || f
 struct Mean32 {
   float W, U, Wp, Up, rinv;
 };
-// The mean flow at level i of a member's FP32 transform input (U32: its 3 components; DR32:
-// their radial derivatives, or null: the 7-point parity stencil, u_theta odd and u_z even
-// at m = 0).
 // The mean flow at level i as the theta-inverse recorded it (Bufs::MEAN of a member: NR rows).
 __device__ __forceinline__ Mean32 mean_flow32_rec(const Tables& tb, const float* mean, int i) {
   const float* m = mean + (size_t)i * MEAN_N;
@@ -115,6 +112,9 @@ __device__ __forceinline__ Mean32 mean_flow32_rec(const Tables& tb, const float*
   o.rinv = tb.rinv32[i];
   return o;
 }
+// The mean flow at level i of a member's FP32 transform input (U32: its 3 components; DR32:
+// their radial derivatives, or null: the 7-point parity stencil, u_theta odd and u_z even
+// at m = 0).
 __device__ __forceinline__ Mean32 mean_flow32(const Tables& tb, const float2* U32, const float2* DR32, int i) {
   const long long S = tb.S;
   const size_t h = (size_t)i * tb.NTNZ;

@@ -578,10 +578,9 @@ static void launch_z2(const Tables& tb, const Bufs& bf, Ctl* dctl, bool standalo
 constexpr int zp_rows(int n) { return n == 0 || n == 384 || n >= 576 ? 1 : 2; }
 // Two-pass z stage: (NZR, N1, N2, rows per block); the setup-time autotuner picks among
 // the splits and the in-place passes per shape (which win at 432 and 768 points, so those have no
-// split).  Every other 2^a 3^b length up to 576 that a register pass of at most 24 points splits
-// is here: the run-time kernel, bound by its index
-// arithmetic, takes 1066 us where the 18 x 9 split takes 89 (7 members of NR=61, 36 x 54
-// modes); its theta transforms (NTP = 54) 274 and 85 us where the compiled ones take 80 and 27.
+// split).  The run-time kernel, bound by its index arithmetic, takes 1066 us where the 18 x 9 split
+// takes 89 (7 members of NR=61, 36 x 54 modes); its theta transforms (NTP = 54) 274 and 85 us where
+// the compiled ones take 80 and 27.  Of the accepted lengths 6, 12, 18 and 324 points stay with it.
 #define NSP_Z2_LIST(X) X(24, 4, 6, 2) X(36, 6, 6, 2) X(48, 8, 6, 2) X(54, 9, 6, 2) X(72, 12, 6, 2) \
   X(108, 9, 12, 2) X(108, 12, 9, 2) X(144, 12, 12, 2) X(162, 9, 18, 2) X(162, 18, 9, 2) X(216, 18, 12, 2) \
   X(288, 16, 18, 2) X(288, 12, 24, 2) X(96, 8, 12, 2) X(96, 12, 8, 2) X(192, 16, 12, 2) \

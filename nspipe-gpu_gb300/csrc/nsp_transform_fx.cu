@@ -17,10 +17,10 @@
 // scale, and with it every bit, is independent of the order), and the line is converted
 // in place.
 // Bound: integer issue, the barriers between the passes and instruction fetch (z stage, 16
-// members of NR=48 x 32 x 64 modes: ALU pipe 55%, IMAD 49%, FP64 pipe 24%).  FP64 transforms
+// members of NR=48 x 32 x 64 modes: issue 70%, ALU pipe 64%, FMA pipe 31%, FP64 pipe 26%).  FP64 transforms
 // were bound by the FP64 pipe alone.  Per launch there, before and after: theta-inverse 903 ->
-// 282 us, z stage 3457 -> 692 us, theta-forward 283 -> 82 us; one member of 48 x 64 x 256
-// modes: 530 -> 160, 2154 -> 451, 168 -> 46 us.
+// 285 us, z stage 3457 -> 699 us, theta-forward 283 -> 84 us; one member of 48 x 64 x 256
+// modes: 530 -> 160, 2154 -> 450, 168 -> 47 us.
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
